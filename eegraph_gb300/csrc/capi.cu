@@ -103,6 +103,7 @@ static void free_ws(eeg_vgraph* vg) {
     if (w.activity) cudaFree(w.activity);
     if (w.tctrl) cudaFree(w.tctrl);
     vg_free(vg, w.x);
+    vg_free(vg, w.pr_y);
     vg_free(vg, w.contrib[0]);
     vg_free(vg, w.contrib[1]);
     vg_free(vg, w.acc);

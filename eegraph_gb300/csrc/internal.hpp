@@ -72,6 +72,7 @@ struct PRCtrl {
     BarrierWords bw;
     double resid[3];     // ||x_{k+1}-x_k||_1 per sweep (rotating)
     double norm[3];      // ||x_{k+1}||_1 per sweep (rotating)
+    double probe[3];     // residual form: ||f_{k+1} - rho f_k||_1 of a measuring sweep (rotating)
     uint32_t iterations;
     uint32_t pad;
     double last_resid;
@@ -106,6 +107,7 @@ struct Workspace {
     TravCtrl* tctrl = nullptr;
     // PageRank
     float* x = nullptr;           // n
+    float2* pr_y = nullptr;       // n: iterate of the extrapolated sweeps, (value, compensation)
     float* contrib[2] = {nullptr, nullptr};  // n each
     double* acc = nullptr;        // n (partials of vertices whose parts cross warp chunks)
     uint32_t* arrive = nullptr;   // n (chunks that delivered a partial, per vertex)

@@ -18,9 +18,19 @@
 //    the number of chunks spanned finalises it. So a sweep needs ONE grid barrier.
 //  * Stop test in FP64: ||x_{k+1}-x_k||_1 * d/(1-d) <= tol * ||x_{k+1}||_1 bounds the distance to the
 //    fixed point (the Jacobi map contracts by d in the L1 norm).
-//   SYNC variants: contrib double-buffered (deterministic Jacobi up to the FP64 partial order).
-//   ASYNC variants: contrib updated in place (values of this sweep are used as soon as written; same
-//   fixed point, fewer sweeps, order-dependent rounding).
+// Two forms of the sweep (template parameter RES):
+//   Residual form (every run without an explicit sweep cap, SYNC and ASYNC): contrib holds f / outdeg of
+//   the residual f of the iterate, a sweep gathers g = d * sum of them, and the iterate moves by alpha g
+//   with alpha from the extrapolation control (common.cuh). The kernel was bound by the number of its
+//   sweeps (0.18 ms each on R-MAT s22, gathers through L1): R-MAT s22, K = 16, 17.3 -> 3.3 ms, relative
+//   error against 64 bits 1.0e-7 -> 4.7e-8. In value form the same
+//   steps would meet FP32's rounding of x (on a grid the alternating mode then never settles below the
+//   stop test); the residual shrinks, and its rounding with it. The iterate is an FP32 pair
+//   (value, compensation), and after a step the sweeps stop at a quarter of the tolerance, so the result
+//   is closer to the 64-bit fixed point than the plain sweeps leave it.
+//   Value form (runs with an explicit sweep cap, whose result after k sweeps is the k-th Jacobi iterate):
+//   SYNC variants double-buffer contrib, ASYNC variants update it in place (values of this sweep are used
+//   as soon as written; order-dependent rounding).
 #include <algorithm>
 #include <cmath>
 
@@ -46,6 +56,7 @@ struct PRArgs {
     const uint2* __restrict__ info;       // per vertex: (rank in descending out-degree-class order, out-degree)
     uint32_t hot;                         // contributions of ranks < hot are staged in shared memory
     float* x;
+    float2* y;         // residual form: the iterate, (value, compensation)
     float* c0;
     float* c1;
     double* acc;       // FP64 partial sums of vertices whose parts span chunks
@@ -54,6 +65,9 @@ struct PRArgs {
     PRCtrl* ctrl;
     float damping;
     float base;
+    double damping64;  // residual form: d as an FP64 value and split into an FP32 pair, base = 1 - d
+    double base64;
+    float d_hi, d_lo;
     double tol;
     uint64_t timeout_ns;
     uint32_t inplace;
@@ -66,6 +80,38 @@ __device__ __forceinline__ void finalize(const PRArgs& a, uint32_t v, uint32_t r
     nrm += (double)xn;
     a.x[v] = xn;
     cnext[rk] = od ? xn / (float)od : 0.f;
+}
+
+// Residual form: (hi, lo) is the gathered sum, y the iterate's old pair. A vertex without out-edges is
+// never gathered, so its contribution slot keeps its residual itself. `step` (the same in the whole grid)
+// holds the step length and the one to measure for (0 = none).
+__device__ __forceinline__ void finalize_res(const PRArgs& a, uint32_t v, uint32_t rk, float hi, float lo, float2 y,
+                                             uint32_t od, const float* ccur, float* cnext, float2 step, double& r,
+                                             double& nrm, double& q) {
+    const float g = fmaf(a.d_hi, hi, fmaf(a.d_hi, lo, a.d_lo * hi));
+    float f = g, add = g, add_lo = 0.f;
+    if (step.x != 1.f) {
+        // (1 - alpha) f + alpha g cancels: the products go in as exact pairs, and g and the old residual
+        // f = contribution * out-degree (what was gathered) with their low parts
+        const float g_lo = fmaf(a.d_hi, hi, -g) + fmaf(a.d_hi, lo, a.d_lo * hi);
+        const float c = ccur[rk], w = od ? (float)od : 1.f, b = 1.f - step.x;
+        add = step.x * g;
+        add_lo = fmaf(step.x, g, -add) + step.x * g_lo;
+        const float fo = c * w, fo_lo = fmaf(c, w, -fo);
+        const float p = b * fo, p_lo = fmaf(b, fo, -p) + b * fo_lo;
+        float e;
+        two_sum(p, add, f, e);
+        f = __fadd_rn(f, __fadd_rn(e, __fadd_rn(p_lo, add_lo)));
+    } else if (step.y != 0.f) {
+        const float fo = od ? ccur[rk] * (float)od : ccur[rk];
+        q += fabs((double)fmaf(-(1.f - 1.f / step.y), fo, g));
+    }
+    float s, e;
+    two_sum(y.x, add, s, e);
+    a.y[v] = make_float2(s, __fadd_rn(y.y, __fadd_rn(e, add_lo)));
+    cnext[rk] = od ? f / (float)od : f;
+    r += fabs((double)f);
+    nrm += fabs((double)s);
 }
 
 constexpr int XCAP = 64;  // per-warp list of (vertex, chunks spanned) awaiting their arrival count
@@ -90,16 +136,17 @@ __device__ __forceinline__ void settle_spanning(const PRArgs& a, const uint2* xb
     __syncwarp();
 }
 
-template <int K>
+template <int K, bool RES>
 __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
     constexpr int PR_U = InFlight<K>::U;
     extern __shared__ float4 s_hot4[];  // contributions of the `hot` highest out-degree vertices
     const float* s_hot = reinterpret_cast<const float*>(s_hot4);
-    __shared__ double s_red[2][PR_TPB / 32];
+    __shared__ double s_red[RES ? 3 : 2][PR_TPB / 32];
     __shared__ unsigned long long s_zero;
     __shared__ uint2 s_span[PR_TPB / 32][XCAP];
     __shared__ uint32_t s_next;  // next of this CTA's chunks to hand out in the current sweep
     __shared__ double s_rn[2];   // the last sweep's residual and norm
+    __shared__ Extrapolation s_ex;  // residual form: step lengths (thread 0; the same in every CTA)
     uint2* xbuf = s_span[threadIdx.x >> 5];
     PRCtrl* ctrl = a.ctrl;
     const uint32_t gtid = blockIdx.x * PR_TPB + threadIdx.x;
@@ -110,17 +157,27 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
     uint32_t epoch = 0;
 
     // ---- set-up: x0 = 1-d, contrib0, partial slots; count vertices without in-edges
-    if (threadIdx.x == 0) s_zero = 0;
+    if (threadIdx.x == 0) {
+        s_zero = 0;
+        extrapolation_init(s_ex);
+    }
     __syncthreads();
     unsigned long long zero_in = 0;
     for (uint32_t v = gtid; v < a.n; v += gthreads) {
-        a.x[v] = a.base;
         const uint2 inf = a.info[v];
         const uint32_t od = inf.y;
-        const float c = od ? a.base / (float)od : 0.f;
         const uint32_t rk = inf.x;
-        a.c0[rk] = c;
-        a.c1[rk] = c;
+        if (RES) {  // y0 = base; the first sweep's residual is d P base, zero where there is no in-edge
+            const float b = (float)a.base64;
+            a.y[v] = make_float2(b, (float)(a.base64 - (double)b));
+            a.c0[rk] = od ? b / (float)od : 0.f;
+            a.c1[rk] = 0.f;
+        } else {
+            const float c = od ? a.base / (float)od : 0.f;
+            a.x[v] = a.base;
+            a.c0[rk] = c;
+            a.c1[rk] = c;
+        }
         a.acc[v] = 0.0;
         a.arrive[v] = 0u;
         zero_in += (a.rvstart[v + 1] == a.rvstart[v]) ? 1ull : 0ull;
@@ -145,16 +202,28 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 ctrl->resid[(s + 1u) % 3u] = 0.0;
                 ctrl->norm[(s + 1u) % 3u] = 0.0;
+                if (RES) ctrl->probe[(s + 1u) % 3u] = 0.0;
             }
             // ccur is read through L1 (plain loads): the grid barrier's acquire makes the previous sweep's
             // values visible, and within a sweep they do not change (SYNC) or may be stale (ASYNC, allowed)
-            const float* ccur = (s & 1u) && !a.inplace ? a.c1 : a.c0;
-            float* cnext = a.inplace ? a.c0 : ((s & 1u) ? a.c0 : a.c1);
-            double r = 0.0, nrm = 0.0;
+            const bool inplace = !RES && a.inplace;
+            const float* ccur = (s & 1u) && !inplace ? a.c1 : a.c0;
+            float* cnext = inplace ? a.c0 : ((s & 1u) ? a.c0 : a.c1);
+            const float2 step = RES ? make_float2(s_ex.alpha, s_ex.cand) : make_float2(1.f, 0.f);
+            if (RES && s == 1u)  // c0 still holds the base's contributions where no sweep writes
+                for (uint32_t v = gtid; v < a.n; v += gthreads)
+                    if (a.rvstart[v + 1] == a.rvstart[v]) a.c0[a.info[v].x] = 0.f;
+            double r = 0.0, nrm = 0.0, q = 0.0;
             uint32_t nx = 0;  // warp-uniform fill of xbuf
             auto fin = [&](uint32_t vv, double sum) {
                 const uint2 inf = __ldg(&a.info[vv]);
-                finalize(a, vv, inf.x, sum, __ldcg(&a.x[vv]), inf.y, cnext, r, nrm);
+                if (RES) {
+                    const float hi = (float)sum;
+                    finalize_res(a, vv, inf.x, hi, (float)(sum - (double)hi), __ldcg(&a.y[vv]), inf.y, ccur, cnext,
+                                 step, r, nrm, q);
+                } else {
+                    finalize(a, vv, inf.x, sum, __ldcg(&a.x[vv]), inf.y, cnext, r, nrm);
+                }
             };
             // stage this sweep's hot contributions (the barrier before the sweep ordered every CTA's
             // writes of the previous sweep; ASYNC may see some of this sweep's, which it allows)
@@ -207,20 +276,21 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
                 my_edges += nvalid;
                 // segment ends: prefetch what finalisation needs while the gathers are in flight
                 bool last[PR_U];
-                float xo[PR_U];
+                float2 xo[PR_U];  // the old value (residual form: its pair)
                 uint32_t od[PR_U], rk[PR_U];
 #pragma unroll
                 for (int u = 0; u < PR_U; ++u) {
                     const uint32_t vn = __shfl_down_sync(0xffffffffu, v[u], 1);
                     last[u] = valid[u] && (lane == 31u || vn != v[u]);
-                    xo[u] = 0.f;
+                    xo[u] = make_float2(0.f, 0.f);
                     od[u] = 0u;
                     rk[u] = 0u;
                     if (last[u]) {
                         const uint2 inf = __ldg(&a.info[v[u]]);
                         rk[u] = inf.x;
                         od[u] = inf.y;
-                        xo[u] = __ldcg(&a.x[v[u]]);
+                        if (RES) xo[u] = __ldcg(&a.y[v[u]]);
+                        else xo[u].x = __ldcg(&a.x[v[u]]);
                     }
                 }
 #pragma unroll
@@ -249,7 +319,8 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
                     if (last[u]) {
                         // the vertex began before this chunk, or continues after it
                         if (!((seg0 == 0u && before0 == v[u]) || (lane == 31u && vb[u] == v[u]))) {
-                            finalize(a, v[u], rk[u], (double)hi + (double)lo, xo[u], od[u], cnext, r, nrm);
+                            if (RES) finalize_res(a, v[u], rk[u], hi, lo, xo[u], od[u], ccur, cnext, step, r, nrm, q);
+                            else finalize(a, v[u], rk[u], (double)hi + (double)lo, xo[u].x, od[u], cnext, r, nrm);
                         } else {  // partial now, arrival counted in the warp's next settle
                             atomicAdd(&a.acc[v[u]], (double)hi + (double)lo);
                             spans = true;
@@ -274,10 +345,12 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
             for (int off = 16; off > 0; off >>= 1) {
                 r += __shfl_down_sync(0xffffffffu, r, off);
                 nrm += __shfl_down_sync(0xffffffffu, nrm, off);
+                if (RES && step.y != 0.f) q += __shfl_down_sync(0xffffffffu, q, off);
             }
             if (lane == 0) {
                 s_red[0][threadIdx.x >> 5] = r;
                 s_red[1][threadIdx.x >> 5] = nrm;
+                if (RES) s_red[RES ? 2 : 0][threadIdx.x >> 5] = q;
             }
             __syncthreads();
             if (threadIdx.x == 0) {
@@ -288,6 +361,11 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
                 }
                 atomicAdd(&ctrl->resid[slot], rr);
                 atomicAdd(&ctrl->norm[slot], nn);
+                if (RES && step.y != 0.f) {
+                    double qq = 0.0;
+                    for (int w = 0; w < PR_TPB / 32; ++w) qq += s_red[RES ? 2 : 0][w];
+                    atomicAdd(&ctrl->probe[slot], qq);
+                }
             }
             if (!grid_barrier_sync(&ctrl->bw, epoch, a.timeout_ns)) break;
             // one thread per CTA reads the sweep's totals (every warp reading the same two words would
@@ -295,10 +373,23 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
             if (threadIdx.x == 0) {
                 s_rn[0] = *(volatile double*)&ctrl->resid[slot];
                 s_rn[1] = *(volatile double*)&ctrl->norm[slot];
+                if (RES) extrapolation_next(s_ex, s_rn[0], *(volatile double*)&ctrl->probe[slot], a.damping64);
             }
             __syncthreads();
             const double resid = s_rn[0];
             const double norm = s_rn[1] + zero_norm;
+            if (RES) {  // not at the end of a long step (its residual is of the step's start)
+                const double tol = s_ex.steps ? 0.25 * a.tol : a.tol;
+                if (blockIdx.x == 0 && threadIdx.x == 0) {
+                    ctrl->last_resid = resid;
+                    ctrl->last_norm = norm;
+                }
+                if (step.x == 1.f && a.damping64 / (1.0 - a.damping64) * resid <= tol * norm) {
+                    ++s;
+                    break;
+                }
+                continue;
+            }
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 ctrl->last_resid = resid;
                 ctrl->last_norm = norm;
@@ -310,6 +401,11 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
         }
     }
 finish:
+    if (RES)  // the result; every CTA's values are settled (the last sweep's barrier, or an abort)
+        for (uint32_t v = gtid; v < a.n; v += gthreads) {
+            const float2 y = __ldcg(&a.y[v]);
+            a.x[v] = __fadd_rn(y.x, y.y);
+        }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) my_edges += __shfl_down_sync(0xffffffffu, my_edges, off);
     if (lane == 0 && my_edges) atomicAdd(&ctrl->edges_scanned, my_edges);
@@ -317,8 +413,8 @@ finish:
 }
 
 template <int K>
-eeg_status launch_pr(const PRArgs& args, int device, uint32_t bps, uint32_t hot_limit, cudaStream_t st) {
-    auto kern = k_pagerank<K>;
+eeg_status launch_pr(const PRArgs& args, bool res, int device, uint32_t bps, uint32_t hot_limit, cudaStream_t st) {
+    auto kern = res ? k_pagerank<K, true> : k_pagerank<K, false>;
     // shared memory left after the static arrays holds the hot contributions (multiple of 4 floats)
     cudaFuncAttributes fa{};
     EEG_CUDA(cudaFuncGetAttributes(&fa, kern));
@@ -425,10 +521,11 @@ __global__ void k_rank_cols(uint64_t slots, const uint32_t* __restrict__ col, co
 
 }  // namespace
 
-static eeg_status ensure_pr_ws(eeg_vgraph* vg) {
+static eeg_status ensure_pr_ws(eeg_vgraph* vg, bool res) {
     Workspace& ws = vg->ws;
     const size_t n = std::max<uint32_t>(vg->n, 1);
     if (!ws.x) EEG_TRY(vg_alloc(vg, (void**)&ws.x, sizeof(float) * n));
+    if (res && !ws.pr_y) EEG_TRY(vg_alloc(vg, (void**)&ws.pr_y, sizeof(float2) * n));
     if (!ws.contrib[0]) EEG_TRY(vg_alloc(vg, (void**)&ws.contrib[0], sizeof(float) * n));
     if (!ws.contrib[1]) EEG_TRY(vg_alloc(vg, (void**)&ws.contrib[1], sizeof(float) * n));
     if (!ws.acc) EEG_TRY(vg_alloc(vg, (void**)&ws.acc, sizeof(double) * n));
@@ -479,7 +576,9 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
         set_last_error("empty graph");
         return EEG_ERR_INVALID;
     }
-    EEG_TRY(ensure_pr_ws(vg));
+    // a run with an explicit sweep cap keeps the plain iterates
+    const bool res_form = o.max_iterations == 0;
+    EEG_TRY(ensure_pr_ws(vg, res_form));
     EEG_TRY(ensure_pr_rank(vg, st));
     Workspace& ws = vg->ws;
     const float damping = o.pr_damping > 0.f ? o.pr_damping : 0.85f;
@@ -492,6 +591,7 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
     a.rvcol = ws.pr_rcol;
     a.info = ws.pr_info;
     a.x = ws.x;
+    a.y = ws.pr_y;
     a.c0 = ws.contrib[0];
     a.c1 = ws.contrib[1];
     a.acc = ws.acc;
@@ -500,6 +600,10 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
     a.ctrl = ws.pctrl;
     a.damping = damping;
     a.base = 1.0f - damping;
+    a.damping64 = o.pr_damping > 0.f ? (double)o.pr_damping : 0.85;
+    a.base64 = 1.0 - a.damping64;
+    a.d_hi = (float)a.damping64;
+    a.d_lo = (float)(a.damping64 - (double)a.d_hi);
     a.tol = o.pr_tolerance > 0.f ? (double)o.pr_tolerance : 1e-7;
     a.timeout_ns = wait_limit_ns(o);
     a.inplace = (variant == EEG_ASYNC_PUSH_TD || variant == EEG_ASYNC_PUSH_DD) ? 1u : 0u;
@@ -507,9 +611,9 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
     EEG_CUDA(cudaEventRecord(ws.ev[0], st));
     eeg_status s;
     switch (vg->K) {
-        case 4: s = launch_pr<4>(a, vg->device, o.blocks_per_sm, o.pr_hot_limit, st); break;
-        case 8: s = launch_pr<8>(a, vg->device, o.blocks_per_sm, o.pr_hot_limit, st); break;
-        case 16: s = launch_pr<16>(a, vg->device, o.blocks_per_sm, o.pr_hot_limit, st); break;
+        case 4: s = launch_pr<4>(a, res_form, vg->device, o.blocks_per_sm, o.pr_hot_limit, st); break;
+        case 8: s = launch_pr<8>(a, res_form, vg->device, o.blocks_per_sm, o.pr_hot_limit, st); break;
+        case 16: s = launch_pr<16>(a, res_form, vg->device, o.blocks_per_sm, o.pr_hot_limit, st); break;
         default: set_last_error("K must be 4, 8 or 16"); return EEG_ERR_UNSUPPORTED;
     }
     if (s != EEG_OK) return s;
