@@ -19,6 +19,16 @@
 //   lane q of a group the float4 of columns 4q..4q+3, so one gather instruction moves G rows.
 //   Single column (the plain form): a lane owns a slot; part sums by K-lane butterflies, vertex sums by
 //   a segmented warp scan.
+// Two forms of a sweep (template parameter RES):
+//   Residual form (runs without an explicit sweep cap): a sweep gathers the rows of the residual f, the
+//   iterate moves by alpha g with g = d * (gathered sum), and the step length alpha comes from the
+//   extrapolation control (common.cuh): 94 + 78 sweeps of forward and adjoint become 21 + 21 on R-MAT
+//   graphs, which the gathers through L2 bound (R-MAT s18 x 64 columns, step with gradients 27.0 -> 8.6 ms). The first
+//   sweep gathers the source rows themselves; rows without parts in the direction keep a zero residual.
+//   The iterate is accumulated in FP32, so two last value-form sweeps (x = s b + d sum) replace the
+//   rounding of the additions by that of one sweep: relative L2 error of the adjoint at R-MAT s18 in a
+//   CPU model 9.1e-8 without them, 5.2e-8 with one, 2.8e-8 with two (plain sweeps: 1.0e-7).
+//   Value form (runs with an explicit cap, whose result after k sweeps is the k-th Jacobi iterate).
 // Stop test: d/(1-d) * ||Y_{k+1}-Y_k||_1 <= tol * ||Y_{k+1}||_1 over all columns, reduced in FP64
 // (FP32 per-chunk partials, FP64 per lane and across the grid); everything else is FP32.
 #include <algorithm>
@@ -62,7 +72,13 @@ struct DirTab {
     uint32_t* harrive;  // group completions per hub
     float* partial;     // hub chunk partials (slots x width)
     float* gpartial;    // group partials (groups x width)
+    const uint32_t* __restrict__ vstart;
 };
+
+// What a sweep of the solve does at a vertex's end (uniform over the grid). VALUE: x = s b + d sum.
+// Residual form, g = d sum: FIRST (gathers the source rows), PLAIN (y += g, f = g), PROBE (PLAIN, and q
+// for the control), STEP (y += alpha g, f = (1 - alpha) f + alpha g).
+enum Sweep : int { SW_VALUE = 0, SW_FIRST = 1, SW_PLAIN = 2, SW_PROBE = 3, SW_STEP = 4 };
 
 struct SolveArgs {
     DirTab g;
@@ -70,8 +86,11 @@ struct SolveArgs {
     const float* __restrict__ b;  // n x width source rows
     float scale_b;                // 1-d (forward) or 1 (adjoint)
     float d;
-    float* y0;
+    float scale_lo, d_lo;         // their low parts (runs without a cap; 0 in value-form runs)
+    float* y0;      // iterates (residual form: residuals)
     float* y1;
+    float* y;       // residual form: the iterate
+    float* res;     //                and the buffer of the result (y1 may share it: not read in the last sweep)
     PRCtrl* ctrl;
     uint32_t max_iters;
     double tol;
@@ -103,9 +122,13 @@ __device__ __forceinline__ float4 shfl_xor4(const float4& v, int o) {
 __device__ __forceinline__ float4 add4(const float4& a, const float4& b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
-__device__ __forceinline__ float4 affine4(float d, const float4& acc, float sb, const float4& b) {
-    return make_float4(fmaf(d, acc.x, sb * b.x), fmaf(d, acc.y, sb * b.y), fmaf(d, acc.z, sb * b.z),
-                       fmaf(d, acc.w, sb * b.w));
+// d acc + s b, both factors as (high, low) pairs
+__device__ __forceinline__ float affine(float d, float dl, float acc, float s, float sl, float b) {
+    return fmaf(d, acc, fmaf(dl, acc, fmaf(sl, b, s * b)));
+}
+__device__ __forceinline__ float4 affine4(float d, float dl, const float4& acc, float s, float sl, const float4& b) {
+    return make_float4(affine(d, dl, acc.x, s, sl, b.x), affine(d, dl, acc.y, s, sl, b.y),
+                       affine(d, dl, acc.z, s, sl, b.z), affine(d, dl, acc.w, s, sl, b.w));
 }
 __device__ __forceinline__ float l1diff4(const float4& a, const float4& b) {
     return fabsf(a.x - b.x) + fabsf(a.y - b.y) + fabsf(a.z - b.z) + fabsf(a.w - b.w);
@@ -358,24 +381,30 @@ __device__ bool hub_scalar(const DirTab& g, const Chunk& ch, float tot, uint32_t
     return true;
 }
 
-// End of a sweep: reduce the residual / norm, barrier, stop test. Returns 0 = continue, 1 = converged,
-// 2 = grid aborting.
-__device__ __forceinline__ int end_sweep(const SolveArgs& a, uint32_t s, double dr, double dn, uint32_t& epoch) {
+// End of a sweep: reduce the residual / norm (and the probe), barrier, stop test. Returns 0 = continue,
+// 1 = converged, 2 = grid aborting. With RES the control's next step is in *ex (shared).
+template <bool RES>
+__device__ __forceinline__ int end_sweep(const SolveArgs& a, uint32_t s, double dr, double dn, double dq, int mode,
+                                         Extrapolation* ex, uint32_t& epoch) {
     PRCtrl* ctrl = a.ctrl;
+    const bool probe = RES && mode == SW_PROBE;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         dr += __shfl_down_sync(FULL, dr, off);
         dn += __shfl_down_sync(FULL, dn, off);
+        if (probe) dq += __shfl_down_sync(FULL, dq, off);
     }
     if ((threadIdx.x & 31u) == 0 && (dr != 0.0 || dn != 0.0)) {
         atomicAdd(&ctrl->resid[s % 3], dr);
         atomicAdd(&ctrl->norm[s % 3], dn);
+        if (probe) atomicAdd(&ctrl->probe[s % 3], dq);
     }
     if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) return 2;
     __shared__ double s_rn[2];  // one read per CTA instead of one per warp
     if (threadIdx.x == 0) {
         s_rn[0] = __ldcg(&ctrl->resid[s % 3]);
         s_rn[1] = __ldcg(&ctrl->norm[s % 3]);
+        if (RES) extrapolation_next(*ex, s_rn[0], __ldcg(&ctrl->probe[s % 3]), (double)a.d);
     }
     __syncthreads();
     const double resid = s_rn[0], norm = s_rn[1];
@@ -383,28 +412,76 @@ __device__ __forceinline__ int end_sweep(const SolveArgs& a, uint32_t s, double 
         // slot (s+2)%3 was last read before barrier s and is next accumulated after barrier s+1
         ctrl->resid[(s + 2) % 3] = 0.0;
         ctrl->norm[(s + 2) % 3] = 0.0;
+        if (RES) ctrl->probe[(s + 2) % 3] = 0.0;
         ctrl->last_resid = resid;
         ctrl->last_norm = norm;
     }
-    return ((double)a.d / (1.0 - (double)a.d) * resid <= a.tol * norm) ? 1 : 0;
+    if (RES && mode == SW_STEP) return 0;  // its residual is that of the step's start
+    const double tol = RES && ex->steps ? 0.25 * a.tol : a.tol;
+    return ((double)a.d / (1.0 - (double)a.d) * resid <= tol * norm) ? 1 : 0;
+}
+
+// One element of a vertex's end in residual form: yv the iterate's (FIRST: the source row's) old value, fo
+// the old residual (PROBE and STEP), acc the gathered sum. Returns the new residual; yv becomes the new
+// iterate. A long step cancels: its products go in as exact pairs.
+__device__ __forceinline__ float res_elem(const SolveArgs& a, int mode, float alpha, float acc, float fo, float& yv,
+                                          float& q) {
+    float g = fmaf(a.d_lo, acc, a.d * acc);
+    if (mode == SW_FIRST) {
+        g = fmaf(a.scale_lo, g, a.scale_b * g);
+        yv = fmaf(a.scale_lo, yv, a.scale_b * yv);
+    } else if (mode == SW_PROBE) {
+        q += fabsf(fmaf(-(1.f - 1.f / alpha), fo, g));
+    } else if (mode == SW_STEP) {
+        const float add = alpha * g, add_lo = fmaf(alpha, g, -add), b = 1.f - alpha;
+        const float p = b * fo, p_lo = fmaf(b, fo, -p);
+        float f, e, s, es;
+        two_sum(p, add, f, e);
+        two_sum(yv, add, s, es);
+        yv = __fadd_rn(s, __fadd_rn(es, add_lo));
+        return __fadd_rn(f, __fadd_rn(e, __fadd_rn(p_lo, add_lo)));
+    }
+    yv += g;
+    return g;
 }
 
 // ------------------------------------------------------------------ batched rows: solve
-template <int NQ>
-__device__ __forceinline__ void flush_row(const SolveArgs& a, float4* out, uint32_t v, float4 acc, const float4& bv,
-                                          const float4& ov, uint32_t grp, uint32_t q, float& rr, float& nn) {
-    acc = across_groups<NQ>(acc);
-    const float4 y = affine4(a.d, acc, a.scale_b, bv);
+// The vertex's end: its sum over the lane groups, then the new rows. bv: the source row (VALUE) or the
+// iterate's old row (FIRST: the source row); ov: the old iterate (VALUE) or residual (PROBE, STEP).
+struct SweepEnd {
+    int mode;
+    float alpha;  // STEP: the step length; PROBE: the one measured for
+    float4* out;  // VALUE: iterates; residual form: residuals
+    float4* y;    // residual form: iterates
+};
+template <int NQ, bool RES>
+__device__ __forceinline__ void finish_row(const SolveArgs& a, const SweepEnd& e, uint32_t v, const float4& sum, float4 bv,
+                                           const float4& ov, uint32_t grp, uint32_t q, float& rr, float& nn, float& qq) {
+    if (!RES || e.mode == SW_VALUE) {
+        const float4 y = affine4(a.d, a.d_lo, sum, a.scale_b, a.scale_lo, bv);
+        if (grp == 0) {
+            e.out[(size_t)v * NQ + q] = y;
+            rr += l1diff4(y, ov);
+            nn += l14(y);
+        }
+        return;
+    }
     if (grp == 0) {
-        out[(size_t)v * NQ + q] = y;
-        rr += l1diff4(y, ov);
-        nn += l14(y);
+        float4 f;
+        f.x = res_elem(a, e.mode, e.alpha, sum.x, ov.x, bv.x, qq);
+        f.y = res_elem(a, e.mode, e.alpha, sum.y, ov.y, bv.y, qq);
+        f.z = res_elem(a, e.mode, e.alpha, sum.z, ov.z, bv.z, qq);
+        f.w = res_elem(a, e.mode, e.alpha, sum.w, ov.w, bv.w, qq);
+        e.out[(size_t)v * NQ + q] = f;
+        e.y[(size_t)v * NQ + q] = bv;
+        rr += l14(f);
+        nn += l14(bv);
     }
 }
 
 // 3 CTAs per SM (<= 85 registers, a few spilled): the solve is latency-bound, and 24 warps per SM
 // instead of 16 measured 1.3x faster on R-MAT s20 x 64 columns. NQ = W/4 lanes per row.
-template <int K, int NQ>
+template <int K, int NQ, bool RES>
 __global__ void __launch_bounds__(PPR_TPB, 3) k_ppr_rows(SolveArgs a) {
     constexpr int G = 32 / NQ;               // lane groups (rows per gather instruction)
     constexpr int H = K / G;                 // slots per group per part
@@ -416,87 +493,130 @@ __global__ void __launch_bounds__(PPR_TPB, 3) k_ppr_rows(SolveArgs a) {
     __syncthreads();
     const uint64_t pol = l2_evict_first_policy();
     const float4* b = reinterpret_cast<const float4*>(a.b);
+    __shared__ Extrapolation s_ex;
     uint32_t epoch = 0, s = 0;
     bool conv = false;
+    uint32_t tail = 0;  // residual form: value-form sweeps left before the end
+    if (threadIdx.x == 0) extrapolation_init(s_ex);
     {
         float4* y0 = reinterpret_cast<float4*>(a.y0);
         float4* y1 = reinterpret_cast<float4*>(a.y1);
+        float4* yy = reinterpret_cast<float4*>(a.y);
+        float4* re = reinterpret_cast<float4*>(a.res);
         const uint64_t tot = (uint64_t)a.n * NQ;
         for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < tot;
              i += (uint64_t)gridDim.x * blockDim.x) {
+            if (RES) {  // only the rows no sweep writes: iterate s b, residual 0
+                const uint32_t v = (uint32_t)(i / NQ);
+                if (a.g.vstart[v + 1] != a.g.vstart[v]) continue;
+            }
             const float4 v = b[i];
-            const float4 y = make_float4(a.scale_b * v.x, a.scale_b * v.y, a.scale_b * v.z, a.scale_b * v.w);
-            y0[i] = y;
-            y1[i] = y;
+            const float4 y = affine4(0.f, 0.f, f4(0.f), a.scale_b, a.scale_lo, v);
+            if (RES) {
+                y0[i] = y1[i] = f4(0.f);
+                yy[i] = y;
+            } else {
+                y0[i] = y;
+                y1[i] = y;
+            }
         }
-    }
-    if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) goto finish;
-    for (; s < a.max_iters; ++s) {
-        const float4* in = reinterpret_cast<const float4*>((s & 1u) ? a.y1 : a.y0);
-        float4* out = reinterpret_cast<float4*>((s & 1u) ? a.y0 : a.y1);
-        double dr = 0.0, dn = 0.0;
-        if (threadIdx.x == 0) s_next[(s + 1u) & 1u] = 0u;  // next sweep's; ordered by the sweep's grid barrier
-        for (uint32_t c; (c = next_chunk(&s_next[s & 1u], a.g.nchunks, lane)) != NONE;) {
-            const Chunk ch = a.g.chunk[c];
-            const uint32_t np = ch.p1 - ch.p0;
-            const uint32_t own_l = lane < np ? ld_nc(a.g.vowner + ch.p0 + lane) : NONE;
-            uint32_t cur = __shfl_sync(FULL, own_l, 0);
-            float4 bv = b[(size_t)cur * NQ + q];
-            float4 ov = in[(size_t)cur * NQ + q];
-            float4 acc = f4(0.f);
-            float rr = 0.f, nn = 0.f;
-            for (uint32_t pp = 0; pp < np; pp += U) {
-                uint32_t colg[U][H], wbg[U][H];
-                load_group_slots<K, G>(a.g, ch.p0, pp, np, grp, pol, colg, wbg);
-                float4 xv[U][H];
+        if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) goto finish;
+        for (; s < a.max_iters || tail; ++s) {
+            SweepEnd e;
+            e.mode = SW_VALUE;
+            e.alpha = 1.f;
+            e.out = (s & 1u) ? y0 : y1;
+            e.y = yy;
+            const float4* in = (s & 1u) ? y1 : y0;
+            const float4* own = b;  // the row a vertex's end adds to
+            if (RES && tail) {
+                in = tail == 2u ? yy : y0;
+                e.out = tail == 2u ? y0 : re;
+            } else if (RES) {
+                e.mode = s == 0u ? SW_FIRST : (s_ex.alpha != 1.f ? SW_STEP : (s_ex.cand != 0.f ? SW_PROBE : SW_PLAIN));
+                e.alpha = e.mode == SW_STEP ? s_ex.alpha : s_ex.cand;
+                if (s == 0u) in = b;
+                else own = yy;
+            }
+            // the rows whose old values a vertex's end reads; the other sweeps skip the load
+            const bool want_old = !RES || e.mode == SW_PROBE || e.mode == SW_STEP;
+            double dr = 0.0, dn = 0.0, dq = 0.0;
+            if (threadIdx.x == 0) s_next[(s + 1u) & 1u] = 0u;  // next sweep's; ordered by the sweep's grid barrier
+            for (uint32_t c; (c = next_chunk(&s_next[s & 1u], a.g.nchunks, lane)) != NONE;) {
+                const Chunk ch = a.g.chunk[c];
+                const uint32_t np = ch.p1 - ch.p0;
+                const uint32_t own_l = lane < np ? ld_nc(a.g.vowner + ch.p0 + lane) : NONE;
+                uint32_t cur = __shfl_sync(FULL, own_l, 0);
+                float4 bv = own[(size_t)cur * NQ + q];
+                float4 ov = want_old ? in[(size_t)cur * NQ + q] : f4(0.f);
+                float4 acc = f4(0.f);
+                float rr = 0.f, nn = 0.f, qq = 0.f;
+                for (uint32_t pp = 0; pp < np; pp += U) {
+                    uint32_t colg[U][H], wbg[U][H];
+                    load_group_slots<K, G>(a.g, ch.p0, pp, np, grp, pol, colg, wbg);
+                    float4 xv[U][H];
 #pragma unroll
-                for (int u = 0; u < U; ++u)
+                    for (int u = 0; u < U; ++u)
 #pragma unroll
-                    for (int j = 0; j < H; ++j) {
-                        const uint32_t id = colg[u][j];
-                        xv[u][j] = id != NONE ? in[(size_t)id * NQ + q] : f4(0.f);
-                    }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (pp + u < np) {
-                        const uint32_t o = __shfl_sync(FULL, own_l, pp + u);
-                        if (o != cur) {
-                            flush_row<NQ>(a, out, cur, acc, bv, ov, grp, q, rr, nn);
-                            acc = f4(0.f);
-                            cur = o;
-                            bv = b[(size_t)cur * NQ + q];
-                            ov = in[(size_t)cur * NQ + q];
+                        for (int j = 0; j < H; ++j) {
+                            const uint32_t id = colg[u][j];
+                            xv[u][j] = id != NONE ? in[(size_t)id * NQ + q] : f4(0.f);
                         }
 #pragma unroll
-                        for (int j = 0; j < H; ++j) fma4(acc, __uint_as_float(wbg[u][j]), xv[u][j]);
+                    for (int u = 0; u < U; ++u) {
+                        if (pp + u < np) {
+                            const uint32_t o = __shfl_sync(FULL, own_l, pp + u);
+                            if (o != cur) {
+                                finish_row<NQ, RES>(a, e, cur, across_groups<NQ>(acc), bv, ov, grp, q, rr, nn, qq);
+                                acc = f4(0.f);
+                                cur = o;
+                                bv = own[(size_t)cur * NQ + q];
+                                if (want_old) ov = in[(size_t)cur * NQ + q];
+                            }
+#pragma unroll
+                            for (int j = 0; j < H; ++j) fma4(acc, __uint_as_float(wbg[u][j]), xv[u][j]);
+                        }
                     }
                 }
-            }
-            if (ch.hub == NONE) {
-                flush_row<NQ>(a, out, cur, acc, bv, ov, grp, q, rr, nn);
-            } else {
                 const float4 tot = across_groups<NQ>(acc);
-                float4 full;
-                uint32_t v;
-                if (hub_rows<NQ>(a.g, ch, tot, s + 1, lane, full, v)) {
-                    const float4 y = affine4(a.d, full, a.scale_b, b[(size_t)v * NQ + q]);
-                    if (grp == 0) {
-                        const float4 o = in[(size_t)v * NQ + q];
-                        out[(size_t)v * NQ + q] = y;
-                        rr += l1diff4(y, o);
-                        nn += l14(y);
-                    }
+                if (ch.hub == NONE) {
+                    finish_row<NQ, RES>(a, e, cur, tot, bv, ov, grp, q, rr, nn, qq);
+                } else {
+                    float4 full;
+                    uint32_t v;
+                    if (hub_rows<NQ>(a.g, ch, tot, s + 1, lane, full, v))
+                        finish_row<NQ, RES>(a, e, v, full, own[(size_t)v * NQ + q],
+                                            want_old ? in[(size_t)v * NQ + q] : f4(0.f), grp, q, rr, nn, qq);
+                }
+                dr += (double)rr;
+                dn += (double)nn;
+                if (RES) dq += (double)qq;
+            }
+            if (RES && tail) {  // rows without parts: the value is s b
+                for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < tot;
+                     i += (uint64_t)gridDim.x * blockDim.x) {
+                    const uint32_t v = (uint32_t)(i / NQ);
+                    if (a.g.vstart[v + 1] == a.g.vstart[v]) e.out[i] = yy[i];
+                }
+                if (--tail) {
+                    if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) goto finish;
+                    continue;
+                }
+                conv = true;
+                ++s;
+                break;
+            }
+            const int st = end_sweep<RES>(a, s, dr, dn, dq, e.mode, &s_ex, epoch);
+            if (st == 2) goto finish;
+            if (st == 1) {
+                if (RES) {
+                    tail = 2u;
+                } else {
+                    ++s;
+                    conv = true;
+                    break;
                 }
             }
-            dr += (double)rr;
-            dn += (double)nn;
-        }
-        const int st = end_sweep(a, s, dr, dn, epoch);
-        if (st == 2) goto finish;
-        if (st == 1) {
-            ++s;
-            conv = true;
-            break;
         }
     }
     if (!conv && blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&a.ctrl->bw.status, (uint32_t)DEV_OK, (uint32_t)DEV_ITER_CAP);
@@ -505,7 +625,7 @@ finish:
 }
 
 // ------------------------------------------------------------------ single column: solve
-template <int K>
+template <int K, bool RES>
 __global__ void __launch_bounds__(PPR_TPB, 4) k_ppr_scalar(SolveArgs a) {
     constexpr int PPS = 32 / K;                   // parts per 32-slot step
     constexpr int STEPS = (int)PPR_SLOTS / 32;    // steps per chunk
@@ -514,18 +634,56 @@ __global__ void __launch_bounds__(PPR_TPB, 4) k_ppr_scalar(SolveArgs a) {
     if (threadIdx.x == 0) s_next[0] = s_next[1] = 0u;
     __syncthreads();
     const float* b = a.b;
+    __shared__ Extrapolation s_ex;
     uint32_t epoch = 0, s = 0;
     bool conv = false;
+    uint32_t tail = 0;  // residual form: value-form sweeps left before the end
+    if (threadIdx.x == 0) extrapolation_init(s_ex);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const float y = a.scale_b * b[i];
-        a.y0[i] = y;
-        a.y1[i] = y;
+        if (RES && a.g.vstart[i + 1] != a.g.vstart[i]) continue;  // only the rows no sweep writes
+        const float y = fmaf(a.scale_lo, b[i], a.scale_b * b[i]);
+        if (RES) {
+            a.y0[i] = a.y1[i] = 0.f;
+            a.y[i] = y;
+        } else {
+            a.y0[i] = y;
+            a.y1[i] = y;
+        }
     }
     if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) goto finish;
-    for (; s < a.max_iters; ++s) {
+    for (; s < a.max_iters || tail; ++s) {
         const float* in = (s & 1u) ? a.y1 : a.y0;
         float* out = (s & 1u) ? a.y0 : a.y1;
-        double dr = 0.0, dn = 0.0;
+        const float* own = b;  // the value a vertex's end adds to
+        int mode = SW_VALUE;
+        float alpha = 1.f;
+        if (RES && tail) {
+            in = tail == 2u ? a.y : a.y0;
+            out = tail == 2u ? a.y0 : a.res;
+        } else if (RES) {
+            mode = s == 0u ? SW_FIRST : (s_ex.alpha != 1.f ? SW_STEP : (s_ex.cand != 0.f ? SW_PROBE : SW_PLAIN));
+            alpha = mode == SW_STEP ? s_ex.alpha : s_ex.cand;
+            if (s == 0u) in = b;
+            else own = a.y;
+        }
+        const bool want_old = !RES || mode == SW_PROBE || mode == SW_STEP;
+        double dr = 0.0, dn = 0.0, dq = 0.0;
+        // one vertex's end, by one lane
+        auto finish_one = [&](uint32_t v, float sum, float& rr, float& nn, float& qq) {
+            float ov = want_old ? in[v] : 0.f, bv = own[v];
+            if (!RES || mode == SW_VALUE) {
+                const float y = affine(a.d, a.d_lo, sum, a.scale_b, a.scale_lo, bv);
+                rr += fabsf(y - ov);
+                nn += fabsf(y);
+                out[v] = y;
+            } else {
+                const float f = res_elem(a, mode, alpha, sum, ov, bv, qq);
+                out[v] = f;
+                a.y[v] = bv;
+                rr += fabsf(f);
+                nn += fabsf(bv);
+            }
+        };
         if (threadIdx.x == 0) s_next[(s + 1u) & 1u] = 0u;  // next sweep's; ordered by the sweep's grid barrier
         for (uint32_t c; (c = next_chunk(&s_next[s & 1u], a.g.nchunks, lane)) != NONE;) {
             const Chunk ch = a.g.chunk[c];
@@ -567,36 +725,43 @@ __global__ void __launch_bounds__(PPR_TPB, 4) k_ppr_scalar(SolveArgs a) {
                 const float t = __shfl_up_sync(FULL, psum, o);
                 if (lane >= (uint32_t)o && lane - (uint32_t)o >= start) psum += t;
             }
-            float rr = 0.f, nn = 0.f;
+            float rr = 0.f, nn = 0.f, qq = 0.f;
             if (ch.hub == NONE) {
                 const uint32_t next = __shfl_down_sync(FULL, own_l, 1);
                 const bool lastl = lane < np && (lane == np - 1 || next != own_l);
-                if (lastl) {
-                    const float y = fmaf(a.d, psum, a.scale_b * b[own_l]);
-                    rr += fabsf(y - in[own_l]);
-                    nn += fabsf(y);
-                    out[own_l] = y;
-                }
+                if (lastl) finish_one(own_l, psum, rr, nn, qq);
             } else {
                 const float tot = __shfl_sync(FULL, psum, np - 1);
                 float full;
                 uint32_t v;
-                if (hub_scalar(a.g, ch, tot, s + 1, lane, full, v) && lane == 0) {
-                    const float y = fmaf(a.d, full, a.scale_b * b[v]);
-                    rr += fabsf(y - in[v]);
-                    nn += fabsf(y);
-                    out[v] = y;
-                }
+                if (hub_scalar(a.g, ch, tot, s + 1, lane, full, v) && lane == 0) finish_one(v, full, rr, nn, qq);
             }
             dr += (double)rr;
             dn += (double)nn;
+            if (RES) dq += (double)qq;
         }
-        const int st = end_sweep(a, s, dr, dn, epoch);
+        if (RES && tail) {  // rows without parts: the value is s b
+            for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
+                 i += (uint64_t)gridDim.x * blockDim.x)
+                if (a.g.vstart[i + 1] == a.g.vstart[i]) out[i] = a.y[i];
+            if (--tail) {
+                if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) goto finish;
+                continue;
+            }
+            conv = true;
+            ++s;
+            break;
+        }
+        const int st = end_sweep<RES>(a, s, dr, dn, dq, mode, &s_ex, epoch);
         if (st == 2) goto finish;
         if (st == 1) {
-            ++s;
-            conv = true;
-            break;
+            if (RES) {
+                tail = 2u;
+            } else {
+                ++s;
+                conv = true;
+                break;
+            }
         }
     }
     if (!conv && blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&a.ctrl->bw.status, (uint32_t)DEV_OK, (uint32_t)DEV_ITER_CAP);
@@ -843,8 +1008,8 @@ struct eeg_ppr {
     float* w_raw = nullptr;  // m
     float* s = nullptr;      // n
     uint32_t* bad = nullptr;
-    float* Y[2] = {nullptr, nullptr};  // forward iterates
-    float* Lb[2] = {nullptr, nullptr}; // adjoint iterates
+    float* Y[2] = {nullptr, nullptr};  // forward iterates (X in one of them until the next forward)
+    float* Lb[2] = {nullptr, nullptr}; // adjoint iterates; residuals of the solves in residual form
     float* b = nullptr;                // staged input rows (n x W)
     float* gslot = nullptr;            // forward slots
     float* r = nullptr;                // n
@@ -945,6 +1110,7 @@ DirTab tab(const VDir& vd, const PPRDir& d) {
     t.harrive = d.harrive;
     t.partial = d.partial;
     t.gpartial = d.gpartial;
+    t.vstart = vd.vstart;
     return t;
 }
 
@@ -971,12 +1137,12 @@ eeg_status launch_coop(Kern kern, void* arg, int device, uint32_t bps, uint64_t 
     return EEG_OK;
 }
 
-template <int K>
+template <int K, bool RES>
 eeg_status launch_solve(eeg_ppr* p, SolveArgs& a, uint32_t bps, cudaStream_t st) {
     const uint64_t work = std::max<uint64_t>(a.g.nchunks, ((uint64_t)a.n * 16 + 31) / 32);
-    if (p->W == 1) return launch_coop(k_ppr_scalar<K>, &a, p->vg->device, bps, work, st);
-    if (p->W == 32) return launch_coop(k_ppr_rows<K, 8>, &a, p->vg->device, bps, work, st);
-    return launch_coop(k_ppr_rows<K, 16>, &a, p->vg->device, bps, work, st);
+    if (p->W == 1) return launch_coop(k_ppr_scalar<K, RES>, &a, p->vg->device, bps, work, st);
+    if (p->W == 32) return launch_coop(k_ppr_rows<K, 8, RES>, &a, p->vg->device, bps, work, st);
+    return launch_coop(k_ppr_rows<K, 16, RES>, &a, p->vg->device, bps, work, st);
 }
 
 template <int K>
@@ -1021,12 +1187,12 @@ eeg_status unstage_rows(eeg_ppr* p, const float* src, float* dst, int on_device,
     return EEG_OK;
 }
 
+// X = p->Y[p->xi] is kept by an adjoint solve. *result: the buffer holding the solution.
 eeg_status solve(eeg_ppr* p, bool adjoint, const float* bsrc, const eeg_options& o, cudaStream_t st,
-                 eeg_result* res, int* which) {
+                 eeg_result* res, float** result) {
     eeg_vgraph* vg = p->vg;
     const VDir& vd = adjoint ? vg->fwd : vg->rev;
     PPRDir& d = adjoint ? p->fwd : p->rev;
-    float** Y = adjoint ? p->Lb : p->Y;
     const float damping = o.pr_damping > 0.f ? o.pr_damping : 0.85f;
     SolveArgs a{};
     a.g = tab(vd, d);
@@ -1034,24 +1200,48 @@ eeg_status solve(eeg_ppr* p, bool adjoint, const float* bsrc, const eeg_options&
     a.b = bsrc;
     a.scale_b = adjoint ? 1.0f : 1.0f - damping;
     a.d = damping;
-    a.y0 = Y[0];
-    a.y1 = Y[1];
+    const bool res_form = o.max_iterations == 0;
+    if (res_form) {
+        const double d64 = o.pr_damping > 0.f ? (double)o.pr_damping : 0.85, s64 = adjoint ? 1.0 : 1.0 - d64;
+        a.d_lo = (float)(d64 - (double)a.d);
+        a.scale_b = (float)s64;
+        a.scale_lo = (float)(s64 - (double)a.scale_b);
+    }
+    if (!res_form) {
+        a.y0 = adjoint ? p->Lb[0] : p->Y[0];
+        a.y1 = adjoint ? p->Lb[1] : p->Y[1];
+    } else if (!adjoint) {  // residuals in the adjoint's buffers
+        a.y0 = p->Lb[0];
+        a.y1 = p->Lb[1];
+        a.y = p->Y[0];
+        a.res = p->Y[1];
+    } else {  // the forward's other buffer is free
+        a.y0 = p->Y[p->xi ^ 1];
+        a.y1 = p->Lb[0];
+        a.y = p->Lb[1];
+        a.res = p->Lb[0];
+    }
     a.ctrl = p->ctrl;
     a.max_iters = o.max_iterations ? o.max_iterations : 10000u;
     a.tol = o.pr_tolerance > 0.f ? (double)o.pr_tolerance : 1e-7;
     a.timeout_ns = wait_limit_ns(o);
     EEG_CUDA(cudaMemsetAsync(p->ctrl, 0, sizeof(PRCtrl), st));
     EEG_TRY(reset_counters(d, st));
+#define EEG_PPR_SOLVE(KV) \
+    EEG_TRY(res_form ? (launch_solve<KV, true>(p, a, o.blocks_per_sm, st)) : (launch_solve<KV, false>(p, a, o.blocks_per_sm, st)))
     switch (vg->K) {
-        case 4: EEG_TRY(launch_solve<4>(p, a, o.blocks_per_sm, st)); break;
-        case 8: EEG_TRY(launch_solve<8>(p, a, o.blocks_per_sm, st)); break;
-        case 16: EEG_TRY(launch_solve<16>(p, a, o.blocks_per_sm, st)); break;
+        case 4: EEG_PPR_SOLVE(4); break;
+        case 8: EEG_PPR_SOLVE(8); break;
+        case 16: EEG_PPR_SOLVE(16); break;
         default: set_last_error("K must be 4, 8 or 16"); return EEG_ERR_UNSUPPORTED;
     }
+#undef EEG_PPR_SOLVE
     PRCtrl hc;
     EEG_CUDA(cudaMemcpyAsync(&hc, p->ctrl, sizeof(PRCtrl), cudaMemcpyDeviceToHost, st));
     EEG_CUDA(cudaStreamSynchronize(st));
-    *which = (int)(hc.iterations & 1u);
+    // residual form, cap of 10000 sweeps reached: the iterate as it stands
+    if (!res_form) *result = (hc.iterations & 1u) ? a.y1 : a.y0;
+    else *result = hc.bw.status == DEV_ITER_CAP ? a.y : a.res;
     const double m = (double)vg->m, n = (double)vg->n;
     res->iterations += hc.iterations;
     res->pr_residual = hc.last_resid;
@@ -1188,11 +1378,11 @@ EEG_API eeg_status eeg_ppr_forward(eeg_ppr* p, const float* teleport, int in_on_
     const float* bsrc = nullptr;
     EEG_CUDA(cudaEventRecord(p->ev[0], st));
     EEG_TRY(stage_rows(p, teleport, in_on_device, st, &bsrc));
-    int which = 0;
-    eeg_status s = solve(p, false, bsrc, o, st, &r, &which);
+    float* X = nullptr;
+    eeg_status s = solve(p, false, bsrc, o, st, &r, &X);
     if (s != EEG_OK && s != EEG_ERR_ITER_CAP) return s;
-    p->xi = which;
-    if (x_out) EEG_TRY(unstage_rows(p, p->Y[which], x_out, out_on_device, st));
+    p->xi = X == p->Y[1] ? 1 : 0;
+    if (x_out) EEG_TRY(unstage_rows(p, X, x_out, out_on_device, st));
     EEG_CUDA(cudaEventRecord(p->ev[1], st));
     EEG_CUDA(cudaEventSynchronize(p->ev[1]));
     float ms = 0.f;
@@ -1228,10 +1418,9 @@ EEG_API eeg_status eeg_ppr_adjoint(eeg_ppr* p, const float* dl_dx, int in_on_dev
     const float* bsrc = nullptr;
     EEG_CUDA(cudaEventRecord(p->ev[0], st));
     EEG_TRY(stage_rows(p, dl_dx, in_on_device, st, &bsrc));
-    int which = 0;
-    eeg_status s = solve(p, true, bsrc, o, st, &r, &which);
+    float* L = nullptr;
+    eeg_status s = solve(p, true, bsrc, o, st, &r, &L);
     if (s != EEG_OK && s != EEG_ERR_ITER_CAP) return s;
-    const float* L = p->Lb[which];
     // edge gradients
     GradArgs g{};
     g.g = tab(vg->fwd, p->fwd);
@@ -1273,7 +1462,8 @@ EEG_API eeg_status eeg_ppr_adjoint(eeg_ppr* p, const float* dl_dx, int in_on_dev
         const bool direct = out_on_device && p->C == p->W;
         if (!direct && !p->stage_nw) EEG_TRY(ppr_alloc(p, (void**)&p->stage_nw, sizeof(float) * cnt));
         float* dst = direct ? dl_dteleport : p->stage_nw;
-        k_ppr_scale<<<grid_1d(cnt, vg->device), PPR_TPB, 0, st>>>(cnt, 1.0f - damping, L, dst);
+        const float s32 = o.pr_damping > 0.f ? (float)(1.0 - (double)o.pr_damping) : (float)0.15;
+        k_ppr_scale<<<grid_1d(cnt, vg->device), PPR_TPB, 0, st>>>(cnt, s32, L, dst);
         EEG_CUDA(cudaGetLastError());
         r.launches += 1;
         if (!direct) EEG_TRY(unstage_rows(p, dst, dl_dteleport, out_on_device, st));

@@ -68,3 +68,49 @@ def test_pagerank_capped_runs_keep_the_plain_iterates(gpu, name):
                 want = 0.15 + 0.85 * np.bincount(d, weights=(want / np.maximum(deg, 1))[s], minlength=n)
             err = np.abs(x - want).sum() / want.sum()
             assert err <= 2.0 ** -24 * (1 + 4 / 0.15), (k, err)
+
+
+@pytest.mark.parametrize("C", [1, 5, 32, 64])
+@pytest.mark.parametrize("K", [4, 8, 16])
+@pytest.mark.parametrize("name", NAMES)
+def test_ppr_extrapolated(gpu, name, K, C):
+    """Forward and adjoint in residual form against the 64-bit oracle, in the norm of the solve's own bound
+    (L1 over all columns). The adjoint's rows, not its columns, sum to at most 1, so its L1 error may exceed
+    the bound by the condition of the L1 norm: it is compared in the maximum norm, where the tolerance holds
+    up to the norms' ratio on the residual (at most the number of entries), reached on none of these graphs:
+    1e-5 of the largest entry."""
+    n, s, d = _graph(gpu, name)
+    rng = np.random.default_rng(3)
+    w = rng.uniform(0.1, 1, s.size).astype(np.float32)
+    T = rng.uniform(0, 1, (n, C)).astype(np.float32)
+    G = rng.standard_normal((n, C)).astype(np.float32)
+    X_ref, _ = oracle.ppr_solve(n, s, d, w, T)
+    L_ref, _ = oracle.ppr_solve(n, s, d, w, G, transpose=True)
+    with gpu.VirtualGraph.build(n, s, d, None, K=K, reverse=True, edge_ids=True) as vg, gpu.PPR(vg, C) as p:
+        p.set_weights(w)
+        X, _ = p.forward(T)
+        out, _ = p.adjoint(G)
+        again, _ = p.adjoint(G)  # the forward's solution survives an adjoint solve
+        assert np.array_equal(out["dt"], again["dt"]) and np.array_equal(out["dw"], again["dw"])
+    # FP32 weights normalised in FP32 (relative 2^-23), long row sums (star: up to 1500 terms, each addition
+    # 2^-24 of the running sum, of random sign: a factor of 8 covers sqrt(1500) / 5), amplified by 1/(1-d)
+    bound = 1e-7 + 8 * 2.0 ** -24 / 0.15
+    assert np.abs(X - X_ref).sum() <= bound * np.abs(X_ref).sum()
+    assert np.abs(out["dt"] - 0.15 * L_ref).max() <= 1e-5 * np.abs(0.15 * L_ref).max()
+
+
+def test_ppr_capped_runs_keep_the_plain_iterates(gpu):
+    n, s, d = _graph(gpu, "rmat")
+    rng = np.random.default_rng(4)
+    w = rng.uniform(0.1, 1, s.size).astype(np.float32)
+    T = rng.uniform(0, 1, (n, 3)).astype(np.float32)
+    wn = w / np.bincount(s, weights=w, minlength=n)[s]
+    with gpu.VirtualGraph.build(n, s, d, None, K=8, reverse=True, edge_ids=True) as vg, gpu.PPR(vg, 3) as p:
+        p.set_weights(w)
+        for k in (1, 6):
+            X, res = p.forward(T, max_iterations=k, check=False)
+            assert res["status"] == gpu.ERR_ITER_CAP and res["iterations"] == k
+            want = 0.15 * T.astype(np.float64)
+            for _ in range(k):
+                want = 0.15 * T + 0.85 * np.stack([np.bincount(d, weights=wn * want[s, c], minlength=n) for c in range(3)], 1)
+            assert np.abs(X - want).sum() <= 8 * 2.0 ** -24 / 0.15 * want.sum()
