@@ -90,7 +90,9 @@ struct PRDDCtrl {
     unsigned long long pushes;    // edge pushes over the run
     unsigned long long parts;     // parts expanded over the run
     unsigned long long consumed;  // residuals taken (vertex activations) over the run
-    double resid;        // sum of the residuals left at the end (error bound: resid / (1-d))
+    double rsum[3];      // long steps: residuals taken per round (L1), and the probe (rotating)
+    double probe[3];
+    double resid;        // L1 norm of the residuals left at the end (error bound: resid / (1-d))
     double norm;         // sum of the values at the end
 };
 
@@ -119,6 +121,7 @@ struct Workspace {
     double* dd_r = nullptr;       // n: residuals
     double* dd_x = nullptr;       // n: values (FP64 accumulation; the output is written to x)
     double* dd_amt = nullptr;     // n: push amount of each vertex activated in the current round
+    double* dd_taken = nullptr;   // n: residual each vertex took in the last round (long steps)
     uint32_t* dd_pq = nullptr;    // P: part queue of the current round
     PRDDCtrl* ddctrl = nullptr;
     // misc

@@ -23,6 +23,13 @@
 // would not hold the 1e-6 L1 bound); the output is FP32. Tracking which pushes lift a residual past acc
 // instead of scanning needs the atomics' old values: 25 % slower on R-MAT s22 (154.6 against 123.4 ms),
 // every returning FP64 atomic a long-scoreboard wait.
+// Long steps (runs without --accuracy and without a round cap): a round is a Jacobi sweep in residual form
+// on the active vertices, and with the threshold derived from the tolerance nearly all of them stay
+// active for ~135 rounds of 0.84 each. So phase A also sums the taken residuals and compares them with
+// the last round's (the control of common.cuh, whose evidence here is one round old when the step is
+// taken); a round with step length alpha adds alpha t to the value, keeps (1 - alpha) t as residual and
+// pushes alpha times the amount. Residuals may then be negative: |r| is compared with acc. R-MAT s17,
+// K = 8: 10.5 -> 2.3 ms.
 // The reference's two DD kernels differ only in when a vertex's label is cleared (in the kernel that
 // processes it, or by clearLabel after it); with the residual taken once per round in a phase of its
 // own that makes no difference, so SYNC_PUSH_DD and ASYNC_PUSH_DD run these same rounds.
@@ -45,6 +52,7 @@ struct DDArgs {
     double* r;
     double* xv;
     double* amt;
+    double* taken;  // long steps: the residual each vertex had taken in the last round (0 = inactive)
     float* x;
     uint32_t* pq;
     PRDDCtrl* ctrl;
@@ -52,6 +60,7 @@ struct DDArgs {
     double damping;
     double base;
     uint32_t max_iters;
+    uint32_t accel;  // long steps
     uint64_t timeout_ns;
 };
 
@@ -98,6 +107,9 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
     uint32_t epoch = 0;
     uint32_t it = 0;
     unsigned long long my_pushes = 0, my_parts = 0, my_taken = 0;
+    __shared__ Extrapolation s_ex;
+    bool stepped = false;  // the last round took a long step
+    if (threadIdx.x == 0) extrapolation_init(s_ex);
 
     for (uint32_t v = gtid; v < a.n; v += gthreads) {
         a.r[v] = a.base;
@@ -112,20 +124,34 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
                 atomicCAS(&ctrl->bw.status, (uint32_t)DEV_OK, (uint32_t)DEV_ITER_CAP);
             break;
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->plen[nxt] = 0u;  // last read in round it-2
+        if (blockIdx.x == 0 && threadIdx.x == 0) {  // last read in round it-2
+            ctrl->plen[nxt] = 0u;
+            ctrl->rsum[nxt] = 0.0;
+            ctrl->probe[nxt] = 0.0;
+        }
+        const double alpha = (double)s_ex.alpha;
+        const double rho = s_ex.cand != 0.f ? 1.0 - 1.0 / (double)s_ex.cand : 0.0;  // measured for when not 0
+        double rs = 0.0, qs = 0.0;
         // ---- phase A: every vertex whose residual exceeds acc takes it (a dense scan of the residuals)
         for (uint32_t b0 = gwarp * 32u; b0 < a.n; b0 += nwarps * 32u) {
             const uint32_t v = b0 + lane;
             uint32_t s0 = 0, np = 0;
             if (v < a.n) {
                 const double t = __ldcg(&a.r[v]);
-                if (t > a.acc) {
-                    a.r[v] = 0.0;
-                    a.xv[v] = __ldcg(&a.xv[v]) + t;
+                const bool act = fabs(t) > a.acc;
+                if (a.accel) {
+                    const double tk = act ? t : 0.0;
+                    if (rho != 0.0) qs += fabs(tk - rho * a.taken[v]);
+                    a.taken[v] = tk;
+                    rs += fabs(tk);
+                }
+                if (act) {
+                    a.r[v] = (1.0 - alpha) * t;
+                    a.xv[v] = __ldcg(&a.xv[v]) + alpha * t;
                     ++my_taken;
                     const uint32_t d = __ldg(&a.deg[v]);
                     if (d) {
-                        a.amt[v] = a.damping * t / (double)d;
+                        a.amt[v] = a.damping * (alpha * t) / (double)d;
                         s0 = __ldg(&a.vstart[v]);
                         np = __ldg(&a.vstart[v + 1]) - s0;
                     }
@@ -133,8 +159,43 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
             }
             append_parts(s0, np, &ctrl->plen[cur], a.pq, a.P, lane);
         }
+        if (a.accel) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                rs += __shfl_down_sync(0xffffffffu, rs, off);
+                qs += __shfl_down_sync(0xffffffffu, qs, off);
+            }
+            if (lane == 0) {
+                s_red[0][threadIdx.x >> 5] = rs;
+                s_red[1][threadIdx.x >> 5] = qs;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                double r2 = 0.0, q2 = 0.0;
+                for (int w = 0; w < DD_TPB / 32; ++w) {
+                    r2 += s_red[0][w];
+                    q2 += s_red[1][w];
+                }
+                atomicAdd(&ctrl->rsum[cur], r2);
+                if (rho != 0.0) atomicAdd(&ctrl->probe[cur], q2);
+            }
+        }
         if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) break;
-        if (threadIdx.x == 0) s_len = ld_relaxed(&ctrl->plen[cur]);
+        if (threadIdx.x == 0) {
+            s_len = ld_relaxed(&ctrl->plen[cur]);
+            if (a.accel) {
+                const double rt = __ldcg(&ctrl->rsum[cur]);
+                if (alpha != 1.0) {  // this round takes the step: rt is the residual before it
+                    s_ex.alpha = 1.f;
+                    s_ex.r_before = rt;
+                    s_ex.r_prev = 0.0;
+                } else {
+                    if (stepped && !(rt <= s_ex.r_before)) s_ex.off = 1u;
+                    extrapolation_next(s_ex, rt, __ldcg(&ctrl->probe[cur]), a.damping);
+                }
+            }
+        }
+        stepped = alpha != 1.0;
         __syncthreads();
         uint32_t npq = s_len;
         __syncthreads();
@@ -170,7 +231,7 @@ finish:
         for (uint32_t v = gtid; v < a.n; v += gthreads) {
             const double xv = __ldcg(&a.xv[v]);
             a.x[v] = (float)xv;
-            rs += __ldcg(&a.r[v]);
+            rs += fabs(__ldcg(&a.r[v]));
             xs += xv;
         }
 #pragma unroll
@@ -243,6 +304,9 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
     if (!ws.dd_r) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_r, sizeof(double) * n));
     if (!ws.dd_x) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_x, sizeof(double) * n));
     if (!ws.dd_amt) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_amt, sizeof(double) * n));
+    // long steps: the threshold and the schedule are the library's own (no --accuracy, no round cap)
+    const bool accel = !(o.pr_accuracy > 0.f) && o.max_iterations == 0;
+    if (accel && !ws.dd_taken) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_taken, sizeof(double) * n));
     if (!ws.dd_pq) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_pq, sizeof(uint32_t) * P));
     if (!ws.ddctrl) EEG_CUDA(cudaMalloc((void**)&ws.ddctrl, sizeof(PRDDCtrl)));
     if (!ws.ev[0]) {
@@ -262,6 +326,8 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
     a.r = ws.dd_r;
     a.xv = ws.dd_x;
     a.amt = ws.dd_amt;
+    a.taken = ws.dd_taken;
+    a.accel = accel ? 1u : 0u;
     a.x = ws.x;
     a.pq = ws.dd_pq;
     a.ctrl = ws.ddctrl;

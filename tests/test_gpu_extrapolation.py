@@ -54,6 +54,23 @@ def test_pagerank_extrapolated(gpu, name, K, damping):
             assert err <= bound, (name, variant, err, bound)
 
 
+@pytest.mark.parametrize("damping", [0.0, 0.5, 0.99])
+@pytest.mark.parametrize("K", [4, 8, 16])
+@pytest.mark.parametrize("name", NAMES)
+def test_pagerank_dd_extrapolated(gpu, name, K, damping):
+    """Data-driven: FP64 residuals all end at most tol (1-d)^2, so the relative L1 error is at most tol
+    (every value is at least 1-d), plus the FP32 rounding of the output."""
+    n, s, d = _graph(gpu, name)
+    dd = float(np.float32(damping)) if damping else 0.85
+    want, _ = oracle.pagerank(n, s, d, damping=dd)
+    with gpu.VirtualGraph.build(n, s, d, None, K=K) as vg:
+        for variant in ("sync_push_dd", "async_push_dd"):
+            x, res = vg.run("pr", variant, pr_damping=damping)
+            err = np.abs(x.astype(np.float64) - want).sum() / np.abs(want).sum()
+            assert err <= 1e-7 + 2.0 ** -24, (name, variant, err)
+            assert res["pr_residual"] <= n * 1e-7 * (1 - dd) ** 2 * 1.0001
+
+
 @pytest.mark.parametrize("name", ["rmat", "grid", "star"])
 def test_pagerank_capped_runs_keep_the_plain_iterates(gpu, name):
     """max_iterations = k: status ITER_CAP and the k-th Jacobi iterate (FP32 rounding of k sweeps)."""
