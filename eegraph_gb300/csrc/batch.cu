@@ -27,6 +27,12 @@ namespace eeg {
 namespace batch {
 
 constexpr int B_TPB = 512;
+// slots whose atomics are issued together in this kernel (single-query kernel: 4): what its 64 registers
+// hold with the query's pointers
+template <int OP>
+__device__ constexpr int atomic_group() {
+    return OP == OP_SSWP ? 2 : 4;
+}
 
 struct BGraph {
     uint32_t n, P, K, pad;
@@ -178,7 +184,7 @@ __device__ __noinline__ uint32_t run_query(const BArgs& a, const BGraph& g, cons
             // the atomics of a group of slots go out before any of their results is used; a won claim
             // on the round stamp means the target improved in this round (by this lane or after its
             // filter read), so the winner appends it (the single-query kernel's rule)
-            constexpr int ATB = K < trav::atomic_group<OP>() ? K : trav::atomic_group<OP>();
+            constexpr int ATB = K < atomic_group<OP>() ? K : atomic_group<OP>();
 #pragma unroll
             for (int i0 = 0; i0 < K; i0 += ATB) {
                 uint32_t prev[ATB], ex[ATB];
@@ -212,7 +218,7 @@ __device__ __noinline__ uint32_t run_query(const BArgs& a, const BGraph& g, cons
                     if (mask) {
                         const uint32_t c = __popc(mask);
                         if (wcnt + c > (uint32_t)trav::WCAP) {
-                            trav::warp_append(g.vstart, &ctrl->qparts[nxt], nullptr, wbuf, wcnt, qnext, lane, g.P);
+                            trav::warp_append(g.vstart, &ctrl->qparts[nxt], wbuf, wcnt, qnext, lane, g.P);
                             wcnt = 0;
                         }
                         if (claim) wbuf[wcnt + __popc(mask & lanemask_lt)] = t;
@@ -221,7 +227,7 @@ __device__ __noinline__ uint32_t run_query(const BArgs& a, const BGraph& g, cons
                 }
             }
         }
-        if (wcnt) trav::warp_append(g.vstart, &ctrl->qparts[nxt], nullptr, wbuf, wcnt, qnext, lane, g.P);
+        if (wcnt) trav::warp_append(g.vstart, &ctrl->qparts[nxt], wbuf, wcnt, qnext, lane, g.P);
         if (!team.sync()) return ABORTED;
     }
     // every CTA has read the final (empty) queue length before the leader initialises the next query

@@ -50,8 +50,11 @@ struct VDir {
 // Control block of the traversal kernel (device memory).
 struct TravCtrl {
     BarrierWords bw;
-    uint32_t qparts[3];   // parts enqueued per round (rotating; TD: improvement flag)
-    uint32_t qverts[3];   // vertices enqueued per round (rotating)
+    // per round (rotating): low word = parts enqueued for it (TD: CTAs that improved a value), high word =
+    // CTAs that have finished the round before it (its top bit: the grid is aborting)
+    unsigned long long queued[3];
+    uint32_t qverts[3];   // vertices enqueued (kept where the pull decision or the activity log needs it)
+    uint32_t pad0;
     uint32_t iterations;
     uint32_t done;        // the traversal reached its end (fixed point, cap or abort)
     unsigned long long parts_processed;
@@ -66,6 +69,7 @@ struct TravCtrl {
     uint32_t lcnt[3];
     uint32_t pull_rounds;
 };
+static_assert(sizeof(TravCtrl) == 256, "eeg_run_noalloc's documented scratch size counts 256 bytes for it");
 
 // Control block of the PageRank kernels.
 struct PRCtrl {

@@ -71,14 +71,14 @@ struct TravArgs {
     uint32_t cc_zero;      // CC: relax with weight 0 (connected components)
 };
 
-// The weights of part p (CC in connected-components mode: zeros, nothing loaded).
+// K weights from slot `at` on (CC in connected-components mode: zeros, nothing loaded).
 template <int OP, int K>
-__device__ __forceinline__ void load_weights(const TravArgs& a, uint32_t p, uint32_t (&wt)[K], uint64_t pol) {
+__device__ __forceinline__ void load_weights(const TravArgs& a, size_t at, uint32_t (&wt)[K], uint64_t pol) {
     if (OP == OP_CC && a.cc_zero) {
 #pragma unroll
         for (int i = 0; i < K; ++i) wt[i] = 0u;
     } else {
-        ld_part<K>(a.vw + (size_t)p * K, wt, pol);
+        ld_part<K>(a.vw + at, wt, pol);
     }
 }
 
@@ -95,13 +95,10 @@ __device__ __forceinline__ bool unreached(uint32_t d) {
     return false;
 }
 // Slots whose atomics are issued together (value atomic + claim, 2 returned values each) under a
-// 64-register budget (512-thread CTAs; the batch kernel): the most that fits without slowing the kernel
-// -- measured on R-MAT s22 with K = 8, groups of 4 for BFS and SSSP (0.39 / 0.75 ms; 2: 0.40 / 0.77),
-// 2 for SSWP and CC (0.73 / 1.30 ms; 4 spilled registers: 0.80 / 1.50; 1: 0.76 / 1.34).
-template <int OP>
-__host__ __device__ constexpr int atomic_group() {
-    return (OP == OP_SSWP || OP == OP_CC) ? 2 : 4;
-}
+// 64-register budget (512-thread CTAs): 4. R-MAT s22, K = 8: SSSP 0.636 ms (2: 0.650), SSWP 0.676 (2:
+// 0.717), CC 1.09 (2: 1.11); 8 spills 90 bytes. Bucketed rounds keep their far-buffer state in registers
+// too and take 2 (4 spills 96 bytes: 5.95 against 5.84 ms on the 4096^2 grid).
+constexpr int ATOMIC_GROUP = 4;
 
 template <int OP>
 __device__ __forceinline__ uint32_t relax_value(uint32_t d, uint32_t w) {
@@ -120,16 +117,13 @@ __device__ __forceinline__ uint32_t atomic_improve(uint32_t* p, uint32_t v) {
 }
 
 constexpr int WCAP = 256;  // per-warp append buffer (claimed vertices) before a flush to the queue
+constexpr int FCAP = 128;  // per-warp buffer of far vertices (bucketed rounds) before a flush to the pile
 constexpr uint32_t PULL_LANE = 4;  // BFS pull rounds: parts a lane walks alone before the warp takes over
 
-// Warp-cooperative append of the warp's claimed vertices to the next queue: one reservation per flush
-// (atomicAdd of the parts total), then every claimed vertex's part ids are written; a vertex with more
-// than 32 parts is written by the whole warp. Called by all 32 lanes with a warp-uniform `cnt`.
-// Entries at or beyond `cap` are not written (each vertex is claimed once per round, so a round never
-// produces more than `cap` = the number of parts; the reader clamps and reports an overflow).
-__device__ __forceinline__ void warp_append(const uint32_t* __restrict__ vstart, uint32_t* parts_ctr,
-                                            uint32_t* verts_ctr, const uint32_t* buf, uint32_t cnt, uint32_t* qnext,
-                                            uint32_t lane, uint32_t cap) {
+// Lane's share of the parts of the buffered vertices: returns the warp's total, *before = the parts of the
+// lanes below. Called by all 32 lanes with a warp-uniform `cnt`.
+__device__ __forceinline__ uint32_t warp_parts(const uint32_t* __restrict__ vstart, const uint32_t* buf, uint32_t cnt,
+                                               uint32_t lane, uint32_t* before) {
     __syncwarp();
     uint32_t sum = 0;
     for (uint32_t e = lane; e < cnt; e += 32u) {
@@ -142,14 +136,16 @@ __device__ __forceinline__ void warp_append(const uint32_t* __restrict__ vstart,
         const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
         if (lane >= (uint32_t)off) inc += y;
     }
-    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-    uint32_t base = 0;
-    if (lane == 0) {
-        if (total) base = atomicAdd(parts_ctr, total);
-        if (verts_ctr) atomicAdd(verts_ctr, cnt);
-    }
-    base = __shfl_sync(0xffffffffu, base, 0);
-    uint32_t pos = base + inc - sum;
+    *before = inc - sum;
+    return __shfl_sync(0xffffffffu, inc, 31);
+}
+
+// The part ids of the buffered vertices, from `pos` (this lane's) on; a vertex with more than 32 parts is
+// written by the whole warp. Entries at or beyond `cap` are not written (each vertex is claimed once per
+// round, so a round never produces more than `cap` = the number of parts; the reader clamps and reports
+// an overflow).
+__device__ __forceinline__ void warp_write(const uint32_t* __restrict__ vstart, const uint32_t* buf, uint32_t cnt,
+                                           uint32_t pos, uint32_t* qnext, uint32_t lane, uint32_t cap) {
     const uint32_t rounds = (cnt + 31u) / 32u;
     for (uint32_t k = 0; k < rounds; ++k) {
         const uint32_t e = k * 32u + lane;
@@ -177,9 +173,132 @@ __device__ __forceinline__ void warp_append(const uint32_t* __restrict__ vstart,
     __syncwarp();
 }
 
+// Warp-cooperative append of the warp's claimed vertices to the next queue: one reservation per flush,
+// then every claimed vertex's part ids are written. Called by all 32 lanes with a warp-uniform `cnt`.
+__device__ __forceinline__ void warp_append(const uint32_t* __restrict__ vstart, uint32_t* parts_ctr, const uint32_t* buf,
+                                            uint32_t cnt, uint32_t* qnext, uint32_t lane, uint32_t cap) {
+    uint32_t before;
+    const uint32_t total = warp_parts(vstart, buf, cnt, lane, &before);
+    uint32_t base = 0;
+    if (lane == 0 && total) base = atomicAdd(parts_ctr, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    warp_write(vstart, buf, cnt, base + before, qnext, lane, cap);
+}
+
+// The same within a round of k_traverse (a full buffer).
 __device__ __forceinline__ void warp_flush(const TravArgs& a, const uint32_t* buf, uint32_t cnt, uint32_t* qnext,
-                                           uint32_t nxt, uint32_t lane) {
-    warp_append(a.vstart, &a.ctrl->qparts[nxt], &a.ctrl->qverts[nxt], buf, cnt, qnext, lane, a.P);
+                                           uint32_t nxt, bool count_verts, uint32_t lane) {
+    uint32_t before;
+    const uint32_t total = warp_parts(a.vstart, buf, cnt, lane, &before);
+    uint32_t base = 0;
+    if (lane == 0) {
+        base = (uint32_t)atomicAdd(&a.ctrl->queued[nxt], (unsigned long long)total);
+        if (count_verts) atomicAdd(&a.ctrl->qverts[nxt], cnt);
+    }
+    base = __shfl_sync(0xffffffffu, base, 0);
+    warp_write(a.vstart, buf, cnt, base + before, qnext, lane, a.P);
+}
+
+// End of a round: what the CTA's warps still hold, in one reservation per CTA (with one per warp, and the
+// vertices counted always, BFS on the 4096^2 grid took 2.24 ms, against 2.07). Called by all threads.
+template <int NW>
+__device__ __forceinline__ void cta_flush(const TravArgs& a, const uint32_t* buf, uint32_t cnt, uint32_t* qnext,
+                                          uint32_t nxt, bool count_verts, uint32_t lane, uint2* s_tot) {
+    const uint32_t warp = threadIdx.x >> 5;
+    uint32_t before = 0, total = 0;
+    if (cnt) total = warp_parts(a.vstart, buf, cnt, lane, &before);
+    if (lane == 0) s_tot[warp] = make_uint2(total, cnt);
+    __syncthreads();
+    if (warp == 0) {
+        uint2 t = lane < NW ? s_tot[lane] : make_uint2(0u, 0u);
+        uint32_t inc = t.x;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= (uint32_t)off) inc += y;
+        }
+        const uint32_t verts = __reduce_add_sync(0xffffffffu, t.y);
+        uint32_t base = 0;
+        if (lane == 31u && verts) {
+            base = (uint32_t)atomicAdd(&a.ctrl->queued[nxt], (unsigned long long)inc);
+            if (count_verts) atomicAdd(&a.ctrl->qverts[nxt], verts);
+        }
+        base = __shfl_sync(0xffffffffu, base, 31);
+        if (lane < NW) s_tot[lane].x = base + inc - t.x;
+    }
+    __syncthreads();
+    if (cnt) warp_write(a.vstart, buf, cnt, s_tot[warp].x + before, qnext, lane, a.P);
+}
+
+// Bucketed rounds, a warp's buffered far vertices: all flag exchanges go out together; a vertex enters the
+// pile once (its flag). Returns the number that enter, *bits = this lane's entries among them.
+__device__ __forceinline__ uint32_t far_flags(uint32_t* fflag, const uint32_t* buf, uint32_t cnt, uint32_t lane,
+                                              uint32_t* bits, uint32_t* before) {
+    __syncwarp();
+    uint32_t old[FCAP / 32];
+#pragma unroll
+    for (int k = 0; k < FCAP / 32; ++k) {
+        const uint32_t e = k * 32u + lane;
+        old[k] = e < cnt ? atomicExch(&fflag[buf[e]], 1u) : 1u;
+    }
+    uint32_t b = 0;
+#pragma unroll
+    for (int k = 0; k < FCAP / 32; ++k) b |= (old[k] != 1u ? 1u : 0u) << k;
+    *bits = b;
+    uint32_t inc = __popc(b);
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= (uint32_t)off) inc += y;
+    }
+    *before = inc - __popc(b);
+    return __shfl_sync(0xffffffffu, inc, 31);
+}
+__device__ __forceinline__ void far_write(const TravArgs& a, const uint32_t* buf, uint32_t bits, uint32_t pos,
+                                          uint32_t* pile, uint32_t lane) {
+#pragma unroll
+    for (int k = 0; k < FCAP / 32; ++k)
+        if ((bits >> k) & 1u) {
+            if (pos < a.n) pile[pos] = buf[k * 32 + lane];
+            else atomicCAS(&a.ctrl->bw.status, (uint32_t)DEV_OK, (uint32_t)DEV_OVERFLOW);
+            ++pos;
+        }
+    __syncwarp();
+}
+
+// The barrier that ends a round, on the word that also counts the next round's parts: the last poll of the
+// arrivals brings the queue length along, so a round starts without reading control words (one L2 round
+// trip and one CTA barrier less), and the arrival is a release-ordered reduction instead of a fence and an
+// atomic. R-MAT s22 SSSP 0.707 -> 0.667 ms, s20 0.250 -> 0.233, s16 97 -> 91 us. Bounded like grid_barrier
+// (common.cuh); a CTA that gives up sets the word's top bit for the others. Returns false when aborting.
+__device__ __forceinline__ bool round_barrier(unsigned long long* w, BarrierWords* bw, uint64_t timeout_ns,
+                                              uint32_t* s_len) {
+    __shared__ uint32_t s_ok3;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        red_release_add64(w, 1ull << 32);
+        uint32_t ok = 1;
+        const uint64_t t0 = global_timer_ns();  // the wait is measured from this CTA's arrival
+        uint32_t spins = 0;
+        unsigned long long v;
+        while (true) {
+            v = ld_acquire64(w);
+            const uint32_t arrived = (uint32_t)(v >> 32);
+            if (arrived & 0x80000000u) { ok = 0; break; }
+            if (arrived == gridDim.x) break;
+            __nanosleep(32);
+            if ((++spins & 7u) == 0 && global_timer_ns() - t0 > timeout_ns) {
+                atomicCAS(&bw->status, (uint32_t)DEV_OK, (uint32_t)DEV_TIMEOUT);
+                atomicOr(w, 1ull << 63);
+                ok = 0;
+                break;
+            }
+        }
+        *s_len = (uint32_t)v;
+        s_ok3 = ok;
+    }
+    __syncthreads();
+    return s_ok3 != 0;
 }
 
 // BK (SSSP/SSWP, SYNC_PUSH_DD, delta > 0): bucketed rounds. A claimed vertex whose key (SSSP: distance,
@@ -194,6 +313,9 @@ template <int OP, int K, bool TD, bool BK = false>
 __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
     constexpr int T_TPB = trav_tpb<OP>();
     __shared__ uint32_t s_buf[TD ? 1 : T_TPB / 32][TD ? 1 : WCAP];
+    __shared__ uint2 s_tot[TD ? 1 : T_TPB / 32];
+    __shared__ uint32_t s_far[BK ? T_TPB / 32 : 1][BK ? FCAP : 1];
+    __shared__ uint32_t s_fbase[BK ? T_TPB / 32 : 1], s_fkey[BK ? T_TPB / 32 : 1];
     __shared__ uint32_t s_next[2];  // per round (alternating): next of this CTA's 32-entry chunks
     __shared__ uint32_t s_ctl[6];   // this round's control words, read once per CTA
 
@@ -203,10 +325,26 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lanemask_lt = (1u << lane) - 1u;
     uint32_t* wbuf = s_buf[TD ? 0 : threadIdx.x >> 5];
+    uint32_t* fbuf = s_far[BK ? threadIdx.x >> 5 : 0];
     const uint64_t pol = l2_evict_first_policy();
     uint32_t epoch = 0;
 
-    unsigned long long my_parts = 0, my_edges = 0, my_updates = 0;
+    // statistics, 32 bits each (a thread's share of 64 rounds is far below 2^32); every 64 rounds a warp's
+    // totals go to shared memory. As 64-bit sums they took three more of the 64 registers.
+    uint32_t my_parts = 0, my_edges = 0, my_updates = 0;
+    __shared__ unsigned long long s_stat[T_TPB / 32][3];
+    if (lane < 3u) s_stat[threadIdx.x >> 5][lane] = 0ull;
+    __syncwarp();
+    auto stat_round = [&]() {
+        const uint32_t r0 = __reduce_add_sync(0xffffffffu, my_parts), r1 = __reduce_add_sync(0xffffffffu, my_edges),
+                       r2 = __reduce_add_sync(0xffffffffu, my_updates);
+        if (lane == 0) {
+            s_stat[threadIdx.x >> 5][0] += r0;
+            s_stat[threadIdx.x >> 5][1] += r1;
+            s_stat[threadIdx.x >> 5][2] += r2;
+        }
+        my_parts = my_edges = my_updates = 0u;
+    };
     // BFS seeded with the source only: every round's queue holds exactly the vertices at level `it`
     // (a round sets values to it+1 only, and a vertex leaves INF once, so atomicMin alone makes each claim
     // unique). Seeding every vertex (ASYNC_PUSH_DD) makes round 0 dense and in place: a vertex reached in
@@ -231,6 +369,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
     // (a superset of the unreached vertices with in-edges, whatever rounds came between). Same levels;
     // R-MAT s22 from the hub pulls in its two large rounds, the second over 6.5 % of the vertices.
     constexpr bool BFSBU = OP == OP_BFS && !TD && !BK;
+    constexpr int KH = K > 8 && trav_tpb<OP>() == 512 ? 8 : K;  // slots of a part expanded at a time
     constexpr int PVL = K <= 8 ? 4 : 2;  // vertices per lane in a pull round, their loads issued together
     const bool can_bu = BFSBU && bfs_levels && a.rvstart != nullptr && a.rounds_limit == 0;
     uint32_t seen_parts = 0;  // forward parts of the vertices reached so far
@@ -262,7 +401,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
             const uint32_t s0 = a.vstart[a.source], s1 = a.vstart[a.source + 1];
             for (uint32_t j = threadIdx.x; j < s1 - s0; j += T_TPB) a.q0[j] = s0 + j;
             if (threadIdx.x == 0) {
-                ctrl->qparts[0] = s1 - s0;
+                ctrl->queued[0] = s1 - s0;
                 ctrl->qverts[0] = 1u;
             }
         }
@@ -276,23 +415,29 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
         }
         const uint32_t cur = it % 3u, nxt = (it + 1u) % 3u, old = (it + 2u) % 3u;
         const bool dense = TD || (a.seed_all && it == 0);
-        // one thread per CTA reads the control words the previous round settled (not every warp of the
-        // grid: those same-address reads queue at one L2 slice); the CTA takes them from shared memory
+        // The queue length came with the barrier that ended the last round (the launch's first round reads
+        // it). What else the round needs is read by one thread per CTA (not by every warp of the grid:
+        // those same-address reads queue at one L2 slice) and shared.
+        const bool first = it == a.it_start;
         if (threadIdx.x == 0) {
-            s_ctl[0] = ld_relaxed(&ctrl->qparts[cur]);
-            if (BFSBU) {
-                s_ctl[5] = ld_relaxed(&ctrl->qverts[cur]);
-                s_ctl[1] = ld_relaxed(&ctrl->lcnt[(pj + 2u) % 3u]);  // the last pull round's list
-            }
+            if (first) s_ctl[0] = (uint32_t)ld_relaxed64(&ctrl->queued[cur]);
+            if (can_bu || a.activity) s_ctl[5] = ld_relaxed(&ctrl->qverts[cur]);
+            if (can_bu) s_ctl[1] = ld_relaxed(&ctrl->lcnt[(pj + 2u) % 3u]);  // the last pull round's list
             if (BK) {
                 const uint32_t f = ld_relaxed(&ctrl->fcsel[it & 1u]);
+                uint32_t c[3], m[3];  // every pile's words, not those of pile f after it is known
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    c[i] = ld_relaxed(&ctrl->fcnt[i]);
+                    m[i] = ld_relaxed(&ctrl->fmin[i]);
+                }
                 s_ctl[1] = f;
                 s_ctl[2] = ld_relaxed(&ctrl->tsel[it & 1u]);
-                s_ctl[3] = ld_relaxed(&ctrl->fcnt[f]);
-                s_ctl[4] = ld_relaxed(&ctrl->fmin[f]);
+                s_ctl[3] = f == 0u ? c[0] : (f == 1u ? c[1] : c[2]);
+                s_ctl[4] = f == 0u ? m[0] : (f == 1u ? m[1] : m[2]);
             }
         }
-        __syncthreads();
+        if (first || can_bu || a.activity || BK) __syncthreads();
         uint32_t fc = 0, T = 0xFFFFFFFFu, fcount = 0;
         if (BK) {
             fc = s_ctl[1];
@@ -302,7 +447,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
         if (it > 0) {
             const uint32_t produced = s_ctl[0];
             if (a.activity && blockIdx.x == 0 && threadIdx.x == 0 && it - 1 < a.activity_cap)
-                a.activity[it - 1] = TD ? produced : ld_relaxed(&ctrl->qverts[cur]);
+                a.activity[it - 1] = TD ? produced : s_ctl[5];
             if (produced == 0u && fcount == 0u) break;
         }
         if (can_bu) {
@@ -342,7 +487,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
             break;
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {
-            ctrl->qparts[old] = 0u;
+            ctrl->queued[old] = 0ull;
             ctrl->qverts[old] = 0u;
             if (BFSBU && bu) ctrl->lcnt[(pj + 1u) % 3u] = 0u;  // the next pull round's list
             if (BK) {  // what the next round reads; the pile two far rounds back is free again
@@ -356,27 +501,28 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
         }
         const uint32_t* pile_src = BK ? a.fpile + (size_t)fc * a.n : nullptr;
         uint32_t* pile_dst = BK ? a.fpile + (size_t)fdst * a.n : nullptr;
-        // Warp-collective: the lanes with `fl` send vertex t (key `key`) to the far pile. A vertex enters
-        // the pile once (its flag); the pile's count and smallest key take one atomic per warp, not per
-        // vertex (same-address atomics from every warp queue at one L2 slice).
+        uint32_t fcnt = 0, fkmin = 0xFFFFFFFFu;  // fill of the far buffer (warp-uniform); this lane's smallest key
+        // Warp-collective: the lanes with `fl` send vertex t (key `key`) to the far pile, through a per-warp
+        // buffer: one flag exchange, one reservation and one minimum per slot and warp (each with its
+        // result waited for, the latter two on the same two words for the whole grid) took two thirds of a
+        // bucketed round of the 4096^2 grid.
         auto to_far = [&](bool fl, uint32_t t, uint32_t key) {
             const uint32_t fmask = __ballot_sync(0xffffffffu, fl);
             if (!fmask) return;
-            const bool app = fl && atomicExch(&a.fflag[t], 1u) != 1u;
-            const uint32_t amask = __ballot_sync(0xffffffffu, app);
-            const uint32_t kmin = __reduce_min_sync(0xffffffffu, fl ? key : 0xFFFFFFFFu);
-            const uint32_t leader = __ffs(fmask) - 1u;
-            uint32_t base = 0;
-            if (lane == leader) {
-                if (amask) base = atomicAdd(&ctrl->fcnt[fdst], (uint32_t)__popc(amask));
-                atomicMin(&ctrl->fmin[fdst], kmin);
+            const uint32_t c = __popc(fmask);
+            if (fcnt + c > (uint32_t)FCAP) {
+                uint32_t bits, before, base = 0;
+                const uint32_t tot = far_flags(a.fflag, fbuf, fcnt, lane, &bits, &before);
+                if (lane == 0 && tot) base = atomicAdd(&ctrl->fcnt[fdst], tot);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                far_write(a, fbuf, bits, base + before, pile_dst, lane);
+                fcnt = 0;
             }
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (app) {
-                const uint32_t pos = base + (uint32_t)__popc(amask & lanemask_lt);
-                if (pos < a.n) pile_dst[pos] = t;
-                else atomicCAS(&ctrl->bw.status, (uint32_t)DEV_OK, (uint32_t)DEV_OVERFLOW);
+            if (fl) {
+                fbuf[fcnt + __popc(fmask & lanemask_lt)] = t;
+                fkmin = key < fkmin ? key : fkmin;
             }
+            fcnt += c;
         };
         // no __restrict__/const-qualified read-only path here: each queue is rewritten every other round
         const uint32_t* qcur = (it & 1u) ? a.q1 : a.q0;
@@ -390,6 +536,10 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
         if (threadIdx.x == 0) s_next[(it + 1u) & 1u] = 0u;
         const uint32_t items = far_round ? fcount : len;
         const uint32_t nch = (items + 31u) / 32u;
+        // A round of at most two chunks per warp is a chain of dependent loads: the part ranges of the
+        // claimed vertices are fetched while the chunk is still expanded (BFS on the 2047^2 grid 1.28 ->
+        // 1.21 ms). In large rounds the fetches only take L1 from the filter reads (R-MAT s22 BFS +2 %).
+        const bool small = (OP == OP_BFS || BK) && items <= 2u * gthreads;
         // A pull round's chunks are vertex ranges, and a vertex id's low bits set its degree on R-MAT-like
         // graphs: with chunk b + i * grid (grid = 304 = 16 * 19) a CTA saw the same low bits in every
         // chunk, and CTAs took 115 to 360 thousand cycles over the same chunk counts (R-MAT s22). In a
@@ -442,7 +592,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                 if (mask) {
                     const uint32_t c = __popc(mask);
                     if (wcnt + c > (uint32_t)WCAP) {
-                        warp_flush(a, wbuf, wcnt, qnext, nxt, lane);
+                        warp_flush(a, wbuf, wcnt, qnext, nxt, can_bu || a.activity, lane);
                         wcnt = 0;
                     }
                     if (move) wbuf[wcnt + __popc(mask & lanemask_lt)] = p;
@@ -546,7 +696,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                     if (mask) {
                         const uint32_t cn = __popc(mask);
                         if (wcnt + cn > (uint32_t)WCAP) {
-                            warp_flush(a, wbuf, wcnt, qnext, nxt, lane);
+                            warp_flush(a, wbuf, wcnt, qnext, nxt, can_bu || a.activity, lane);
                             wcnt = 0;
                         }
                         if (claim[k]) wbuf[wcnt + __popc(mask & lanemask_lt)] = vv[k];
@@ -578,20 +728,21 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                 continue;
             }
             const bool valid = p < a.P;
-            uint32_t col[K], wt[K];
+            uint32_t col[KH], wt[KH];
+            const size_t row = (size_t)p * K;
             uint32_t d = 0;
             bool active = false;
             if (valid) {
                 if (bfs_levels) {  // no owner or value load: the level is the round number
-                    ld_part<K>(a.vcol + (size_t)p * K, col, pol);
+                    ld_part<KH>(a.vcol + row, col, pol);
                     d = it;
                     active = true;
                 } else {
                     const uint32_t v = __ldg(&a.vowner[p]);
                     uint32_t pv = PSENT;
                     if (!TD) {  // DD: the part is almost surely live -- fetch its row alongside the owner's value
-                        ld_part<K>(a.vcol + (size_t)p * K, col, pol);
-                        if (OP != OP_BFS) load_weights<OP, K>(a, p, wt, pol);
+                        ld_part<KH>(a.vcol + row, col, pol);
+                        if (OP != OP_BFS) load_weights<OP, KH>(a, row, wt, pol);
                         if (use_push) pv = __ldcg(&a.pushed[p]);  // written in earlier rounds by any CTA
                     }
                     // plain (L1-cached) value reads: the grid barrier's acquire makes the previous round's
@@ -603,112 +754,159 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                         else a.pushed[p] = d;
                     }
                     if (TD && active) {
-                        ld_part<K>(a.vcol + (size_t)p * K, col, pol);
-                        if (OP != OP_BFS) load_weights<OP, K>(a, p, wt, pol);
+                        ld_part<KH>(a.vcol + row, col, pol);
+                        if (OP != OP_BFS) load_weights<OP, KH>(a, row, wt, pol);
                     }
                 }
                 if (active) ++my_parts;
             }
-            // all K filter reads are issued before the first atomic (the compiler may not move a load of
-            // dist[] across an atomic on dist[]); a stale value only costs an atomic. Queued parts are
-            // almost always live, so their filter reads do not wait for the owner's value.
-            uint32_t cd[K];
+            // A 16-slot row is taken in two halves where its targets, values and filter reads together do not
+            // fit the registers (they spilled 150 bytes in this loop).
             const bool fetch = (dense || use_push) ? active : valid;
+#pragma unroll 1
+            for (int h = 0; h < K / KH; ++h) {
+                if (h > 0 && fetch) {
+                    ld_part<KH>(a.vcol + row + h * KH, col, pol);
+                    if (OP != OP_BFS) load_weights<OP, KH>(a, row + h * KH, wt, pol);
+                }
+                // all filter reads are issued before the first atomic (the compiler may not move a load of
+                // dist[] across an atomic on dist[]); a stale value only costs an atomic. Queued parts are
+                // almost always live, so their filter reads do not wait for the owner's value.
+                uint32_t cd[KH];
 #pragma unroll
-            for (int i = 0; i < K; ++i) cd[i] = (fetch && col[i] != NO_EDGE) ? a.dist[col[i]] : 0u;
-            // The atomics of ATB slots go out before any of their results is used: for each slot whose
-            // filter read says the target improves, the value atomic and (DD, except BFS levels) the
-            // claim on the target's round stamp are issued together. A won claim means the target
-            // improved in this round -- by this lane, or by another after this lane's filter read (that
-            // read is no older than the round's start, and values move one way only) -- so the winner
-            // appends the target, whoever improved it, and a target improved in a round is appended
-            // exactly once.
-            // the far-pile path takes registers too; the 384-thread shape has room for a whole part
-            constexpr int ATG = BK ? 2 : (trav_tpb<OP>() == 384 ? 8 : atomic_group<OP>());
-            constexpr int ATB = K < ATG ? K : ATG;
+                for (int i = 0; i < KH; ++i) cd[i] = (fetch && col[i] != NO_EDGE) ? a.dist[col[i]] : 0u;
+                // What each slot would push, in the place of its weight, and the slots that pass the filter: the
+                // filter values and the owner's value are dead before the first atomic (7 % of SSSP's time on
+                // R-MAT s22, where they spilled).
+                uint32_t hit = 0;
 #pragma unroll
-            for (int i0 = 0; i0 < K; i0 += ATB) {
-                uint32_t prev[ATB], ex[ATB];
-                uint32_t hit = 0;  // slots whose filter passed
-#pragma unroll
-                for (int j = 0; j < ATB; ++j) {
-                    const int i = i0 + j;
-                    prev[j] = 0u;
-                    ex[j] = tag;
+                for (int i = 0; i < KH; ++i) {
                     if (active && col[i] != NO_EDGE) {
                         ++my_edges;
                         const uint32_t nd = relax_value<OP>(d, OP == OP_BFS ? 1u : wt[i]);
-                        if (better<OP>(nd, cd[i])) {
-                            hit |= 1u << j;
-                            prev[j] = atomic_improve<OP>(&a.dist[col[i]], nd);
+                        if (OP != OP_BFS && better<OP>(nd, cd[i])) hit |= 1u << i;
+                        if (OP != OP_BFS) wt[i] = nd;
+                    }
+                }
+                // The atomics of ATB slots go out before any of their results is used: for each slot whose
+                // filter read says the target improves, the value atomic and (DD, except BFS levels) the
+                // claim on the target's round stamp are issued together. A won claim means the target
+                // improved in this round -- by this lane, or by another after this lane's filter read (that
+                // read is no older than the round's start, and values move one way only) -- so the winner
+                // appends the target, whoever improved it, and a target improved in a round is appended
+                // exactly once.
+                // the 384-thread shape has room for a whole part
+                constexpr int ATG = BK ? 2 : (trav_tpb<OP>() == 384 ? 8 : ATOMIC_GROUP);
+                constexpr int ATB = KH < ATG ? KH : ATG;
+#pragma unroll
+                for (int i0 = 0; i0 < KH; i0 += ATB) {
+                    uint32_t prev[ATB], ex[ATB];
+#pragma unroll
+                    for (int j = 0; j < ATB; ++j) {
+                        const int i = i0 + j;
+                        prev[j] = 0u;
+                        ex[j] = tag;
+                        // (BFS, with registers to spare, filters here: 0.201 ms on R-MAT s22, 0.213 above)
+                        if (OP == OP_BFS && active && col[i] != NO_EDGE && better<OP>(d + 1u, cd[i])) hit |= 1u << i;
+                        if ((hit >> i) & 1u) {
+                            prev[j] = atomic_improve<OP>(&a.dist[col[i]], OP == OP_BFS ? d + 1u : wt[i]);
                             if (!TD && !bfs_levels) ex[j] = atomicExch(&a.stamp[col[i]], tag);
                         }
                     }
-                }
 #pragma unroll
-                for (int j = 0; j < ATB; ++j) {
-                    const int i = i0 + j;
-                    bool claim = false, far = false;
-                    uint32_t fkey = 0;
-                    const uint32_t t = col[i];
-                    if ((hit >> j) & 1u) {
-                        const uint32_t nd = relax_value<OP>(d, OP == OP_BFS ? 1u : wt[i]);
-                        const bool imp = better<OP>(nd, prev[j]);
-                        if (imp) ++my_updates;
-                        if (TD) {
-                            if (imp) changed = 1u;
-                        } else if (bfs_levels) {
-                            claim = imp;  // atomicMin admits one first improvement
-                        } else {
-                            claim = ex[j] != tag;
-                        }
-                        if (BK && claim) {
-                            const uint32_t now = imp ? nd : prev[j];  // the target's value after this atomic
-                            const uint32_t key = OP == OP_SSWP ? INF - now : now;
-                            if (key >= T) {  // not in this bucket: wait in the far pile
-                                far = true;
-                                fkey = key;
-                                claim = false;
+                    for (int j = 0; j < ATB; ++j) {
+                        const int i = i0 + j;
+                        bool claim = false, far = false;
+                        uint32_t fkey = 0;
+                        const uint32_t t = col[i];
+                        if ((hit >> i) & 1u) {
+                            const uint32_t nd = OP == OP_BFS ? d + 1u : wt[i];
+                            const bool imp = better<OP>(nd, prev[j]);
+                            if (imp) ++my_updates;
+                            if (TD) {
+                                if (imp) changed = 1u;
+                            } else if (bfs_levels) {
+                                claim = imp;  // atomicMin admits one first improvement
+                            } else {
+                                claim = ex[j] != tag;
+                            }
+                            if (BK && claim) {
+                                const uint32_t now = imp ? nd : prev[j];  // the target's value after this atomic
+                                const uint32_t key = OP == OP_SSWP ? INF - now : now;
+                                if (key >= T) {  // not in this bucket: wait in the far pile
+                                    far = true;
+                                    fkey = key;
+                                    claim = false;
+                                }
                             }
                         }
-                    }
-                    if (BK) to_far(far, t, fkey);
-                    if (!TD) {
-                        const uint32_t mask = __ballot_sync(0xffffffffu, claim);
-                        if (mask) {
-                            const uint32_t c = __popc(mask);
-                            if (wcnt + c > (uint32_t)WCAP) {
-                                warp_flush(a, wbuf, wcnt, qnext, nxt, lane);
-                                wcnt = 0;
+                        if (BK) to_far(far, t, fkey);
+                        if (!TD) {
+                            const uint32_t mask = __ballot_sync(0xffffffffu, claim);
+                            if (mask) {
+                                const uint32_t c = __popc(mask);
+                                if (wcnt + c > (uint32_t)WCAP) {
+                                    warp_flush(a, wbuf, wcnt, qnext, nxt, can_bu || a.activity, lane);
+                                    wcnt = 0;
+                                }
+                                if (claim) {
+                                    wbuf[wcnt + __popc(mask & lanemask_lt)] = t;
+                                    if (small) prefetch_l1(a.vstart + t);
+                                }
+                                wcnt += c;
                             }
-                            if (claim) wbuf[wcnt + __popc(mask & lanemask_lt)] = t;
-                            wcnt += c;
                         }
                     }
                 }
             }
         }
         if (TD) {
-            if (__syncthreads_or(changed) && threadIdx.x == 0) atomicAdd(&ctrl->qparts[nxt], 1u);
-        } else if (wcnt) {
-            warp_flush(a, wbuf, wcnt, qnext, nxt, lane);
+            if (__syncthreads_or(changed) && threadIdx.x == 0) atomicAdd(&ctrl->queued[nxt], 1ull);
+        } else {
+            if (BK) {  // the far buffers, one reservation per CTA
+                constexpr int NW = T_TPB / 32;
+                const uint32_t warp = threadIdx.x >> 5;
+                uint32_t bits = 0, before = 0, tot = 0;
+                if (fcnt) tot = far_flags(a.fflag, fbuf, fcnt, lane, &bits, &before);
+                const uint32_t km = __reduce_min_sync(0xffffffffu, fkmin);
+                if (lane == 0) {
+                    s_fbase[warp] = tot;
+                    s_fkey[warp] = km;
+                }
+                __syncthreads();
+                if (warp == 0) {
+                    const uint32_t c = lane < NW ? s_fbase[lane] : 0u;
+                    const uint32_t k = __reduce_min_sync(0xffffffffu, lane < NW ? s_fkey[lane] : 0xFFFFFFFFu);
+                    uint32_t inc = c;
+#pragma unroll
+                    for (int off = 1; off < 32; off <<= 1) {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+                        if (lane >= (uint32_t)off) inc += y;
+                    }
+                    uint32_t base = 0;
+                    if (lane == 31u && inc) base = atomicAdd(&ctrl->fcnt[fdst], inc);
+                    if (lane == 31u && k != 0xFFFFFFFFu) atomicMin(&ctrl->fmin[fdst], k);
+                    base = __shfl_sync(0xffffffffu, base, 31);
+                    if (lane < NW) s_fbase[lane] = base + inc - c;
+                }
+                __syncthreads();
+                if (fcnt) far_write(a, fbuf, bits, s_fbase[warp] + before, pile_dst, lane);
+            }
+            cta_flush<T_TPB / 32>(a, wbuf, wcnt, qnext, nxt, can_bu || a.activity, lane, s_tot);
         }
+        if ((it & 63u) == 63u) stat_round();
         if (BFSBU && bu) ++pj;
-        if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) break;
+        if (!round_barrier(&ctrl->queued[nxt], &ctrl->bw, a.timeout_ns, &s_ctl[0])) break;
     }
 
 finish:
     // ---- statistics
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        my_parts += __shfl_down_sync(0xffffffffu, my_parts, off);
-        my_edges += __shfl_down_sync(0xffffffffu, my_edges, off);
-        my_updates += __shfl_down_sync(0xffffffffu, my_updates, off);
-    }
+    stat_round();
     if (lane == 0) {
-        if (my_parts) atomicAdd(&ctrl->parts_processed, my_parts);
-        if (my_edges) atomicAdd(&ctrl->edges_scanned, my_edges);
-        if (my_updates) atomicAdd(&ctrl->updates, my_updates);
+        const unsigned long long* st = s_stat[threadIdx.x >> 5];
+        if (st[0]) atomicAdd(&ctrl->parts_processed, st[0]);
+        if (st[1]) atomicAdd(&ctrl->edges_scanned, st[1]);
+        if (st[2]) atomicAdd(&ctrl->updates, st[2]);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         ctrl->iterations = it;
