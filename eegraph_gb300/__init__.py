@@ -378,11 +378,10 @@ class VirtualGraph:
         o.timeout_us = timeout_us
         o.pr_accuracy = pr_accuracy
         o.bfs_push_only = 1 if bfs_push_only else 0
-        n = self.info()["num_nodes"]
         if out_device_ptr is not None:
             outp, on_dev, vals = C.c_void_p(out_device_ptr), 1, None
         else:
-            vals = out if out is not None else np.empty(n, np.float32 if a == PR else np.uint32)
+            vals = out if out is not None else np.empty(self.info()["num_nodes"], np.float32 if a == PR else np.uint32)
             outp, on_dev = _ptr(vals), 0
         act = np.zeros(activity_cap, np.uint32) if activity_cap else None
         r = Result()

@@ -13,6 +13,8 @@
 #include <tuple>
 #include <vector>
 
+#include <cuda.h>
+
 #include "internal.hpp"
 
 namespace eeg {
@@ -118,7 +120,6 @@ static void free_ws(eeg_vgraph* vg) {
     vg_free(vg, w.dd_taken);
     vg_free(vg, w.dd_pq);
     if (w.ddctrl) cudaFree(w.ddctrl);
-    if (w.stats) cudaFree(w.stats);
     if (w.ev[0]) cudaEventDestroy(w.ev[0]);
     if (w.ev[1]) cudaEventDestroy(w.ev[1]);
     w = Workspace{};
@@ -521,6 +522,32 @@ EEG_API void eeg_vgraph_destroy(eeg_vgraph* vg) {
     delete vg;
 }
 
+// True when [p, p + bytes) lies within one 4-byte aligned allocation of `device` that its kernels can
+// write: what a device-to-device copy would accept, checked without making one.
+static bool writable_on(int device, const void* p, size_t bytes) {
+    cudaPointerAttributes at;
+    if (((uintptr_t)p & 3u) || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
+    using RangeFn = CUresult(CUDAAPI*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const RangeFn range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            f = nullptr;
+        }
+        return (RangeFn)f;
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (!range || range(&base, &size, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    return (CUdeviceptr)p + bytes <= base + size;
+}
+
 EEG_API eeg_status eeg_run(eeg_vgraph* vg, eeg_algo algo, eeg_variant variant, uint32_t source,
                            const eeg_options* opts, void* out, int out_on_device, uint32_t* activity,
                            uint32_t activity_cap, void* stream, eeg_result* res) {
@@ -570,19 +597,18 @@ EEG_API eeg_status eeg_run(eeg_vgraph* vg, eeg_algo algo, eeg_variant variant, u
             case EEG_CC: op = OP_CC; break;
             default: set_last_error("unknown algorithm"); return EEG_ERR_INVALID;
         }
-        s = run_traversal(vg, op, variant, source, o, st, &r, activity, activity_cap);
+        // the run's last kernel writes a device array itself; anything a copy has to judge goes to the copy
+        const bool direct = out && out_on_device && writable_on(vg->device, out, sizeof(uint32_t) * (size_t)vg->n);
+        s = run_traversal(vg, op, variant, source, o, st, direct ? (uint32_t*)out : nullptr, &r, activity, activity_cap);
         if (s == EEG_OK || s == EEG_ERR_ITER_CAP) {
-            if (out) {
+            const bool copy = out && !direct;
+            if (copy)
                 EEG_CUDA(cudaMemcpyAsync(out, vg->ws.dist, sizeof(uint32_t) * vg->n,
                                          out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
-            }
-            uint64_t nr = 0, mr = 0;
-            eeg_status s2 = reached_stats(vg, op, vg->ws.dist, st, &nr, &mr);
-            if (s2 != EEG_OK) return s2;
-            r.reached_vertices = nr;
-            r.reached_edges = mr;
-            r.algorithmic_bytes = 12.0 * (double)nr + (op == OP_BFS ? 8.0 : 12.0) * (double)mr;
-            r.gteps = r.kernel_ms > 0 ? (double)mr / (r.kernel_ms * 1e-3) / 1e9 : 0.0;
+            const double nr = (double)r.reached_vertices, mr = (double)r.reached_edges;
+            r.algorithmic_bytes = 12.0 * nr + (op == OP_BFS ? 8.0 : 12.0) * mr;
+            r.gteps = r.kernel_ms > 0 ? mr / (r.kernel_ms * 1e-3) / 1e9 : 0.0;
+            if (copy) EEG_CUDA(cudaStreamSynchronize(st));
         }
     }
     if (res) *res = r;

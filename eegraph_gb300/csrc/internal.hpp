@@ -129,7 +129,6 @@ struct Workspace {
     uint32_t* dd_pq = nullptr;    // P: part queue of the current round
     PRDDCtrl* ddctrl = nullptr;
     // misc
-    unsigned long long* stats = nullptr;  // reached counters
     cudaEvent_t ev[2] = {nullptr, nullptr};
 };
 
@@ -172,11 +171,12 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
 eeg_status build_out_degrees(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const uint32_t* d_dst, cudaStream_t st);
 
 // kernels (traverse.cu / pagerank.cu)
+// out_dev (may be null): device array of num_nodes values, written unless the run gives up.
 eeg_status run_traversal(eeg_vgraph* vg, int op, eeg_variant variant, uint32_t source, const eeg_options& o,
-                         cudaStream_t st, eeg_result* res, uint32_t* activity_host, uint32_t activity_cap);
+                         cudaStream_t st, uint32_t* out_dev, eeg_result* res, uint32_t* activity_host,
+                         uint32_t activity_cap);
 eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& o, cudaStream_t st, eeg_result* res);
 eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_options& o, cudaStream_t st,
                            eeg_result* res);
-eeg_status reached_stats(eeg_vgraph* vg, int op, const uint32_t* d_dist, cudaStream_t st, uint64_t* n_r, uint64_t* m_r);
 
 }  // namespace eeg

@@ -24,6 +24,7 @@
 // any other fixed point.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 
 #include "internal.hpp"
@@ -943,6 +944,62 @@ __global__ void k_reached(const uint32_t* __restrict__ dist, const uint32_t* __r
     }
 }
 
+// End of a run: the values into the caller's device array (out may be null) and the reached-set statistics
+// in one pass, skipped when the run gave up (its output stays untouched). One pair of atomics per CTA: with
+// one per warp, 20 000 of them on two words took as long as the pass.
+template <int OP>
+__global__ void __launch_bounds__(512) k_finish(const uint32_t* __restrict__ dist, const uint32_t* __restrict__ deg,
+                                                uint32_t n, const BarrierWords* bw, uint32_t* __restrict__ out,
+                                                int out16, unsigned long long* stats) {
+    __shared__ unsigned long long s_n[16], s_m[16];
+    const uint32_t status = bw->status;
+    if (status != DEV_OK && status != DEV_ITER_CAP) return;
+    unsigned long long nr = 0, mr = 0;
+    auto one = [&](uint32_t d, uint32_t g) {
+        const bool r = OP == OP_CC || (OP == OP_SSWP ? d != 0u : d != INF);
+        nr += r ? 1u : 0u;
+        mr += r ? g : 0u;
+    };
+    const uint32_t n4 = n / 4u, t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (uint32_t i = t0; i < n4; i += step) {  // both arrays are 256-byte aligned
+        const uint4 d = reinterpret_cast<const uint4*>(dist)[i], g = reinterpret_cast<const uint4*>(deg)[i];
+        one(d.x, g.x);
+        one(d.y, g.y);
+        one(d.z, g.z);
+        one(d.w, g.w);
+        if (out16) {
+            reinterpret_cast<uint4*>(out)[i] = d;
+        } else if (out) {
+            out[4u * i] = d.x;
+            out[4u * i + 1u] = d.y;
+            out[4u * i + 2u] = d.z;
+            out[4u * i + 3u] = d.w;
+        }
+    }
+    for (uint32_t v = 4u * n4 + t0; v < n; v += step) {
+        one(dist[v], deg[v]);
+        if (out) out[v] = dist[v];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        nr += __shfl_down_sync(0xffffffffu, nr, off);
+        mr += __shfl_down_sync(0xffffffffu, mr, off);
+    }
+    if ((threadIdx.x & 31u) == 0) {
+        s_n[threadIdx.x >> 5] = nr;
+        s_m[threadIdx.x >> 5] = mr;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 16; ++w) {
+            nr += s_n[w];
+            mr += s_m[w];
+        }
+        atomicAdd(&stats[0], nr);
+        atomicAdd(&stats[1], mr);
+    }
+}
+
 template <int OP, int K, bool TD>
 eeg_status launch_one(const TravArgs& args, int device, uint32_t blocks_per_sm_req, cudaStream_t st) {
     constexpr bool CAN_BK = !TD && (OP == OP_SSSP || OP == OP_SSWP);
@@ -950,10 +1007,16 @@ eeg_status launch_one(const TravArgs& args, int device, uint32_t blocks_per_sm_r
     constexpr int T_TPB = trav_tpb<OP>();
     // The filter reads of dist[] are L1 hits in part, and L1 is what shared memory leaves: ask for the
     // smallest carveout that still holds the two CTAs per SM the kernel is built for (R-MAT s22: SSSP
-    // 0.725 -> 0.706 ms, SSWP 0.726 -> 0.709, CC 1.215 -> 1.193 against the CUDA driver's default).
-    EEG_TRY(prefer_l1(kern, 2, device));
-    int per_sm = 0;
-    EEG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T_TPB, 0));
+    // 0.725 -> 0.706 ms, SSWP 0.726 -> 0.709, CC 1.215 -> 1.193 against the CUDA driver's default). The hint
+    // and the occupancy belong to the kernel and the device: asked for once (four runtime calls less per run).
+    static std::atomic<int> resident[2][64];
+    std::atomic<int>& slot = resident[args.delta && !args.seed_all ? 1 : 0][device & 63];
+    int per_sm = slot.load(std::memory_order_acquire);
+    if (per_sm == 0) {
+        EEG_TRY(prefer_l1(kern, 2, device));
+        EEG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T_TPB, 0));
+        if (per_sm > 0 && device < 64) slot.store(per_sm, std::memory_order_release);
+    }
     if (per_sm <= 0) {
         set_last_error("traversal kernel does not fit on an SM");
         return EEG_ERR_CUDA;

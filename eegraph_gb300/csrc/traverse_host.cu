@@ -4,26 +4,22 @@
 namespace eeg {
 using namespace trav;
 
-eeg_status reached_stats(eeg_vgraph* vg, int op, const uint32_t* d_dist, cudaStream_t st, uint64_t* n_r,
-                         uint64_t* m_r) {
-    Workspace& ws = vg->ws;
-    if (!ws.stats) EEG_CUDA(cudaMalloc((void**)&ws.stats, 4 * sizeof(unsigned long long)));
-    EEG_CUDA(cudaMemsetAsync(ws.stats, 0, 2 * sizeof(unsigned long long), st));
-    const unsigned blocks = (unsigned)std::min<uint64_t>((vg->n + 255) / 256 + 1, (uint64_t)sm_count(vg->device) * 8);
-    switch (op) {
-        case OP_BFS: k_reached<OP_BFS><<<blocks, 256, 0, st>>>(d_dist, vg->fwd.deg, vg->n, ws.stats); break;
-        case OP_SSSP: k_reached<OP_SSSP><<<blocks, 256, 0, st>>>(d_dist, vg->fwd.deg, vg->n, ws.stats); break;
-        case OP_SSWP: k_reached<OP_SSWP><<<blocks, 256, 0, st>>>(d_dist, vg->fwd.deg, vg->n, ws.stats); break;
-        default: k_reached<OP_CC><<<blocks, 256, 0, st>>>(d_dist, vg->fwd.deg, vg->n, ws.stats); break;
-    }
-    EEG_CUDA(cudaGetLastError());
-    unsigned long long h[2];
-    EEG_CUDA(cudaMemcpyAsync(h, ws.stats, sizeof(h), cudaMemcpyDeviceToHost, st));
-    EEG_CUDA(cudaStreamSynchronize(st));
-    *n_r = h[0];
-    *m_r = h[1];
-    return EEG_OK;
+namespace {
+
+// What a run brings back to the host in one copy.
+struct RunWords {
+    TravCtrl c;
+    unsigned long long reached[2];  // vertices, and their out-edges
+};
+
+template <int OP>
+void finish(const eeg_vgraph* vg, uint32_t* out, unsigned blocks, cudaStream_t st) {
+    RunWords* w = (RunWords*)vg->ws.tctrl;
+    k_finish<OP><<<blocks, 512, 0, st>>>(vg->ws.dist, vg->fwd.deg, vg->n, &w->c.bw, out,
+                                         out && ((uintptr_t)out & 15u) == 0 ? 1 : 0, w->reached);
 }
+
+}  // namespace
 
 static eeg_status ensure_traversal_ws(eeg_vgraph* vg, uint32_t activity_cap) {
     Workspace& ws = vg->ws;
@@ -33,7 +29,7 @@ static eeg_status ensure_traversal_ws(eeg_vgraph* vg, uint32_t activity_cap) {
     if (!ws.pushed) EEG_TRY(vg_alloc(vg, (void**)&ws.pushed, sizeof(uint32_t) * P));
     if (!ws.q[0]) EEG_TRY(vg_alloc(vg, (void**)&ws.q[0], sizeof(uint32_t) * P));
     if (!ws.q[1]) EEG_TRY(vg_alloc(vg, (void**)&ws.q[1], sizeof(uint32_t) * P));
-    if (!ws.tctrl) EEG_CUDA(cudaMalloc((void**)&ws.tctrl, sizeof(TravCtrl)));
+    if (!ws.tctrl) EEG_CUDA(cudaMalloc((void**)&ws.tctrl, sizeof(RunWords)));
     if (activity_cap > ws.activity_cap) {
         if (ws.activity) cudaFree(ws.activity);
         ws.activity = nullptr;
@@ -48,7 +44,8 @@ static eeg_status ensure_traversal_ws(eeg_vgraph* vg, uint32_t activity_cap) {
 }
 
 eeg_status run_traversal(eeg_vgraph* vg, int op, eeg_variant variant, uint32_t source, const eeg_options& o,
-                         cudaStream_t st, eeg_result* res, uint32_t* activity_host, uint32_t activity_cap) {
+                         cudaStream_t st, uint32_t* out_dev, eeg_result* res, uint32_t* activity_host,
+                         uint32_t activity_cap) {
     const bool td = (variant == EEG_ASYNC_PUSH_TD || variant == EEG_SYNC_PUSH_TD);
     // ASYNC_PUSH_DD starts with every vertex active, SYNC_PUSH_DD with the source only
     // (src/eegraph.cu:41-49); for CC that gives SYNC_PUSH_DD its own fixed point (src/eegraph.cu:544-553).
@@ -74,7 +71,7 @@ eeg_status run_traversal(eeg_vgraph* vg, int op, eeg_variant variant, uint32_t s
     Workspace& ws = vg->ws;
     const bool bucketed = o.delta && !td && !seed_all && (op == OP_SSSP || op == OP_SSWP);
     if (bucketed && !ws.far) EEG_TRY(vg_alloc(vg, (void**)&ws.far, sizeof(uint32_t) * 4 * (size_t)vg->n));
-    EEG_CUDA(cudaMemsetAsync(ws.tctrl, 0, sizeof(TravCtrl), st));
+    EEG_CUDA(cudaMemsetAsync(ws.tctrl, 0, sizeof(RunWords), st));
 
     TravArgs a{};
     a.n = vg->n;
@@ -115,7 +112,8 @@ eeg_status run_traversal(eeg_vgraph* vg, int op, eeg_variant variant, uint32_t s
     a.rounds_limit = o.host_loop ? 1u : 0u;
 
     EEG_CUDA(cudaEventRecord(ws.ev[0], st));
-    TravCtrl hc;
+    RunWords words;
+    TravCtrl& hc = words.c;
     uint32_t launches = 0;
     for (;;) {
         eeg_status s;
@@ -138,10 +136,18 @@ eeg_status run_traversal(eeg_vgraph* vg, int op, eeg_variant variant, uint32_t s
         EEG_CUDA(cudaMemsetAsync(&ws.tctrl->bw.arrive, 0, sizeof(uint32_t), st));
     }
     EEG_CUDA(cudaEventRecord(ws.ev[1], st));
-
-    EEG_CUDA(cudaMemcpyAsync(&hc, ws.tctrl, sizeof(TravCtrl), cudaMemcpyDeviceToHost, st));
+    // output copy and statistics follow on the stream; one copy and one wait bring everything back
+    const unsigned blocks = (unsigned)std::min<uint64_t>(vg->n / 2048 + 1, (uint64_t)sm_count(vg->device) * 2);
+    switch (op) {
+        case OP_BFS: finish<OP_BFS>(vg, out_dev, blocks, st); break;
+        case OP_SSSP: finish<OP_SSSP>(vg, out_dev, blocks, st); break;
+        case OP_SSWP: finish<OP_SSWP>(vg, out_dev, blocks, st); break;
+        default: finish<OP_CC>(vg, out_dev, blocks, st); break;
+    }
+    EEG_CUDA(cudaGetLastError());
+    EEG_CUDA(cudaMemcpyAsync(&words, ws.tctrl, sizeof(RunWords), cudaMemcpyDeviceToHost, st));
     EEG_CUDA(cudaStreamSynchronize(st));
-    if (res) res->launches = launches + 1;  // + the reached-set statistics kernel
+    if (res) res->launches = launches + 1;  // + the output and statistics kernel
     float ms = 0.f;
     EEG_CUDA(cudaEventElapsedTime(&ms, ws.ev[0], ws.ev[1]));
     if (res) {
@@ -151,6 +157,8 @@ eeg_status run_traversal(eeg_vgraph* vg, int op, eeg_variant variant, uint32_t s
         res->edges_scanned = hc.edges_scanned;
         res->updates = hc.updates;
         res->pull_rounds = hc.pull_rounds;
+        res->reached_vertices = words.reached[0];
+        res->reached_edges = words.reached[1];
     }
     if (activity_host && activity_cap) {
         const uint32_t cnt = std::min<uint32_t>(hc.iterations, activity_cap);
