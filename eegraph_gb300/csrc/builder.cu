@@ -4,12 +4,17 @@
 // UM twin src/um_virtual_graph.cu:36-111), which build an interleaved host array on one core and
 // drop every edge whose slot index reaches num_edges (src/virtual_graph.cpp:86-88). Here:
 //
-//   1. stable radix sort           (owner, neighbour[, weight]) by owner, 8-bit digits (no hot atomics:
-//                                  a hub's edges are ranked inside each 2048-key tile)
-//   2. runs                        first/last index of each owner -> degree
-//   3. part counts + scan          np[v] = ceil(deg[v] / K); vstart = exclusive scan; vstart[n] = P
-//   4. owner table (segmented)     vowner[vstart[v]] = v for v with parts, then inclusive max-scan
-//   5. placement                   sorted edge of rank r of vertex s -> slot vstart[s]*K + r (part r/K)
+// The low 11 bits of the owner id are a vertex's place in its bucket, the bits above them name the bucket:
+//   1. partition    stable, by bucket, in tiles of 8192 edges: (low bits, neighbour[, weight]). One pass up
+//                   to 2^22 vertices; above, the bucket bits are sorted in passes of at most 11 bits. The
+//                   first pass reads the caller's arrays (shift, both directions, range check).
+//   2. counts       per tile of one bucket and vertex; prefix sums over a bucket's tiles give the degrees
+//   3. part counts  np[v] = ceil(deg[v] / K); vstart = exclusive scan; vstart[n] = P
+//   4. owners       vowner of every part, unused slots of a vertex's last part
+//   5. placement    stable, each tile: edge of rank r of vertex v -> slot vstart[v]*K + r (part r/K)
+// What bounds it is memory traffic: 8-bit radix passes over all 22 bits, a preparing copy, run detection,
+// cleared slots and a separate placement moved 9.7 GB for 67 M weighted edges; this moves 4 GB (2.95 ->
+// 1.98 ms from device arrays; now the tile kernels' shared-memory and store throughput, 0.65 ms each).
 //
 // The result is lossless and deterministic. Part p of vertex v holds out-edges [ (p - vstart[v]) * K,
 // +K ) of v in one K-slot row, in input order (the order MakeGraph gives them), so a thread reads a
@@ -140,256 +145,540 @@ eeg_status device_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, bool i
 namespace {
 
 constexpr int B_TPB = 256;
-// stable LSD radix sort of (owner, neighbour[, weight]) by owner: 8-bit digits, tiles of 2048 keys;
-// warp w of a tile owns keys [w*256, w*256+256) of it and takes them 32 at a time, in order.
-constexpr int R_TPB = 256;
-constexpr int R_WARPS = R_TPB / 32;
-constexpr int R_ITEMS = 8;  // rounds of 32 keys per warp
-constexpr int R_TILE = R_TPB * R_ITEMS;
-constexpr int R_BINS = 256;
-static_assert(R_TPB == R_BINS, "one thread per digit in the cross-warp prefix");
+// Tiles of the partition and the placement: warp w of a tile owns keys [w*512, w*512+512) of it and takes
+// them 32 at a time, in order, so ranks keep the input order. 2048 bins leave runs of at least 4 keys per
+// bin on average (16-byte writes; 4096-key tiles would halve them and double the count tables). Two CTAs
+// per SM, so that one ranks while the other loads or writes: the tile's words share the shared memory of
+// the per-warp counters (102-110 KB), and the neighbours and payloads are loaded only when their places
+// are known (64 registers).
+constexpr int S_TPB = 512;
+constexpr int S_WARPS = S_TPB / 32;
+constexpr int S_ITEMS = 16;
+constexpr int S_TILE = S_TPB * S_ITEMS;
+constexpr int S_BITS = 11;
+constexpr int S_BINS = 1 << S_BITS;
+constexpr int S_CHUNK = 64;  // tiles per prefix chunk
+static_assert(S_TILE <= 65535, "per-tile ranks and starts are 16-bit");
+static_assert(S_BINS == 4 * S_TPB, "a thread owns four bins");
 
-// 0-based owner/neighbour (+ weight, or the arc index when eid != 0) of the m input edges into the sort
-// buffers; with sym, arc m + e is the reverse of edge e. Endpoints outside [0, n) raise err.
-__global__ void k_prepare(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, const uint32_t* __restrict__ w,
-                          uint64_t m, uint32_t n, uint32_t shift, uint32_t* __restrict__ key, uint32_t* __restrict__ nb,
-                          uint32_t* __restrict__ wt, uint32_t* __restrict__ err, int eid, int sym) {
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t s = a[e] - shift, t = b[e] - shift;
-        if (s >= n || t >= n) {
-            atomicOr(err, 1u);
-            s = 0;
-            t = 0;
-        }
-        const uint32_t wv = w ? w[e] : 1u;
-        key[e] = s;
-        nb[e] = t;
-        if (wt) wt[e] = eid ? (uint32_t)e : wv;
-        if (sym) {
-            key[m + e] = t;
-            nb[m + e] = s;
-            if (wt) wt[m + e] = eid ? (uint32_t)(m + e) : wv;
-        }
+// The caller's edges as arcs: arc e < m_in is input edge e, with sym arc m_in + e its reverse. Owner and
+// neighbour 0-based; an endpoint outside [0, n) raises err (the build is then refused).
+struct Arcs {
+    const uint32_t* __restrict__ a;  // owners
+    const uint32_t* __restrict__ b;  // neighbours
+    const uint32_t* __restrict__ w;  // weights (null: 1), unused with eid
+    uint64_t m_in, m;
+    uint32_t n, shift;
+    int sym, eid;
+    uint32_t* err;
+};
+// Tiles of the first pass: the input edges in order, then (sym) once more for the reverses, so that a tile has
+// one direction. Loads in the tile kernels are unconditional (clamped to the tile's last arc) and checks come
+// after all of them: a check behind each load, or an atomic between two, makes a thread wait for one load
+// after the other (40 of 48 thousand cycles per tile).
+struct ArcTile {
+    const uint32_t* __restrict__ owner;
+    const uint32_t* __restrict__ nb;
+    const uint32_t* __restrict__ w;
+    uint32_t first;  // arc index of the tile's first arc (payload with eid)
+    uint32_t count;
+};
+__device__ __forceinline__ ArcTile arc_tile(const Arcs& s, uint32_t tile) {
+    const uint32_t nt = (uint32_t)((s.m_in + S_TILE - 1) / S_TILE);
+    const bool rev = tile >= nt;
+    const uint64_t e0 = (uint64_t)(rev ? tile - nt : tile) * S_TILE;
+    ArcTile r;
+    r.owner = (rev ? s.b : s.a) + e0;
+    r.nb = (rev ? s.a : s.b) + e0;
+    r.w = s.w ? s.w + e0 : nullptr;
+    r.first = (uint32_t)(e0 + (rev ? s.m_in : 0ull));
+    r.count = (uint32_t)min((uint64_t)S_TILE, s.m_in - e0);
+    return r;
+}
+__device__ __forceinline__ uint32_t checked(const Arcs& s, uint32_t id, bool& bad) {
+    id -= s.shift;
+    bad |= id >= s.n;
+    return id >= s.n ? 0u : id;
+}
+
+// A count in shared memory; when the whole warp counts the same bin (sorted edge lists), by one lane.
+__device__ __forceinline__ void count_bin(uint32_t* h, bool valid, uint32_t bin, uint32_t lane) {
+    const uint32_t v = valid ? bin : 0xFFFFFFFFu;
+    if (__all_sync(0xffffffffu, v == __shfl_sync(0xffffffffu, v, 0))) {
+        if (valid && lane == 0) atomicAdd(&h[bin], 32u);
+    } else if (valid) {
+        atomicAdd(&h[bin], 1u);
     }
 }
 
-// Same, four edges per thread with 128-bit loads and stores (all arrays 16-byte aligned, and m a
-// multiple of 4 with sym): when the inputs are page-locked host memory read in place, four times the
-// bytes are in flight per load.
-__device__ __forceinline__ void prep_one(uint32_t s, uint32_t t, uint32_t n, uint32_t shift, uint32_t& ks, uint32_t& kt,
-                                         uint32_t* err) {
-    s -= shift;
-    t -= shift;
-    if (s >= n || t >= n) {
-        atomicOr(err, 1u);
-        s = 0;
-        t = 0;
+// Partition, counts of one tile per bin (key >> lo) & (bins - 1): hist[tile][bin]. The first pass (RAW) takes
+// the owners from the arcs and leaves a copy where the placement of the pass would read them from host
+// memory again (copy non-null).
+template <bool RAW>
+__global__ void __launch_bounds__(S_TPB) k_bin_counts(Arcs s, const uint32_t* __restrict__ key, uint32_t* __restrict__ copy,
+                                                      uint64_t m, uint32_t lo, uint32_t bins, uint32_t* __restrict__ hist) {
+    __shared__ uint32_t h[S_BINS];
+    for (uint32_t i = threadIdx.x; i < bins; i += S_TPB) h[i] = 0u;
+    __syncthreads();
+    const uint32_t* at = key + (RAW ? 0ull : (uint64_t)blockIdx.x * S_TILE);
+    uint32_t count = 0;
+    if (RAW) {
+        const ArcTile a = arc_tile(s, blockIdx.x);
+        at = a.owner;
+        count = a.count;
+    } else {
+        count = (uint32_t)min((uint64_t)S_TILE, m - (uint64_t)blockIdx.x * S_TILE);
     }
-    ks = s;
-    kt = t;
+    uint32_t k[S_ITEMS];
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) k[j] = __ldg(at + min(j * (uint32_t)S_TPB + threadIdx.x, count - 1u));
+    if (RAW) {
+        bool bad = false;
+#pragma unroll
+        for (int j = 0; j < S_ITEMS; ++j) k[j] = checked(s, k[j], bad);
+        if (bad) atomicOr(s.err, 1u);
+    }
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) {
+        const uint32_t i = j * (uint32_t)S_TPB + threadIdx.x;
+        if (RAW && copy && i < count) copy[(uint64_t)blockIdx.x * S_TILE + i] = k[j];
+        count_bin(h, i < count, (k[j] >> lo) & (bins - 1u), threadIdx.x & 31u);
+    }
+    __syncthreads();
+    uint32_t* out = hist + (size_t)blockIdx.x * bins;
+    for (uint32_t i = threadIdx.x; i < bins; i += S_TPB) out[i] = h[i];
 }
-__global__ void k_prepare4(const uint4* __restrict__ a, const uint4* __restrict__ b, const uint4* __restrict__ w,
-                           uint64_t m, uint32_t n, uint32_t shift, uint4* __restrict__ key, uint4* __restrict__ nb,
-                           uint4* __restrict__ wt, uint32_t* __restrict__ err, int eid, int sym) {
-    const uint64_t m4 = m / 4, stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m4; i += stride) {
-        const uint4 s4 = a[i], t4 = b[i];
-        uint4 w4 = make_uint4(1u, 1u, 1u, 1u);
-        if (w && !eid) w4 = w[i];
-        uint4 k, c;
-        prep_one(s4.x, t4.x, n, shift, k.x, c.x, err);
-        prep_one(s4.y, t4.y, n, shift, k.y, c.y, err);
-        prep_one(s4.z, t4.z, n, shift, k.z, c.z, err);
-        prep_one(s4.w, t4.w, n, shift, k.w, c.w, err);
-        key[i] = k;
-        nb[i] = c;
-        if (wt) {
-            const uint32_t e = (uint32_t)(4 * i);
-            wt[i] = eid ? make_uint4(e, e + 1u, e + 2u, e + 3u) : w4;
+
+// hist[tile][bin] -> prefix within its chunk of S_CHUNK tiles; csum[chunk][bin] = the chunk's total
+__global__ void __launch_bounds__(256) k_tile_prefix(uint32_t* hist, uint32_t ntiles, uint32_t bins, uint32_t* csum) {
+    const uint32_t d = blockIdx.y * 256u + threadIdx.x;
+    if (d >= bins) return;
+    const uint32_t t0 = blockIdx.x * S_CHUNK, t1 = min(t0 + (uint32_t)S_CHUNK, ntiles);
+    uint32_t run = 0;
+    for (uint32_t t = t0; t < t1; t += 8u) {
+        uint32_t x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = t + j < t1 ? hist[(size_t)(t + j) * bins + d] : 0u;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (t + j < t1) hist[(size_t)(t + j) * bins + d] = run;
+            run += x[j];
         }
-        if (sym) {
-            key[m4 + i] = c;
-            nb[m4 + i] = k;
-            if (wt) {
-                const uint32_t e = (uint32_t)(m + 4 * i);
-                wt[m4 + i] = eid ? make_uint4(e, e + 1u, e + 2u, e + 3u) : w4;
+    }
+    csum[(size_t)blockIdx.x * bins + d] = run;
+}
+// csum[chunk][bin] -> prefix over the chunks; tot[bin]
+__global__ void __launch_bounds__(256) k_chunk_prefix(uint32_t* csum, uint32_t nchunks, uint32_t bins, uint32_t* tot) {
+    const uint32_t d = blockIdx.x * 256u + threadIdx.x;
+    if (d >= bins) return;
+    uint32_t run = 0;
+    for (uint32_t c = 0; c < nchunks; c += 8u) {
+        uint32_t x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = c + j < nchunks ? csum[(size_t)(c + j) * bins + d] : 0u;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (c + j < nchunks) csum[(size_t)(c + j) * bins + d] = run;
+            run += x[j];
+        }
+    }
+    tot[d] = run;
+}
+
+// One CTA: exclusive scan of f(i), i < count, written to out[i]; out[count] = the total.
+template <class F>
+__device__ void scan_to(F f, uint32_t count, uint32_t* out) {
+    __shared__ uint32_t s_warp[32], s_inc[SCAN_TPB];
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < count; base += SCAN_TPB) {
+        const uint32_t i = base + threadIdx.x;
+        const uint32_t x = i < count ? f(i) : 0u;
+        uint32_t total;
+        const uint32_t ex = cta_exclusive(x, SCAN_ADD, s_warp, s_inc, &total);
+        if (i < count) out[i] = carry + ex;
+        carry += total;
+    }
+    if (threadIdx.x == 0) out[count] = carry;
+}
+__global__ void __launch_bounds__(SCAN_TPB) k_bin_starts(const uint32_t* tot, uint32_t bins, uint32_t* start) {
+    scan_to([&](uint32_t i) { return tot[i]; }, bins, start);
+}
+// Tiles of the buckets: tstart = first tile of each (a bucket without edges has none), tbucket = each tile's bucket
+__global__ void __launch_bounds__(SCAN_TPB) k_bucket_tiles(const uint32_t* __restrict__ bstart, uint32_t nb,
+                                                           uint32_t* tstart, uint32_t* tbucket) {
+    scan_to([&](uint32_t i) { return (bstart[i + 1] - bstart[i] + (uint32_t)S_TILE - 1u) / (uint32_t)S_TILE; }, nb, tstart);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < nb; i += SCAN_TPB)
+        for (uint32_t t = tstart[i]; t < tstart[i + 1]; ++t) tbucket[t] = i;
+}
+// Bucket starts from keys sorted by bucket (more than one partition pass): entry i closes every bucket up to its own
+__global__ void k_bucket_starts(const uint32_t* __restrict__ key, uint64_t m, uint32_t nb, uint32_t* __restrict__ bstart) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= m; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t from = i == 0 ? 0u : (key[i - 1] >> S_BITS) + 1u, to = i == m ? nb : key[i] >> S_BITS;
+        for (uint32_t b = from; b <= to; ++b) bstart[b] = (uint32_t)i;
+    }
+}
+
+// Stable places of a tile's keys in bin order. bin_of(j) is the bin of this lane's key of its warp's round j
+// (>= bins: none); cnt [S_WARPS][bins] is scratch, free again on return. place_of(place, j) = the key's index
+// among the tile's keys ordered by bin (two to a register), dstart[bin] = the bin's first index. Called by all threads.
+__device__ __forceinline__ uint32_t place_of(const uint32_t (&place)[S_ITEMS / 2], int j) {
+    return (place[j >> 1] >> ((j & 1) * 16)) & 0xFFFFu;
+}
+template <class Bin>
+__device__ __forceinline__ void tile_places(Bin bin_of, uint32_t bins, uint16_t* cnt, uint16_t* dstart,
+                                            uint32_t* s_warp, uint32_t (&place)[S_ITEMS / 2]) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint4* z = reinterpret_cast<uint4*>(cnt);
+    for (uint32_t i = threadIdx.x; i < S_WARPS * bins / 8u; i += S_TPB) z[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    uint16_t* mine = cnt + (size_t)warp * bins;
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) {
+        const uint32_t d = bin_of(j);
+        // lanes of the same bin, bit by bit (__match_any_sync, which takes time with every distinct value
+        // among the lanes, is no faster here)
+        uint32_t peers = __ballot_sync(0xffffffffu, d < bins);
+#pragma unroll 1
+        for (int bit = 0; bit < S_BITS; ++bit) {
+            const uint32_t set = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
+            peers &= (d >> bit) & 1u ? set : ~set;
+        }
+        const uint32_t rk = __popc(peers & ((1u << lane) - 1u));
+        const uint32_t before = d < bins ? mine[d] : 0u;
+        __syncwarp();
+        if (d < bins && rk == 0) mine[d] = (uint16_t)(before + __popc(peers));
+        __syncwarp();
+        if (j & 1) place[j >> 1] |= (before + rk) << 16;
+        else place[j >> 1] = before + rk;
+    }
+    __syncthreads();
+    // four bins per thread: offsets of each warp's keys inside the bin, and the bin's length
+    uint32_t len[4] = {0u, 0u, 0u, 0u};
+    const uint32_t d0 = 4u * threadIdx.x;
+    if (d0 < bins) {
+#pragma unroll
+        for (int w = 0; w < S_WARPS; ++w) {
+            uint2* at = reinterpret_cast<uint2*>(cnt + (size_t)w * bins + d0);
+            const uint2 c = *at;
+            *at = make_uint2(len[0] | len[1] << 16, len[2] | len[3] << 16);
+            len[0] += c.x & 0xFFFFu;
+            len[1] += c.x >> 16;
+            len[2] += c.y & 0xFFFFu;
+            len[3] += c.y >> 16;
+        }
+    }
+    uint32_t total;
+    uint32_t run = block_exclusive_sum(len[0] + len[1] + len[2] + len[3], s_warp, &total);
+    if (d0 < bins) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            dstart[d0 + q] = (uint16_t)run;
+            run += len[q];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) {
+        const uint32_t d = bin_of(j);
+        if (d < bins) place[j >> 1] += ((uint32_t)dstart[d] + mine[d]) << ((j & 1) * 16);
+    }
+    __syncthreads();
+}
+
+// Shared memory of the two tile kernels (bytes): the tile's words in the place of the counters (16-byte
+// aligned for any number of bins: both sizes are multiples of 16 from four bins on), then per bin the output
+// offset and the first index.
+__host__ __device__ constexpr size_t max_size(size_t a, size_t b) { return a > b ? a : b; }
+__host__ __device__ constexpr size_t partition_tile(uint32_t bins, bool payload) {
+    return max_size((size_t)S_WARPS * bins * 2, (size_t)S_TILE * (payload ? 12 : 8));
+}
+__host__ __device__ constexpr size_t place_tile(bool payload) {
+    return max_size((size_t)S_WARPS * S_BINS * 2, (size_t)S_TILE * (payload ? 10 : 6));
+}
+constexpr size_t partition_smem(uint32_t bins, bool payload) { return partition_tile(bins, payload) + (size_t)bins * (4 + 2); }
+constexpr size_t place_smem(bool payload) { return place_tile(payload) + (size_t)S_BINS * (8 + 2); }
+static_assert(S_WARPS * 4 * 2 % 16 == 0 && S_TILE * 6 % 16 == 0, "16-byte aligned counters");
+
+// Partition, scatter of one tile: a key's place = its bin's start + the bin's keys in earlier tiles + its rank
+// in the tile. The tile goes through shared memory in bin order, so a bin's run is written by consecutive
+// threads. KOut = uint16_t: only the low S_BITS of the key are kept (the bucket is known from the place).
+template <bool RAW, typename KOut>
+__global__ void __launch_bounds__(S_TPB, 2) k_partition(Arcs s, const uint32_t* __restrict__ key,
+                                                        const uint32_t* __restrict__ nb, const uint32_t* __restrict__ pay,
+                                                        uint64_t m, uint32_t lo, uint32_t bins,
+                                                        const uint32_t* __restrict__ hist, const uint32_t* __restrict__ csum,
+                                                        const uint32_t* __restrict__ start, KOut* __restrict__ key_out,
+                                                        uint32_t* __restrict__ nb_out, uint32_t* __restrict__ pay_out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t s_warp[33];
+    uint16_t* s_cnt = reinterpret_cast<uint16_t*>(smem);
+    uint32_t* s_key = reinterpret_cast<uint32_t*>(smem);  // over the counters, once the places are known
+    uint32_t* s_nb = s_key + S_TILE;
+    uint32_t* s_pay = s_nb + S_TILE;
+    uint32_t* s_goff = reinterpret_cast<uint32_t*>(smem + partition_tile(bins, pay_out != nullptr));
+    uint16_t* s_dstart = reinterpret_cast<uint16_t*>(s_goff + bins);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t first = warp * (32u * S_ITEMS) + lane;  // this lane's keys: first, first + 32, ...
+    ArcTile a{};
+    const uint64_t e0 = (uint64_t)blockIdx.x * S_TILE;
+    if (RAW) a = arc_tile(s, blockIdx.x);
+    else a.count = (uint32_t)min((uint64_t)S_TILE, m - e0);
+    const uint32_t total = a.count;
+    const uint32_t* kp = key ? key + e0 : a.owner;
+    const uint32_t* np = RAW ? a.nb : nb + e0;
+    uint32_t k[S_ITEMS], x[S_ITEMS];
+    uint32_t place[S_ITEMS / 2];
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) k[j] = __ldg(kp + min(first + j * 32u, total - 1u));  // coalesced
+    for (uint32_t d = threadIdx.x; d < bins; d += S_TPB)
+        s_goff[d] = start[d] + csum[(size_t)(blockIdx.x / S_CHUNK) * bins + d] + hist[(size_t)blockIdx.x * bins + d];
+    if (RAW && !key) {
+#pragma unroll
+        for (int j = 0; j < S_ITEMS; ++j) k[j] = checked(s, k[j], bad);
+    }
+    tile_places([&](int j) { return first + j * 32u < total ? (k[j] >> lo) & (bins - 1u) : 0xFFFFFFFFu; }, bins, s_cnt,
+                s_dstart, s_warp, place);
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j)
+        if (first + j * 32u < total) s_key[place_of(place, j)] = k[j];
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) x[j] = __ldg(np + min(first + j * 32u, total - 1u));
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) {
+        if (RAW) x[j] = checked(s, x[j], bad);
+        if (first + j * 32u < total) s_nb[place_of(place, j)] = x[j];
+    }
+    if (RAW && bad) atomicOr(s.err, 1u);
+    if (pay_out) {
+        const uint32_t* pp = RAW ? (s.eid ? nullptr : a.w) : pay + e0;
+        if (pp) {
+#pragma unroll
+            for (int j = 0; j < S_ITEMS; ++j) x[j] = __ldg(pp + min(first + j * 32u, total - 1u));
+        } else {  // arc indices, or weights all 1
+#pragma unroll
+            for (int j = 0; j < S_ITEMS; ++j) x[j] = s.eid ? a.first + first + j * 32u : 1u;
+        }
+#pragma unroll
+        for (int j = 0; j < S_ITEMS; ++j)
+            if (first + j * 32u < total) s_pay[place_of(place, j)] = x[j];
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < total; i += S_TPB) {
+        const uint32_t kk = s_key[i];
+        const uint32_t d = (kk >> lo) & (bins - 1u);
+        const uint32_t gp = s_goff[d] + (i - s_dstart[d]);
+        key_out[gp] = (KOut)(sizeof(KOut) == 2 ? kk & (uint32_t)(S_BINS - 1) : kk);
+        nb_out[gp] = s_nb[i];
+        if (pay_out) pay_out[gp] = s_pay[i];
+    }
+}
+
+// Placement, counts of one tile of a bucket per vertex of the bucket: cnt[tile][vertex]
+template <typename KeyT>
+__global__ void __launch_bounds__(S_TPB) k_vertex_counts(const KeyT* __restrict__ key, const uint32_t* __restrict__ bstart,
+                                                         const uint32_t* __restrict__ tstart,
+                                                         const uint32_t* __restrict__ tbucket, uint32_t nb,
+                                                         uint32_t* __restrict__ cnt) {
+    __shared__ uint32_t h[S_BINS];
+    if (blockIdx.x >= tstart[nb]) return;
+    const uint32_t b = tbucket[blockIdx.x];
+    const uint32_t e0 = bstart[b] + (blockIdx.x - tstart[b]) * (uint32_t)S_TILE;
+    const uint32_t e1 = e0 + min(bstart[b + 1] - e0, (uint32_t)S_TILE);
+    for (uint32_t i = threadIdx.x; i < (uint32_t)S_BINS; i += S_TPB) h[i] = 0u;
+    __syncthreads();
+    uint32_t k[S_ITEMS];
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) {
+        const uint64_t e = min((uint64_t)e0 + j * S_TPB + threadIdx.x, (uint64_t)e1 - 1u);
+        k[j] = (uint32_t)key[e] & (uint32_t)(S_BINS - 1);
+    }
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j)
+        count_bin(h, (uint64_t)e0 + j * S_TPB + threadIdx.x < e1, k[j], threadIdx.x & 31u);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < (uint32_t)S_BINS; i += S_TPB) cnt[(size_t)blockIdx.x * S_BINS + i] = h[i];
+}
+
+// cnt[tile][vertex] -> prefix over the bucket's tiles; deg[v], np[v] = ceil(deg/K) (np[n] = 0) and the
+// max-degree vertex (lowest id among ties). A CTA takes 256 vertices of one bucket: a thread per vertex where
+// the bucket has few tiles (the CTAs of grid row 0); where it has many (a hub's bucket has hundreds), each
+// grid row takes 32 of the vertices, with eight spans of the tiles. R-MAT s22: one chain of loads per vertex
+// everywhere 0.17 ms, spans everywhere 0.16.
+constexpr uint32_t FEW_TILES = 32;
+__global__ void __launch_bounds__(256) k_degrees(uint32_t* cnt, const uint32_t* __restrict__ tstart, uint32_t n, uint32_t K,
+                                                 uint32_t* __restrict__ deg, uint32_t* __restrict__ np,
+                                                 unsigned long long* __restrict__ best) {
+    __shared__ uint32_t s_sum[8][32];
+    const uint32_t lane = threadIdx.x & 31u, span = threadIdx.x >> 5;
+    unsigned long long mine = 0;
+    auto settle = [&](uint32_t v, uint32_t total) {
+        if (v >= n) return;
+        deg[v] = total;
+        np[v] = (total + K - 1) / K;
+        const unsigned long long key = ((unsigned long long)total << 32) | (unsigned long long)(0xFFFFFFFFu - v);
+        mine = key > mine ? key : mine;
+    };
+    // prefix of the tiles [a, b) of one vertex from `run` on, eight loads at a time
+    auto prefix = [&](uint32_t* at, uint32_t a, uint32_t b, uint32_t run) {
+        for (uint32_t t = a; t < b; t += 8u) {
+            uint32_t x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = t + j < b ? at[(size_t)(t + j) * S_BINS] : 0u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (t + j < b) at[(size_t)(t + j) * S_BINS] = run;
+                run += x[j];
             }
         }
-    }
-    // tail (m % 4 edges)
-    const uint32_t* a1 = reinterpret_cast<const uint32_t*>(a);
-    const uint32_t* b1 = reinterpret_cast<const uint32_t*>(b);
-    const uint32_t* w1 = reinterpret_cast<const uint32_t*>(w);
-    for (uint64_t e = 4 * m4 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) {
-        uint32_t ks, kt;
-        prep_one(a1[e], b1[e], n, shift, ks, kt, err);
-        reinterpret_cast<uint32_t*>(key)[e] = ks;
-        reinterpret_cast<uint32_t*>(nb)[e] = kt;
-        if (wt) reinterpret_cast<uint32_t*>(wt)[e] = eid ? (uint32_t)e : (w1 ? w1[e] : 1u);
-        if (sym) {  // not reached: sym takes this kernel only when m is a multiple of 4
-            reinterpret_cast<uint32_t*>(key)[m + e] = kt;
-            reinterpret_cast<uint32_t*>(nb)[m + e] = ks;
-            if (wt) reinterpret_cast<uint32_t*>(wt)[m + e] = eid ? (uint32_t)(m + e) : (w1 ? w1[e] : 1u);
-        }
-    }
-}
-
-// digit counts of one tile, stored digit-major: hist[digit * ntiles + tile]
-__global__ void __launch_bounds__(R_TPB) k_radix_hist(const uint32_t* __restrict__ key, uint64_t m, uint32_t shift,
-                                                      uint32_t* __restrict__ hist, uint32_t ntiles) {
-    __shared__ uint32_t h[R_BINS];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const uint64_t base = (uint64_t)blockIdx.x * R_TILE;
-    uint32_t k[R_ITEMS];
-#pragma unroll
-    for (int j = 0; j < R_ITEMS; ++j) {
-        const uint64_t idx = base + (uint64_t)j * R_TPB + threadIdx.x;
-        k[j] = idx < m ? key[idx] : 0xFFFFFFFFu;
-    }
-#pragma unroll
-    for (int j = 0; j < R_ITEMS; ++j) {
-        const uint64_t idx = base + (uint64_t)j * R_TPB + threadIdx.x;
-        if (idx < m) atomicAdd(&h[(k[j] >> shift) & (R_BINS - 1)], 1u);
-    }
-    __syncthreads();
-    hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
-}
-
-// Stable scatter of one tile by digit: a key's place = the tile's global offset for its digit + the keys
-// with that digit earlier in the tile (earlier warps, earlier rounds of its warp, lower lanes).
-__global__ void __launch_bounds__(R_TPB) k_radix_scatter(const uint32_t* __restrict__ key_in,
-                                                         const uint32_t* __restrict__ nb_in,
-                                                         const uint32_t* __restrict__ w_in, uint32_t* __restrict__ key_out,
-                                                         uint32_t* __restrict__ nb_out, uint32_t* __restrict__ w_out,
-                                                         uint64_t m, uint32_t shift, const uint32_t* __restrict__ offs,
-                                                         uint32_t ntiles) {
-    __shared__ uint32_t s_cnt[R_WARPS][R_BINS];
-    __shared__ uint32_t s_key[R_TILE], s_nb[R_TILE], s_w[R_TILE];
-    __shared__ uint32_t s_dstart[R_BINS], s_goff[R_BINS], s_warp[33];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t wbase = (uint64_t)blockIdx.x * R_TILE + (uint64_t)warp * (32 * R_ITEMS);
-#pragma unroll
-    for (int w = 0; w < R_WARPS; ++w) s_cnt[w][threadIdx.x] = 0;
-    uint32_t k[R_ITEMS], v[R_ITEMS], wv[R_ITEMS], rank[R_ITEMS];
-#pragma unroll
-    for (int j = 0; j < R_ITEMS; ++j) {  // all loads first (coalesced: 32 consecutive keys per round)
-        const uint64_t idx = wbase + (uint64_t)j * 32 + lane;
-        const bool valid = idx < m;
-        k[j] = valid ? key_in[idx] : 0u;
-        v[j] = valid ? nb_in[idx] : 0u;
-        wv[j] = (valid && w_out) ? w_in[idx] : 0u;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < R_ITEMS; ++j) {
-        const uint64_t idx = wbase + (uint64_t)j * 32 + lane;
-        const uint32_t digit = idx < m ? (k[j] >> shift) & (R_BINS - 1) : (uint32_t)R_BINS;
-        const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-        const uint32_t rk = __popc(peers & ((1u << lane) - 1u));
-        const uint32_t before = digit < R_BINS ? s_cnt[warp][digit] : 0u;
-        __syncwarp();
-        if (digit < R_BINS && rk == 0) s_cnt[warp][digit] = before + __popc(peers);
-        __syncwarp();
-        rank[j] = before + rk;
-    }
-    __syncthreads();
-    // per digit (thread = digit): offsets of each warp's keys inside the digit's run, and the run length
-    uint32_t cnt = 0;
-#pragma unroll
-    for (int w = 0; w < R_WARPS; ++w) {
-        const uint32_t c = s_cnt[w][threadIdx.x];
-        s_cnt[w][threadIdx.x] = cnt;
-        cnt += c;
-    }
-    // the tile in digit order in shared memory: digit runs start at the exclusive scan of the counts
-    uint32_t total;
-    const uint32_t dstart = block_exclusive_sum(cnt, s_warp, &total);
-    s_dstart[threadIdx.x] = dstart;
-    s_goff[threadIdx.x] = offs[(size_t)threadIdx.x * ntiles + blockIdx.x];
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < R_ITEMS; ++j) {
-        const uint64_t idx = wbase + (uint64_t)j * 32 + lane;
-        if (idx < m) {
-            const uint32_t d = (k[j] >> shift) & (R_BINS - 1);
-            const uint32_t lp = s_dstart[d] + s_cnt[warp][d] + rank[j];
-            s_key[lp] = k[j];
-            s_nb[lp] = v[j];
-            if (w_out) s_w[lp] = wv[j];
-        }
-    }
-    __syncthreads();
-    // write the digit runs out: consecutive threads -> consecutive addresses inside each run
-    for (uint32_t i = threadIdx.x; i < total; i += R_TPB) {
-        const uint32_t kk = s_key[i];
-        const uint32_t d = (kk >> shift) & (R_BINS - 1);
-        const uint32_t gp = s_goff[d] + (i - s_dstart[d]);
-        key_out[gp] = kk;
-        nb_out[gp] = s_nb[i];
-        if (w_out) w_out[gp] = s_w[i];
-    }
-}
-
-// first and one-past-last index of every owner's run in the sorted keys
-__global__ void k_runs(const uint32_t* __restrict__ key, uint64_t m, uint32_t* __restrict__ rs,
-                       uint32_t* __restrict__ re) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t o = key[i];
-        if (i == 0 || key[i - 1] != o) rs[o] = (uint32_t)i;
-        if (i + 1 == m || key[i + 1] != o) re[o] = (uint32_t)(i + 1);
-    }
-}
-
-// deg[v] = run length; np[v] = ceil(deg/K) for v < n, np[n] = 0; also the max-degree vertex
-// (lowest id among ties).
-__global__ void k_nparts(const uint32_t* __restrict__ rs, const uint32_t* __restrict__ re, uint32_t n, uint32_t K,
-                         uint32_t* __restrict__ deg, uint32_t* __restrict__ np, unsigned long long* __restrict__ best) {
-    unsigned long long mine = 0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x) {
-        if (v == n) {
-            np[v] = 0;
+        return run;
+    };
+    for (uint64_t v0 = (uint64_t)blockIdx.x * 256u; v0 < n; v0 += (uint64_t)gridDim.x * 256u) {  // 256 divides a bucket
+        const uint32_t t0 = tstart[v0 >> S_BITS], tiles = tstart[(v0 >> S_BITS) + 1] - t0;
+        if (tiles <= FEW_TILES) {
+            if (blockIdx.y) continue;
+            const uint32_t v = (uint32_t)v0 + threadIdx.x;
+            settle(v, prefix(cnt + (v & (S_BINS - 1)), t0, t0 + tiles, 0u));
             continue;
         }
-        const uint32_t d = re[v] - rs[v];
-        deg[v] = d;
-        np[v] = (d + K - 1) / K;
-        unsigned long long key = ((unsigned long long)d << 32) | (unsigned long long)(0xFFFFFFFFu - v);
-        mine = key > mine ? key : mine;
+        const uint32_t a = t0 + (uint32_t)((uint64_t)tiles * span / 8u), b = t0 + (uint32_t)((uint64_t)tiles * (span + 1u) / 8u);
+        const uint32_t v = (uint32_t)v0 + blockIdx.y * 32u + lane;
+        uint32_t* at = cnt + (v & (S_BINS - 1));
+        uint32_t sum = 0;
+#pragma unroll 8
+        for (uint32_t t = a; t < b; ++t) sum += at[(size_t)t * S_BINS];
+        s_sum[span][lane] = sum;
+        __syncthreads();
+        uint32_t run = 0, total = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 8u; ++q) {
+            run += q < span ? s_sum[q][lane] : 0u;
+            total += s_sum[q][lane];
+        }
+        prefix(at, a, b, run);
+        if (span == 0u) settle(v, total);
+        __syncthreads();
     }
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) np[n] = 0;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
-        unsigned long long o = __shfl_down_sync(0xffffffffu, mine, off);
+        const unsigned long long o = __shfl_down_sync(0xffffffffu, mine, off);
         mine = o > mine ? o : mine;
     }
-    if ((threadIdx.x & 31u) == 0 && mine) atomicMax(best, mine);
+    if (lane == 0u && mine) atomicMax(best, mine);
 }
 
-__global__ void k_heads(const uint32_t* __restrict__ vstart, uint32_t n, uint32_t* __restrict__ vowner) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        uint32_t a = vstart[v], b = vstart[v + 1];
-        if (b > a) vowner[a] = v;
+// Owner of every part, and the unused slots of each vertex's last part (targets and edge indices NO_EDGE,
+// weights 0). A vertex of more than 32 parts is written by its whole warp. The unused slots end a row aligned
+// to its size, so they are written in at most one store each of 4, 8 and 16 bytes (and one more 16 for K =
+// 16): a store of 32 lanes here touches 32 sectors whatever its width, 0.16 ms on R-MAT s22 word by word.
+__device__ __forceinline__ void pad_row(uint32_t* p, size_t i, size_t end, uint32_t x) {
+    if ((i & 1u) && i < end) p[i++] = x;
+    if ((i & 2u) && i < end) {
+        *reinterpret_cast<uint2*>(p + i) = make_uint2(x, x);
+        i += 2;
+    }
+    for (; i < end; i += 4) *reinterpret_cast<uint4*>(p + i) = make_uint4(x, x, x, x);
+}
+__global__ void k_owners(uint32_t n, uint32_t K, const uint32_t* __restrict__ vstart, const uint32_t* __restrict__ deg,
+                         uint32_t* __restrict__ vowner, uint32_t* __restrict__ vcol, uint32_t* __restrict__ vw,
+                         uint32_t* __restrict__ veid) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t v0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; v0 < n;
+         v0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t v = v0 + lane;
+        uint32_t s0 = 0, np = 0;
+        if (v < n) {
+            s0 = vstart[v];
+            np = vstart[v + 1] - s0;
+            if (np) {
+                const size_t end = (size_t)(s0 + np) * K;
+                const size_t used = (size_t)s0 * K + deg[v];
+                pad_row(vcol, used, end, NO_EDGE);
+                if (vw) pad_row(vw, used, end, 0u);
+                if (veid) pad_row(veid, used, end, NO_EDGE);
+                if (np <= 32u)
+                    for (uint32_t j = 0; j < np; ++j) vowner[s0 + j] = (uint32_t)v;
+            }
+        }
+        uint32_t big = __ballot_sync(0xffffffffu, np > 32u);
+        while (big) {
+            const int l = __ffs(big) - 1;
+            big &= big - 1u;
+            const uint32_t bs = __shfl_sync(0xffffffffu, s0, l), bn = __shfl_sync(0xffffffffu, np, l);
+            for (uint32_t j = lane; j < bn; j += 32u) vowner[bs + j] = (uint32_t)v0 + (uint32_t)l;
+        }
     }
 }
 
-// sorted edge i of owner o (rank r = i - rs[o]) goes to slot vstart[o]*K + r: part r/K, lane r%K
-// With veid (edge-index mode) the sorted payload is the arc index: the weight is gathered from the
-// input array by it (arc e >= m_in of a symmetrised build is the reverse of input edge e - m_in; m_in
-// is 0 otherwise) and the index is kept per slot.
-__global__ void k_place(const uint32_t* __restrict__ key, const uint32_t* __restrict__ nb, const uint32_t* __restrict__ wt,
-                        uint64_t m, uint32_t K, const uint32_t* __restrict__ rs, const uint32_t* __restrict__ vstart,
-                        uint32_t* __restrict__ vcol, uint32_t* __restrict__ vw, const uint32_t* __restrict__ w_in,
-                        uint32_t* __restrict__ veid, uint64_t m_in) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t o = key[i];
-        const size_t slot = (size_t)vstart[o] * K + (i - rs[o]);
-        vcol[slot] = nb[i];
+// Placement of one tile of a bucket: edge of rank r of vertex v -> slot vstart[v]*K + r, through shared memory
+// in vertex order (the partition's scheme). With veid the payload is the arc index: the weight is gathered
+// from the input array by it (arc e >= m_in of a symmetrised build is the reverse of input edge e - m_in;
+// m_in is 0 otherwise) and the index is kept per slot.
+template <typename KeyT>
+__global__ void __launch_bounds__(S_TPB, 2) k_place(const KeyT* __restrict__ key, const uint32_t* __restrict__ nb,
+                                                    const uint32_t* __restrict__ pay, const uint32_t* __restrict__ bstart,
+                                                    const uint32_t* __restrict__ tstart,
+                                                    const uint32_t* __restrict__ tbucket, uint32_t nbuckets, uint32_t n,
+                                                    uint32_t K, const uint32_t* __restrict__ cnt,
+                                                    const uint32_t* __restrict__ vstart, uint32_t* __restrict__ vcol,
+                                                    uint32_t* __restrict__ vw, const uint32_t* __restrict__ w_in,
+                                                    uint32_t* __restrict__ veid, uint64_t m_in) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t s_warp[33];
+    uint16_t* s_cnt = reinterpret_cast<uint16_t*>(smem);
+    uint32_t* s_nb = reinterpret_cast<uint32_t*>(smem);  // over the counters, once the places are known
+    uint16_t* s_key = reinterpret_cast<uint16_t*>(s_nb + S_TILE);
+    uint32_t* s_pay = reinterpret_cast<uint32_t*>(s_key + S_TILE);
+    unsigned long long* s_goff = reinterpret_cast<unsigned long long*>(smem + place_tile(pay != nullptr));
+    uint16_t* s_dstart = reinterpret_cast<uint16_t*>(s_goff + S_BINS);
+    if (blockIdx.x >= tstart[nbuckets]) return;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t b = tbucket[blockIdx.x];
+    const uint32_t e0 = bstart[b] + (blockIdx.x - tstart[b]) * (uint32_t)S_TILE;
+    const uint32_t total = min(bstart[b + 1] - e0, (uint32_t)S_TILE);  // at least 1
+    const uint32_t wbase = warp * (32u * S_ITEMS) + lane;
+    const KeyT* kp = key + e0;
+    const uint32_t* np = nb + e0;
+    KeyT bin[S_ITEMS];
+    uint32_t x[S_ITEMS];
+    uint32_t place[S_ITEMS / 2];
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) bin[j] = kp[min(wbase + j * 32u, total - 1u)];
+    for (uint32_t d = threadIdx.x; d < (uint32_t)S_BINS; d += S_TPB) {
+        const uint32_t vx = (b << S_BITS) + d;
+        s_goff[d] = vx < n ? (unsigned long long)vstart[vx] * K + cnt[(size_t)blockIdx.x * S_BINS + d] : 0ull;
+    }
+    tile_places([&](int j) { return wbase + j * 32u < total ? (uint32_t)bin[j] & (uint32_t)(S_BINS - 1) : 0xFFFFFFFFu; },
+                S_BINS, s_cnt, s_dstart, s_warp, place);
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j) x[j] = __ldg(np + min(wbase + j * 32u, total - 1u));
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j)
+        if (wbase + j * 32u < total) s_key[place_of(place, j)] = (uint16_t)((uint32_t)bin[j] & (uint32_t)(S_BINS - 1));
+#pragma unroll
+    for (int j = 0; j < S_ITEMS; ++j)
+        if (wbase + j * 32u < total) s_nb[place_of(place, j)] = x[j];
+    if (pay) {
+        const uint32_t* pp = pay + e0;
+#pragma unroll
+        for (int j = 0; j < S_ITEMS; ++j) x[j] = __ldg(pp + min(wbase + j * 32u, total - 1u));
+#pragma unroll
+        for (int j = 0; j < S_ITEMS; ++j)
+            if (wbase + j * 32u < total) s_pay[place_of(place, j)] = x[j];
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < total; i += S_TPB) {
+        const uint32_t d = s_key[i];
+        const size_t slot = (size_t)(s_goff[d] + (i - s_dstart[d]));
+        vcol[slot] = s_nb[i];
         if (veid) {
-            const uint32_t e = wt[i];
+            const uint32_t e = s_pay[i];
             veid[slot] = e;
             if (vw) vw[slot] = w_in ? w_in[(m_in && e >= m_in) ? e - m_in : e] : 1u;
         } else if (vw) {
-            vw[slot] = wt ? wt[i] : 1u;
+            vw[slot] = s_pay[i];  // a weighted direction always carries a payload
         }
     }
 }
@@ -450,11 +739,11 @@ namespace {
 // stream-ordered temporaries released on every exit path
 struct TempSet {
     cudaStream_t st;
-    void* p[16] = {nullptr};
+    void* p[32] = {nullptr};
     int k = 0;
     explicit TempSet(cudaStream_t s) : st(s) {}
     eeg_status get(void** out, size_t bytes) {
-        if (k == 16) {
+        if (k == 32) {
             set_last_error("builder: too many temporaries");
             return EEG_ERR_INVALID;
         }
@@ -496,71 +785,125 @@ eeg_status build_out_degrees(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, con
     return EEG_OK;
 }
 
-// Build one direction. reverse: edges (s,t) are inserted as (t,s) -- the transposed graph.
-// Edges are sorted by owner with a stable radix sort, so each vertex's edges keep the input order
-// (the order the reference's MakeGraph gives them) and the layout is deterministic. With
-// EEG_VG_SYMMETRIZE the vg->m arcs are the vg->m / 2 input edges followed by their reverses.
+// Build one direction. reverse: edges (s,t) are inserted as (t,s) -- the transposed graph. Each vertex's
+// edges keep the input order (the order the reference's MakeGraph gives them) and the layout is
+// deterministic. With EEG_VG_SYMMETRIZE the vg->m arcs are the vg->m / 2 input edges followed by their
+// reverses. host_in: the input arrays are page-locked host memory, each read once over the link.
 eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const uint32_t* d_dst,
-                           const uint32_t* d_w, bool reverse, cudaStream_t st) {
+                           const uint32_t* d_w, bool reverse, bool host_in, cudaStream_t st) {
     const uint32_t n = vg->n, K = vg->K;
     const uint64_t m = vg->m;
     const bool sym = (vg->flags & EEG_VG_SYMMETRIZE) != 0;
     const uint64_t m_in = sym ? m / 2 : m;  // input edges
-    const uint32_t shift = (vg->flags & EEG_VG_SHIFT_ONE) ? 1u : 0u;
-    const uint32_t* a = reverse ? d_dst : d_src;
-    const uint32_t* b = reverse ? d_src : d_dst;
     const bool with_w = (d_w != nullptr) || (!reverse && vg->weighted);
     const bool eid = (vg->flags & EEG_VG_EDGE_IDS) != 0;
-    const bool payload = with_w || eid;  // the sort carries a third word: weight, or edge index
+    const bool payload = with_w || eid;  // a third word per edge: weight, or edge index
+    const uint32_t bits = n > 1 ? 32u - (uint32_t)__builtin_clz(n - 1) : 1u;
+    const uint32_t high = bits > (uint32_t)S_BITS ? bits - (uint32_t)S_BITS : 0u;  // bucket bits
+    const uint32_t passes = std::max<uint32_t>(1u, (high + S_BITS - 1) / S_BITS);
+    const uint32_t nb_buckets = n ? ((n - 1) >> S_BITS) + 1u : 1u;
+    // the first pass's tiles have one direction each (later passes have no more of them)
+    const uint64_t ntiles = ((m_in + S_TILE - 1) / S_TILE) * (sym ? 2u : 1u);
+    const uint64_t ntiles2 = (m + S_TILE - 1) / S_TILE;
+    const uint64_t nchunks = (ntiles + S_CHUNK - 1) / S_CHUNK;
+    const uint64_t vtiles = m / S_TILE + std::min<uint64_t>(nb_buckets, m);  // most tiles the buckets can have
 
     EEG_TRY(vg_alloc(vg, (void**)&d->deg, sizeof(uint32_t) * (size_t)(n + 1)));
     EEG_TRY(vg_alloc(vg, (void**)&d->vstart, sizeof(uint32_t) * (size_t)(n + 1)));
     TempSet T(st);
-    uint32_t *key[2] = {nullptr, nullptr}, *nb[2] = {nullptr, nullptr}, *wt[2] = {nullptr, nullptr};
-    uint32_t *rs = nullptr, *re = nullptr, *np = nullptr, *tmp = nullptr, *err = nullptr, *hist = nullptr;
-    for (int i = 0; i < 2; ++i) {
-        EEG_TRY(T.get((void**)&key[i], sizeof(uint32_t) * m));
-        EEG_TRY(T.get((void**)&nb[i], sizeof(uint32_t) * m));
-        if (payload) EEG_TRY(T.get((void**)&wt[i], sizeof(uint32_t) * m));
-    }
-    EEG_TRY(T.get((void**)&rs, sizeof(uint32_t) * (size_t)(n + 1)));
-    EEG_TRY(T.get((void**)&re, sizeof(uint32_t) * (size_t)(n + 1)));
+    uint32_t *np = nullptr, *tmp = nullptr, *err = nullptr;
     EEG_TRY(T.get((void**)&np, sizeof(uint32_t) * (size_t)(n + 1)));
     EEG_TRY(T.get((void**)&err, 16));
+    EEG_TRY(T.get((void**)&tmp, sizeof(uint32_t) * device_scan_tmp_words((uint64_t)n + 1)));
     unsigned long long* best = (unsigned long long*)(err + 2);
-    const uint64_t ntiles = (m + R_TILE - 1) / R_TILE;
-    const uint64_t hwords = std::max<uint64_t>(ntiles * R_BINS, 1);
-    EEG_TRY(T.get((void**)&hist, sizeof(uint32_t) * hwords));
-    EEG_TRY(T.get((void**)&tmp, sizeof(uint32_t) * device_scan_tmp_words(std::max<uint64_t>(hwords, (uint64_t)n + 1))));
     EEG_CUDA(cudaMemsetAsync(err, 0, 16, st));
-    EEG_CUDA(cudaMemsetAsync(rs, 0, sizeof(uint32_t) * (size_t)(n + 1), st));
-    EEG_CUDA(cudaMemsetAsync(re, 0, sizeof(uint32_t) * (size_t)(n + 1), st));
 
-    int cur = 0;
+    // ---- partition by bucket
+    void* key = nullptr;                       // uint16_t low bits (one pass) or the uint32_t owners
+    uint32_t *nb = nullptr, *pay = nullptr;    // partitioned
+    uint32_t *bstart = nullptr, *tstart = nullptr, *tbucket = nullptr, *vcnt = nullptr;
     if (m > 0) {
-        const uint32_t* wi = with_w ? d_w : nullptr;
-        auto al16 = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
-        if (al16(a) && al16(b) && al16(wi) && m_in >= 4 && (!sym || m_in % 4 == 0))
-            k_prepare4<<<grid_for(m_in / 4, vg->device), B_TPB, 0, st>>>(
-                reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(b), reinterpret_cast<const uint4*>(wi),
-                m_in, n, shift, reinterpret_cast<uint4*>(key[0]), reinterpret_cast<uint4*>(nb[0]),
-                payload ? reinterpret_cast<uint4*>(wt[0]) : nullptr, err, eid ? 1 : 0, sym ? 1 : 0);
-        else
-            k_prepare<<<grid_for(m_in, vg->device), B_TPB, 0, st>>>(a, b, wi, m_in, n, shift, key[0], nb[0],
-                                                                     payload ? wt[0] : nullptr, err, eid ? 1 : 0,
-                                                                     sym ? 1 : 0);
-        const uint32_t bits = n > 1 ? 32u - (uint32_t)__builtin_clz(n - 1) : 1u;
-        for (uint32_t sh = 0; sh < bits; sh += 8) {
-            k_radix_hist<<<(unsigned)ntiles, R_TPB, 0, st>>>(key[cur], m, sh, hist, (uint32_t)ntiles);
-            EEG_TRY(device_scan_u32(hist, hist, ntiles * R_BINS, false, SCAN_ADD, tmp, st));
-            k_radix_scatter<<<(unsigned)ntiles, R_TPB, 0, st>>>(key[cur], nb[cur], wt[cur], key[cur ^ 1], nb[cur ^ 1],
-                                                                payload ? wt[cur ^ 1] : nullptr, m, sh, hist,
-                                                                (uint32_t)ntiles);
-            cur ^= 1;
+        Arcs s{};
+        s.a = reverse ? d_dst : d_src;
+        s.b = reverse ? d_src : d_dst;
+        s.w = with_w ? d_w : nullptr;
+        s.m_in = m_in;
+        s.m = m;
+        s.n = n;
+        s.shift = (vg->flags & EEG_VG_SHIFT_ONE) ? 1u : 0u;
+        s.sym = sym ? 1 : 0;
+        s.eid = eid ? 1 : 0;
+        s.err = err;
+        const uint32_t max_bins = 1u << std::max(2u, (high + passes - 1) / passes);
+        uint32_t *hist = nullptr, *csum = nullptr, *tot = nullptr, *start = nullptr, *copy = nullptr;
+        EEG_TRY(T.get((void**)&hist, sizeof(uint32_t) * ntiles * max_bins));
+        EEG_TRY(T.get((void**)&csum, sizeof(uint32_t) * nchunks * max_bins));
+        EEG_TRY(T.get((void**)&tot, sizeof(uint32_t) * max_bins));
+        EEG_TRY(T.get((void**)&start, sizeof(uint32_t) * (max_bins + 1)));
+        if (host_in) EEG_TRY(T.get((void**)&copy, sizeof(uint32_t) * m));
+        uint32_t* in_key = nullptr;  // null: the arcs
+        uint32_t *in_nb = nullptr, *in_pay = nullptr;
+        uint32_t lo = (uint32_t)S_BITS;
+        for (uint32_t p = 0; p < passes; ++p) {
+            const bool last = p + 1 == passes;
+            // bits of this pass (at least 2: the tile kernels take four bins per thread)
+            const uint32_t pbits = std::max(2u, last ? std::max(bits, lo) - lo : (high + passes - 1) / passes);
+            const uint32_t bins = 1u << pbits;
+            void* out_key = nullptr;
+            uint32_t *out_nb = nullptr, *out_pay = nullptr;
+            EEG_TRY(T.get(&out_key, (passes == 1 ? sizeof(uint16_t) : sizeof(uint32_t)) * m));
+            EEG_TRY(T.get((void**)&out_nb, sizeof(uint32_t) * m));
+            if (payload) EEG_TRY(T.get((void**)&out_pay, sizeof(uint32_t) * m));
+            const uint64_t nt = p == 0 ? ntiles : ntiles2, nc = (nt + S_CHUNK - 1) / S_CHUNK;
+            if (p == 0)
+                k_bin_counts<true><<<(unsigned)nt, S_TPB, 0, st>>>(s, nullptr, copy, m, lo, bins, hist);
+            else
+                k_bin_counts<false><<<(unsigned)nt, S_TPB, 0, st>>>(s, in_key, nullptr, m, lo, bins, hist);
+            k_tile_prefix<<<dim3((unsigned)nc, (bins + 255u) / 256u), 256, 0, st>>>(hist, (uint32_t)nt, bins, csum);
+            k_chunk_prefix<<<(bins + 255u) / 256u, 256, 0, st>>>(csum, (uint32_t)nc, bins, tot);
+            k_bin_starts<<<1, SCAN_TPB, 0, st>>>(tot, bins, start);
+            const size_t smem = partition_smem(bins, payload);
+            const uint32_t* kin = p == 0 ? copy : in_key;
+            auto go = [&](auto kern, auto* kout) -> eeg_status {
+                EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                kern<<<(unsigned)nt, S_TPB, smem, st>>>(s, kin, in_nb, in_pay, m, lo, bins, hist, csum, start, kout,
+                                                            out_nb, out_pay);
+                return EEG_OK;
+            };
+            if (passes == 1) EEG_TRY(go(k_partition<true, uint16_t>, (uint16_t*)out_key));
+            else if (p == 0) EEG_TRY(go(k_partition<true, uint32_t>, (uint32_t*)out_key));
+            else EEG_TRY(go(k_partition<false, uint32_t>, (uint32_t*)out_key));
+            EEG_CUDA(cudaGetLastError());
+            in_key = passes == 1 ? nullptr : (uint32_t*)out_key;
+            in_nb = out_nb;
+            in_pay = out_pay;
+            key = out_key;
+            lo += pbits;
         }
-        k_runs<<<grid_for(m, vg->device), B_TPB, 0, st>>>(key[cur], m, rs, re);
+        nb = in_nb;
+        pay = in_pay;
+        // ---- tiles of the buckets, counts per vertex
+        EEG_TRY(T.get((void**)&tstart, sizeof(uint32_t) * ((size_t)nb_buckets + 1)));
+        EEG_TRY(T.get((void**)&tbucket, sizeof(uint32_t) * vtiles));
+        EEG_TRY(T.get((void**)&vcnt, sizeof(uint32_t) * vtiles * S_BINS));
+        if (passes == 1) {
+            bstart = start;  // bins at least the buckets; their starts run on to m
+        } else {
+            EEG_TRY(T.get((void**)&bstart, sizeof(uint32_t) * ((size_t)nb_buckets + 1)));
+            k_bucket_starts<<<grid_for(m + 1, vg->device), B_TPB, 0, st>>>((const uint32_t*)key, m, nb_buckets, bstart);
+        }
+        k_bucket_tiles<<<1, SCAN_TPB, 0, st>>>(bstart, nb_buckets, tstart, tbucket);
+        if (passes == 1)
+            k_vertex_counts<uint16_t><<<(unsigned)vtiles, S_TPB, 0, st>>>((const uint16_t*)key, bstart, tstart, tbucket,
+                                                                          nb_buckets, vcnt);
+        else
+            k_vertex_counts<uint32_t><<<(unsigned)vtiles, S_TPB, 0, st>>>((const uint32_t*)key, bstart, tstart, tbucket,
+                                                                          nb_buckets, vcnt);
+    } else {  // no edges: no tile in any bucket
+        EEG_TRY(T.get((void**)&tstart, sizeof(uint32_t) * ((size_t)nb_buckets + 1)));
+        EEG_CUDA(cudaMemsetAsync(tstart, 0, sizeof(uint32_t) * ((size_t)nb_buckets + 1), st));
     }
-    k_nparts<<<grid_for((uint64_t)n + 1, vg->device), B_TPB, 0, st>>>(rs, re, n, K, d->deg, np, best);
+    k_degrees<<<dim3(grid_for((uint64_t)n, vg->device), 8), 256, 0, st>>>(vcnt, tstart, n, K, d->deg, np, best);
     EEG_TRY(device_scan_u32(np, d->vstart, (uint64_t)n + 1, false, SCAN_ADD, tmp, st));
 
     uint32_t hbuf[4] = {0, 0, 0, 0};
@@ -586,17 +929,17 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
     if (eid) EEG_TRY(vg_alloc(vg, (void**)&d->veid, sizeof(uint32_t) * std::max<size_t>(slots, 4)));
 
     if (P > 0) {
-        EEG_CUDA(cudaMemsetAsync(d->vowner, 0, sizeof(uint32_t) * (size_t)P, st));
-        EEG_CUDA(cudaMemsetAsync(d->vcol, 0xFF, sizeof(uint32_t) * slots, st));
-        if (d->vw) EEG_CUDA(cudaMemsetAsync(d->vw, 0, sizeof(uint32_t) * slots, st));
-        if (d->veid) EEG_CUDA(cudaMemsetAsync(d->veid, 0xFF, sizeof(uint32_t) * slots, st));
-        k_heads<<<grid_for(n, vg->device), B_TPB, 0, st>>>(d->vstart, n, d->vowner);
-        uint32_t* tmp2 = nullptr;
-        EEG_TRY(T.get((void**)&tmp2, sizeof(uint32_t) * (size_t)device_scan_tmp_words(P)));
-        EEG_TRY(device_scan_u32(d->vowner, d->vowner, P, true, SCAN_MAX, tmp2, st));
-        k_place<<<grid_for(m, vg->device), B_TPB, 0, st>>>(key[cur], nb[cur], payload ? wt[cur] : nullptr, m, K, rs,
-                                                            d->vstart, d->vcol, d->vw, with_w ? d_w : nullptr,
-                                                            d->veid, sym ? m_in : 0);
+        k_owners<<<grid_for(n, vg->device), B_TPB, 0, st>>>(n, K, d->vstart, d->deg, d->vowner, d->vcol, d->vw, d->veid);
+        const size_t psm = place_smem(payload);
+        auto go = [&](auto kern, auto* k) -> eeg_status {
+            EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+            kern<<<(unsigned)vtiles, S_TPB, psm, st>>>(k, nb, pay, bstart, tstart, tbucket, nb_buckets, n, K, vcnt,
+                                                             d->vstart, d->vcol, d->vw, with_w ? d_w : nullptr, d->veid,
+                                                             sym ? m_in : 0);
+            return EEG_OK;
+        };
+        if (passes == 1) EEG_TRY(go(k_place<uint16_t>, (const uint16_t*)key));
+        else EEG_TRY(go(k_place<uint32_t>, (const uint32_t*)key));
     }
     EEG_CUDA(cudaGetLastError());
     vg->bytes += sizeof(uint32_t) * ((size_t)(n + 1) * 2 + (size_t)P + slots * (1 + (with_w ? 1 : 0) + (eid ? 1 : 0)));

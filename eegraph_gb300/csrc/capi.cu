@@ -251,10 +251,10 @@ static eeg_status build_impl(uint32_t n, uint64_t m, const uint32_t* src, const 
         return false;
     };
     const uint32_t *ms = nullptr, *md = nullptr, *mw = nullptr;
-    // a two-direction build copies the input once (the copy engine moves it as fast as the in-place
-    // reads) instead of reading it over the host link twice
-    const bool zero_copy = !on_device && m > 0 && !(flags & EEG_VG_REVERSE) && mapped(src, &ms) && mapped(dst, &md) &&
-                           mapped(w, &mw);
+    // a build that reads its input more than once (two directions, both directions of each edge) copies it
+    // once (the copy engine moves it as fast as the in-place reads) instead of reading it over the link twice
+    const bool zero_copy = !on_device && m > 0 && !(flags & EEG_VG_REVERSE) && !symmetrize && mapped(src, &ms) &&
+                           mapped(dst, &md) && mapped(w, &mw);
     cudaEventRecord(e0, st);
     if (zero_copy) {
         ds = ms;
@@ -279,7 +279,7 @@ static eeg_status build_impl(uint32_t n, uint64_t m, const uint32_t* src, const 
         s = build_out_degrees(vg, &vg->fwd, ds, dd, st);
         vg->fwd_parts = false;
     } else {
-        s = build_direction(vg, &vg->fwd, ds, dd, dw, false, st);
+        s = build_direction(vg, &vg->fwd, ds, dd, dw, false, zero_copy, st);
     }
     if (s == EEG_OK && !(flags & EEG_VG_REVERSE) && (flags & (EEG_VG_SYMMETRIC | EEG_VG_SYMMETRIZE))) {
         vg->rev = vg->fwd;  // undirected: in-edges are the out-edges
@@ -287,7 +287,7 @@ static eeg_status build_impl(uint32_t n, uint64_t m, const uint32_t* src, const 
         vg->rev_alias = true;
     }
     if (s == EEG_OK && (flags & EEG_VG_REVERSE)) {
-        s = build_direction(vg, &vg->rev, ds, dd, nullptr, true, st);
+        s = build_direction(vg, &vg->rev, ds, dd, nullptr, true, false, st);
         vg->has_rev = (s == EEG_OK);
     }
     if (tmp) cudaFreeAsync(tmp, st);

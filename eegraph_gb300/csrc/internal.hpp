@@ -166,7 +166,7 @@ void vg_free(eeg_vgraph* vg, void* p);
 
 // builder (builder.cu)
 eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const uint32_t* d_dst,
-                           const uint32_t* d_w, bool reverse, cudaStream_t st);
+                           const uint32_t* d_w, bool reverse, bool host_in, cudaStream_t st);
 // Out-degrees (and the largest, with its vertex) without building the forward parts.
 eeg_status build_out_degrees(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const uint32_t* d_dst, cudaStream_t st);
 
