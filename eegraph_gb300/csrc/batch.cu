@@ -27,13 +27,6 @@ namespace eeg {
 namespace batch {
 
 constexpr int B_TPB = 512;
-// slots whose atomics are issued together in this kernel (single-query kernel: 4): what its 64 registers
-// hold with the query's pointers
-template <int OP>
-__device__ constexpr int atomic_group() {
-    return OP == OP_SSWP ? 2 : 4;
-}
-
 struct BGraph {
     uint32_t n, P, K, pad;
     const uint32_t* vstart;
@@ -98,29 +91,42 @@ struct GridTeam {
     __device__ bool sync() { return grid_barrier(bw, *epoch, timeout_ns); }
 };
 
-constexpr uint32_t ABORTED = 0xFFFFFFFFu;
+constexpr uint32_t ABORTED = 0x80000000u;  // flag beside the rounds run_query returns
 
-// One query (SYNC_PUSH_DD from its source) on `team`; returns its rounds, or ABORTED when a grid barrier
-// gave up. Not inlined, so that each (OP, K, team) body gets its own registers.
+// The query a CTA works on, in shared memory: its fields are read where they are used (a broadcast) instead
+// of living in registers. With them as references to the kernel's parameters and locals, copied to the
+// stack, and the expansion's older form, the hot loops spilled 60-300 bytes.
+struct QCtx {
+    const uint32_t *vstart, *vowner, *vcol, *vw;
+    uint32_t* dist;
+    uint32_t *qa, *qb, *stamp;
+    BCtrl* ctrl;
+    uint32_t* err;
+    uint32_t n, P, source, max_rounds, tag0;
+};
+
+// One query (SYNC_PUSH_DD from its source) on `team`; returns its rounds, with ABORTED set when a grid barrier
+// gave up. Round r uses stamp tag0 + r + 1. Not inlined, so that each (OP, K, team) body gets its own registers.
 template <int OP, int K, class Team>
-__device__ __noinline__ uint32_t run_query(const BArgs& a, const BGraph& g, const BQuery& q, Team team, uint32_t* qa,
-                                           uint32_t* qb, uint32_t* stamp, BCtrl* ctrl, uint32_t& tag, uint32_t* wbuf,
-                                           uint64_t pol) {
-    const uint32_t trank = team.thread_rank(), tsize = team.nthreads();
+__device__ __noinline__ uint32_t run_query(const QCtx& c, Team team, uint32_t* wbuf) {
+    constexpr int KH = K > 8 ? 8 : K;  // slots of a part expanded at a time (trav::k_traverse)
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t crank = team.cta_rank(), ncta = team.ncta();
     __shared__ uint32_t s_next[2];  // per round (alternating): next of this CTA's 32-entry chunks
     if (threadIdx.x == 0) s_next[0] = s_next[1] = 0u;  // ordered before use by the team barrier below
-    const uint32_t lanemask_lt = (1u << lane) - 1u;
-    uint32_t* dist = a.out + q.out_off;
-    for (uint32_t v = trank; v < g.n; v += tsize) dist[v] = trav::init_value<OP>(v, q.source);
-    if (team.leader_cta()) {
-        const uint32_t s0 = g.vstart[q.source], s1 = g.vstart[q.source + 1];
-        for (uint32_t j = threadIdx.x; j < s1 - s0; j += B_TPB) qa[j] = s0 + j;
-        if (threadIdx.x == 0) {
-            ctrl->qparts[0] = s1 - s0;
-            ctrl->qparts[1] = 0u;
-            ctrl->qparts[2] = 0u;
+    const uint64_t pol = l2_evict_first_policy();
+    {
+        const uint32_t tsize = team.nthreads(), n = c.n, source = c.source;
+        uint32_t* dist = c.dist;
+        for (uint32_t v = team.thread_rank(); v < n; v += tsize) dist[v] = trav::init_value<OP>(v, source);
+        if (team.leader_cta()) {
+            const uint32_t s0 = c.vstart[source], s1 = c.vstart[source + 1];
+            for (uint32_t j = threadIdx.x; j < s1 - s0; j += B_TPB) c.qa[j] = s0 + j;
+            if (threadIdx.x == 0) {
+                c.ctrl->qparts[0] = s1 - s0;
+                c.ctrl->qparts[1] = 0u;
+                c.ctrl->qparts[2] = 0u;
+            }
         }
     }
     if (!team.sync()) return ABORTED;
@@ -128,18 +134,17 @@ __device__ __noinline__ uint32_t run_query(const BArgs& a, const BGraph& g, cons
     __shared__ uint32_t s_len;  // the round's queue length, read once per CTA
     for (;; ++it) {
         const uint32_t cur = it % 3u, nxt = (it + 1u) % 3u, old = (it + 2u) % 3u;
-        if (threadIdx.x == 0) s_len = *(volatile uint32_t*)&ctrl->qparts[cur];
+        if (threadIdx.x == 0) s_len = *(volatile uint32_t*)&c.ctrl->qparts[cur];
         __syncthreads();
         uint32_t len = s_len;
-        if (len == 0u || it >= a.max_rounds) break;
-        if (len > g.P) {  // one claim per vertex per round bounds a round by P parts; never read past it
-            if (threadIdx.x == 0) atomicOr(a.err, 1u);
-            len = g.P;
+        if (len == 0u || it >= c.max_rounds) break;
+        if (len > c.P) {  // one claim per vertex per round bounds a round by P parts; never read past it
+            if (threadIdx.x == 0) atomicOr(c.err, 1u);
+            len = c.P;
         }
-        if (team.leader_cta() && threadIdx.x == 0) ctrl->qparts[old] = 0u;
-        ++tag;
-        const uint32_t* qcur = (it & 1u) ? qb : qa;
-        uint32_t* qnext = (it & 1u) ? qa : qb;
+        if (team.leader_cta() && threadIdx.x == 0) c.ctrl->qparts[old] = 0u;
+        const uint32_t* qcur = (it & 1u) ? c.qb : c.qa;
+        uint32_t* qnext = (it & 1u) ? c.qa : c.qb;
         uint32_t wcnt = 0;
         // this CTA's strided share of the round's 32-entry chunks, drawn by its warps from a shared
         // counter; the other counter is reset for the next round (ordered by the team barrier)
@@ -161,89 +166,121 @@ __device__ __noinline__ uint32_t run_query(const BArgs& a, const BGraph& g, cons
             if (ci_next >= my_chunks) break;
             const uint32_t p = p_next;
             ci_next = draw(p_next);
-            const bool valid = p < g.P;
-            uint32_t col[K], wt[K];
+            const bool valid = p < c.P;
+            uint32_t col[KH], wt[KH];
             uint32_t d = 0;
             bool active = false;
             if (valid) {
-                ld_part<K>(g.vcol + (size_t)p * K, col, pol);
+                ld_part<KH>(c.vcol + (size_t)p * K, col, pol);
                 if (OP == OP_BFS) {  // source-seeded BFS: a round's queue holds the vertices at level `it`
                     d = it;
                     active = true;
                 } else {
-                    const uint32_t v = __ldg(&g.vowner[p]);
-                    ld_part<K>(g.vw + (size_t)p * K, wt, pol);
-                    d = __ldcg(&dist[v]);
+                    const uint32_t v = __ldg(&c.vowner[p]);
+                    ld_part<KH>(c.vw + (size_t)p * K, wt, pol);
+                    // plain (L1-cached) value reads, as in k_traverse: the team barrier's acquire makes the
+                    // previous round's values visible, and a value improved later re-enqueues its vertex
+                    d = c.dist[v];
                     active = !trav::unreached<OP>(d);
                 }
             }
-            // every filter read of the part before its first atomic
-            uint32_t cd[K];
+#pragma unroll 1
+            for (int h = 0; h < K / KH; ++h) {
+                if (h > 0 && valid) {
+                    ld_part<KH>(c.vcol + (size_t)p * K + h * KH, col, pol);
+                    if (OP != OP_BFS) ld_part<KH>(c.vw + (size_t)p * K + h * KH, wt, pol);
+                }
+                // every filter read before the first atomic; then what each slot would push, in the place of
+                // its weight, and the slots that pass the filter
+                uint32_t cd[KH];
+                uint32_t* dist = c.dist;
 #pragma unroll
-            for (int i = 0; i < K; ++i) cd[i] = (valid && col[i] != NO_EDGE) ? __ldcg(&dist[col[i]]) : 0u;
-            // the atomics of a group of slots go out before any of their results is used; a won claim
-            // on the round stamp means the target improved in this round (by this lane or after its
-            // filter read), so the winner appends it (the single-query kernel's rule)
-            constexpr int ATB = K < atomic_group<OP>() ? K : atomic_group<OP>();
-#pragma unroll
-            for (int i0 = 0; i0 < K; i0 += ATB) {
-                uint32_t prev[ATB], ex[ATB];
+                for (int i = 0; i < KH; ++i) cd[i] = (valid && col[i] != NO_EDGE) ? dist[col[i]] : 0u;
                 uint32_t hit = 0;
 #pragma unroll
-                for (int j = 0; j < ATB; ++j) {
-                    const int i = i0 + j;
-                    prev[j] = 0u;
-                    ex[j] = tag;
+                for (int i = 0; i < KH; ++i) {
                     if (active && col[i] != NO_EDGE) {
                         const uint32_t nd = trav::relax_value<OP>(d, OP == OP_BFS ? 1u : wt[i]);
-                        if (trav::better<OP>(nd, cd[i])) {
-                            hit |= 1u << j;
-                            prev[j] = trav::atomic_improve<OP>(&dist[col[i]], nd);
-                            if (OP != OP_BFS) ex[j] = atomicExch(&stamp[col[i]], tag);
-                        }
+                        if (trav::better<OP>(nd, cd[i])) hit |= 1u << i;
+                        if (OP != OP_BFS) wt[i] = nd;
                     }
                 }
+                // the atomics of a group of slots go out before any of their results is used; a won claim
+                // on the round stamp means the target improved in this round (by this lane or after its
+                // filter read), so the winner appends it (the single-query kernel's rule)
+                constexpr int ATB = KH < trav::ATOMIC_GROUP ? KH : trav::ATOMIC_GROUP;
 #pragma unroll
-                for (int j = 0; j < ATB; ++j) {
-                    const int i = i0 + j;
-                    bool claim = false;
-                    const uint32_t t = col[i];
-                    if ((hit >> j) & 1u) {
-                        if (OP == OP_BFS)  // atomicMin admits one first improvement
-                            claim = trav::better<OP>(trav::relax_value<OP>(d, 1u), prev[j]);
-                        else
-                            claim = ex[j] != tag;
-                    }
-                    const uint32_t mask = __ballot_sync(0xffffffffu, claim);
-                    if (mask) {
-                        const uint32_t c = __popc(mask);
-                        if (wcnt + c > (uint32_t)trav::WCAP) {
-                            trav::warp_append(g.vstart, &ctrl->qparts[nxt], wbuf, wcnt, qnext, lane, g.P);
-                            wcnt = 0;
+                for (int i0 = 0; i0 < KH; i0 += ATB) {
+                    uint32_t prev[ATB], ex[ATB];
+                    const uint32_t tag = c.tag0 + it + 1u;
+#pragma unroll
+                    for (int j = 0; j < ATB; ++j) {
+                        const int i = i0 + j;
+                        prev[j] = 0u;
+                        ex[j] = tag;
+                        if ((hit >> i) & 1u) {
+                            prev[j] = trav::atomic_improve<OP>(&dist[col[i]], OP == OP_BFS ? d + 1u : wt[i]);
+                            if (OP != OP_BFS) ex[j] = atomicExch(&c.stamp[col[i]], tag);
                         }
-                        if (claim) wbuf[wcnt + __popc(mask & lanemask_lt)] = t;
-                        wcnt += c;
+                    }
+#pragma unroll
+                    for (int j = 0; j < ATB; ++j) {
+                        const int i = i0 + j;
+                        // BFS: atomicMin admits one first improvement
+                        const bool claim = ((hit >> i) & 1u) &&
+                                           (OP == OP_BFS ? trav::better<OP>(d + 1u, prev[j]) : ex[j] != tag);
+                        const uint32_t mask = __ballot_sync(0xffffffffu, claim);
+                        if (mask) {
+                            const uint32_t cn = __popc(mask);
+                            if (wcnt + cn > (uint32_t)trav::WCAP) {
+                                trav::warp_append(c.vstart, &c.ctrl->qparts[nxt], wbuf, wcnt, qnext, lane, c.P);
+                                wcnt = 0;
+                            }
+                            if (claim) wbuf[wcnt + __popc(mask & ((1u << lane) - 1u))] = col[i];
+                            wcnt += cn;
+                        }
                     }
                 }
             }
         }
-        if (wcnt) trav::warp_append(g.vstart, &ctrl->qparts[nxt], wbuf, wcnt, qnext, lane, g.P);
-        if (!team.sync()) return ABORTED;
+        if (wcnt) trav::warp_append(c.vstart, &c.ctrl->qparts[nxt], wbuf, wcnt, qnext, lane, c.P);
+        if (!team.sync()) return it | ABORTED;
     }
     // every CTA has read the final (empty) queue length before the leader initialises the next query
-    if (!team.sync()) return ABORTED;
+    if (!team.sync()) return it | ABORTED;
     return it;
 }
 
+// The query's context into shared memory, then the body for its operator and part size. Called by all threads.
 template <class Team>
-__device__ __forceinline__ uint32_t dispatch(const BArgs& a, const BGraph& g, const BQuery& q, Team team, uint32_t* qa,
-                                             uint32_t* qb, uint32_t* stamp, BCtrl* ctrl, uint32_t& tag, uint32_t* wbuf,
-                                             uint64_t pol) {
-#define EEG_BATCH_K(OPV)                                                                             \
-    switch (g.K) {                                                                                  \
-        case 4: return run_query<OPV, 4, Team>(a, g, q, team, qa, qb, stamp, ctrl, tag, wbuf, pol);  \
-        case 16: return run_query<OPV, 16, Team>(a, g, q, team, qa, qb, stamp, ctrl, tag, wbuf, pol); \
-        default: return run_query<OPV, 8, Team>(a, g, q, team, qa, qb, stamp, ctrl, tag, wbuf, pol);  \
+__device__ __forceinline__ uint32_t dispatch(const BArgs& a, const BQuery& q, Team team, uint32_t* qa, uint32_t* qb,
+                                             uint32_t* stamp, BCtrl* ctrl, uint32_t tag, uint32_t* wbuf, QCtx* c) {
+    const uint32_t K = a.graphs[q.graph].K;
+    __syncthreads();  // the last query's readers are done
+    if (threadIdx.x == 0) {
+        const BGraph g = a.graphs[q.graph];
+        c->vstart = g.vstart;
+        c->vowner = g.vowner;
+        c->vcol = g.vcol;
+        c->vw = g.vw;
+        c->dist = a.out + q.out_off;
+        c->qa = qa;
+        c->qb = qb;
+        c->stamp = stamp;
+        c->ctrl = ctrl;
+        c->err = a.err;
+        c->n = g.n;
+        c->P = g.P;
+        c->source = q.source;
+        c->max_rounds = a.max_rounds;
+        c->tag0 = tag;
+    }
+    __syncthreads();
+#define EEG_BATCH_K(OPV)                                              \
+    switch (K) {                                                      \
+        case 4: return run_query<OPV, 4, Team>(*c, team, wbuf);       \
+        case 16: return run_query<OPV, 16, Team>(*c, team, wbuf);     \
+        default: return run_query<OPV, 8, Team>(*c, team, wbuf);      \
     }
     switch (q.op) {
         case OP_BFS: EEG_BATCH_K(OP_BFS)
@@ -267,8 +304,8 @@ __global__ void __launch_bounds__(B_TPB, 2) k_batch(BArgs a) {
     cg::cluster_group cl = cg::this_cluster();
     const uint32_t csize = cl.num_blocks(), crank = cl.block_rank();
     const uint32_t cid = blockIdx.x / csize;
+    __shared__ QCtx s_ctx;
     uint32_t* wbuf = s_buf[threadIdx.x >> 5];
-    const uint64_t pol = l2_evict_first_policy();
 
     // phase 1: the largest queries, one after another, each on the whole grid
     const uint32_t nbig = min(a.nbig, a.nq);
@@ -278,10 +315,10 @@ __global__ void __launch_bounds__(B_TPB, 2) k_batch(BArgs a) {
         GridTeam gt{a.bw, &epoch, a.timeout_ns};
         for (uint32_t qi = 0; qi < nbig; ++qi) {
             const BQuery q = a.queries[qi];
-            const BGraph g = a.graphs[q.graph];
             const unsigned long long t0 = global_timer_ns();
-            const uint32_t rounds = dispatch(a, g, q, gt, a.tq, a.tq + a.qcap, a.tstamp, a.tctrl, ttag, wbuf, pol);
-            if (rounds == ABORTED) break;
+            const uint32_t rounds = dispatch(a, q, gt, a.tq, a.tq + a.qcap, a.tstamp, a.tctrl, ttag, wbuf, &s_ctx);
+            ttag += (rounds & ~ABORTED) + 1u;
+            if (rounds & ABORTED) break;
             if (blockIdx.x == 0 && threadIdx.x == 0) record(a, q, rounds, t0, ~0ull);
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) a.tctrl->tag = ttag;
@@ -301,9 +338,9 @@ __global__ void __launch_bounds__(B_TPB, 2) k_batch(BArgs a) {
         cl.sync();  // every CTA has read the index before the leader draws the next one
         if (qi >= a.nq) break;
         const BQuery q = a.queries[qi];
-        const BGraph g = a.graphs[q.graph];
         const unsigned long long t0 = global_timer_ns();
-        const uint32_t rounds = dispatch(a, g, q, ct, qa, qb, stamp, ctrl, tag, wbuf, pol);
+        const uint32_t rounds = dispatch(a, q, ct, qa, qb, stamp, ctrl, tag, wbuf, &s_ctx);
+        tag += rounds + 1u;
         if (crank == 0 && threadIdx.x == 0) record(a, q, rounds, t0, cid);
     }
     if (crank == 0 && threadIdx.x == 0) ctrl->tag = tag;
