@@ -470,6 +470,36 @@ eeg_status configure(eeg_batch* b, uint32_t csize) {
     return EEG_OK;
 }
 
+// CTAs per query when the caller leaves the choice open. A query of w edges takes about 39 us of rounds and
+// 1.75 ns w (BFS: 0.4 of it) divided by its CTAs; a batch takes at least its longest query, and all queries'
+// CTA time over the device's CTAs. The longest query of few or uneven ones is what a small cluster waits
+// for, and many small queries pay their rounds once per CTA. Measured against 4 for every batch: 64 graphs of
+// up to 2^18 vertices 4.0 -> 2.8 ms (8), 3 graphs of 2^18-2^20 8.6 -> 4.3 (8), 900 queries on graphs of up
+// to 2^12 0.75 -> 0.40 (1). 4 stays unless another size promises 15 % (between close ones the model is no
+// guide: 148 queries, 8 predicted 4 % faster, 0.28 -> 0.39 ms).
+uint32_t choose_cluster(const eeg_batch* b, const std::vector<BQuery>& queries) {
+    const double ctas = 2.0 * sm_count(b->device);
+    auto model = [&](uint32_t c) {
+        double longest = 0.0, total = 0.0;
+        for (const BQuery& q : queries) {
+            const double w = 1.75e-3 * (double)b->graphs[q.graph]->m * (q.op == OP_BFS ? 0.4 : 1.0);
+            longest = std::max(longest, 39.0 + w / c);
+            total += 39.0 * c + w;
+        }
+        return std::max(longest, total / ctas);
+    };
+    uint32_t best = 4;
+    double t = 0.85 * model(4);
+    for (uint32_t c : {1u, 2u, 8u}) {
+        const double tc = model(c);
+        if (tc < t) {
+            t = tc;
+            best = c;
+        }
+    }
+    return best;
+}
+
 eeg_status capture(eeg_batch* b, uint32_t* out) {
     if (b->exec && b->captured_out == out) return EEG_OK;
     if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -581,7 +611,7 @@ EEG_API eeg_status eeg_batch_set_queries(eeg_batch* b, const eeg_query* queries,
     b->out_words = off;
     b->max_rounds = max_n + 2u;
     if (out_words) *out_words = off;
-    return configure(b, cluster_size ? cluster_size : 4);
+    return configure(b, cluster_size ? cluster_size : choose_cluster(b, hq));
 }
 
 EEG_API eeg_status eeg_batch_query_offset(const eeg_batch* b, uint32_t query, unsigned long long* offset) {

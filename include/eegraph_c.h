@@ -287,7 +287,7 @@ typedef struct eeg_query {
 EEG_API eeg_status eeg_batch_create(eeg_vgraph* const* graphs, uint32_t num_graphs, eeg_batch** out);
 /* Set the queries; *out_words receives the output size: query i writes num_nodes(graph_i) uint32 values
  * at eeg_batch_query_offset(i) (queries laid out in the given order). cluster_size: CTAs per query
- * (1, 2, 4 or 8; 0 = 4). */
+ * (1, 2, 4 or 8; 0 = chosen from the queries' sizes; results are the same). */
 EEG_API eeg_status eeg_batch_set_queries(eeg_batch* b, const eeg_query* queries, uint32_t num_queries,
                                          uint32_t cluster_size, unsigned long long* out_words);
 EEG_API eeg_status eeg_batch_query_offset(const eeg_batch* b, uint32_t query, unsigned long long* offset);
