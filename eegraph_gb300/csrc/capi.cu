@@ -119,6 +119,9 @@ static void free_ws(eeg_vgraph* vg) {
     vg_free(vg, w.dd_amt);
     vg_free(vg, w.dd_taken);
     vg_free(vg, w.dd_pq);
+    vg_free(vg, w.dd_hot);
+    vg_free(vg, w.dd_col);
+    vg_free(vg, w.dd_rep);
     if (w.ddctrl) cudaFree(w.ddctrl);
     if (w.ev[0]) cudaEventDestroy(w.ev[0]);
     if (w.ev[1]) cudaEventDestroy(w.ev[1]);

@@ -23,13 +23,19 @@
 // would not hold the 1e-6 L1 bound); the output is FP32. Tracking which pushes lift a residual past acc
 // instead of scanning needs the atomics' old values: 25 % slower on R-MAT s22 (154.6 against 123.4 ms),
 // every returning FP64 atomic a long-scoreboard wait.
-// Long steps (runs without --accuracy and without a round cap): a round is a Jacobi sweep in residual form
-// on the active vertices, and with the threshold derived from the tolerance nearly all of them stay
-// active for ~135 rounds of 0.84 each. So phase A also sums the taken residuals and compares them with
-// the last round's (the control of common.cuh, whose evidence here is one round old when the step is
-// taken); a round with step length alpha adds alpha t to the value, keeps (1 - alpha) t as residual and
-// pushes alpha times the amount. Residuals may then be negative: |r| is compared with acc. R-MAT s17,
-// K = 8: 10.5 -> 2.3 ms.
+// Long steps (ACC; runs without --accuracy and without a round cap): with the threshold derived from the
+// tolerance nearly every vertex stays active for ~135 rounds of 0.84 each, and a round is a Jacobi sweep in
+// residual form. So these runs take the step lengths of the control in common.cuh (its evidence is one round
+// old when the step is taken): a round with step length alpha adds alpha t to the value, keeps (1 - alpha) t
+// as residual and pushes alpha times the amount. Every residual takes part until none exceeds acc (|r|: they
+// may be negative): with only those above acc, the last decade lost its single mode and some graphs took 60
+// rounds instead of 22-26. So the rounds need no queue: phase A walks the vertices, phase B all parts. A phase
+// A that finds nothing above acc is undone from the recorded residuals. R-MAT s17, K = 8: 10.5 -> 1.2 ms (with the hot targets below).
+// Hot targets: a vertex that takes a large share of the edges receives its pushes on one address, one after
+// another (about 4 ns each: 20 thousand on R-MAT s17's first vertex, 80 of a round's 84 us). Vertices with
+// more than m / 4096 in-edges (and more than 256) therefore collect in 32 places, one per lane, summed when
+// phase A reads the vertex; their ids in a private copy of the targets say so (built once per graph, like
+// the pull sweeps' ranks; none where no vertex is hot). R-MAT s17, K = 8: 2.34 -> HOTNEW ms.
 // The reference's two DD kernels differ only in when a vertex's label is cleared (in the kernel that
 // processes it, or by clearLabel after it); with the residual taken once per round in a phase of its
 // own that makes no difference, so SYNC_PUSH_DD and ASYNC_PUSH_DD run these same rounds.
@@ -41,6 +47,7 @@ namespace eeg {
 namespace {
 
 constexpr int DD_TPB = 512;
+constexpr uint32_t HOT = 0x80000000u;  // private target ids: index of a hot vertex (graphs below 2^31 vertices)
 
 struct DDArgs {
     uint32_t n;
@@ -49,10 +56,14 @@ struct DDArgs {
     const uint32_t* __restrict__ vowner;
     const uint32_t* __restrict__ vcol;
     const uint32_t* __restrict__ deg;
+    const uint32_t* __restrict__ hot;    // nhot hot vertices
+    const uint32_t* __restrict__ hbits;  // bit per vertex: hot
+    uint32_t nhot;
+    double* rep;                         // nhot x 32 partial residuals
     double* r;
     double* xv;
     double* amt;
-    double* taken;  // long steps: the residual each vertex had taken in the last round (0 = inactive)
+    double* taken;  // long steps: each vertex's residual in the last round
     float* x;
     uint32_t* pq;
     PRDDCtrl* ctrl;
@@ -60,7 +71,6 @@ struct DDArgs {
     double damping;
     double base;
     uint32_t max_iters;
-    uint32_t accel;  // long steps
     uint64_t timeout_ns;
 };
 
@@ -94,7 +104,7 @@ __device__ __forceinline__ void append_parts(uint32_t s0, uint32_t np, uint32_t*
     }
 }
 
-template <int K>
+template <int K, bool ACC>
 __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
     __shared__ uint32_t s_len;
     __shared__ double s_red[2][DD_TPB / 32];
@@ -109,12 +119,14 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
     unsigned long long my_pushes = 0, my_parts = 0, my_taken = 0;
     __shared__ Extrapolation s_ex;
     bool stepped = false;  // the last round took a long step
+    double undo = 0.0;     // ACC: step length of a phase A whose residuals are to be put back
     if (threadIdx.x == 0) extrapolation_init(s_ex);
 
     for (uint32_t v = gtid; v < a.n; v += gthreads) {
         a.r[v] = a.base;
         a.xv[v] = 0.0;
     }
+    for (uint32_t i = gtid; i < a.nhot * 32u; i += gthreads) a.rep[i] = 0.0;
     if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) goto finish;
 
     for (;; ++it) {
@@ -133,33 +145,59 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
         const double rho = s_ex.cand != 0.f ? 1.0 - 1.0 / (double)s_ex.cand : 0.0;  // measured for when not 0
         double rs = 0.0, qs = 0.0;
         // ---- phase A: every vertex whose residual exceeds acc takes it (a dense scan of the residuals)
+        uint32_t above = 0;  // ACC: this thread saw a residual above acc
+        // vertex v with residual t: taken when it exceeds acc (ACC: always); its parts [s0, s0 + np) then push
+        auto take = [&](uint32_t v, double t, uint32_t& s0, uint32_t& np) {
+            if (ACC) {
+                if (rho != 0.0) qs += fabs(t - rho * a.taken[v]);
+                a.taken[v] = t;
+                rs += fabs(t);
+                above |= fabs(t) > a.acc ? 1u : 0u;
+                const uint32_t d = __ldg(&a.deg[v]);
+                a.amt[v] = d && t != 0.0 ? a.damping * (alpha * t) / (double)d : 0.0;
+                a.r[v] = (1.0 - alpha) * t;
+                if (t != 0.0) {
+                    a.xv[v] = __ldcg(&a.xv[v]) + alpha * t;
+                    ++my_taken;
+                }
+                return true;
+            }
+            const bool act = t > a.acc;
+            if (act) {
+                a.r[v] = 0.0;
+                a.xv[v] = __ldcg(&a.xv[v]) + t;
+                ++my_taken;
+                const uint32_t d = __ldg(&a.deg[v]);
+                if (d) {
+                    a.amt[v] = a.damping * t / (double)d;
+                    s0 = __ldg(&a.vstart[v]);
+                    np = __ldg(&a.vstart[v + 1]) - s0;
+                }
+            }
+            return act;
+        };
+        for (uint32_t h = gwarp; h < a.nhot; h += nwarps) {  // a warp sums a hot vertex's partial residuals
+            double sum = __ldcg(&a.rep[(size_t)h * 32u + lane]);
+            a.rep[(size_t)h * 32u + lane] = 0.0;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+            uint32_t s0 = 0, np = 0;
+            if (lane == 0) {
+                const uint32_t v = __ldg(&a.hot[h]);
+                const double t = __ldcg(&a.r[v]) + sum;
+                if (!take(v, t, s0, np)) a.r[v] = t;
+            }
+            if (!ACC) append_parts(s0, np, &ctrl->plen[cur], a.pq, a.P, lane);
+        }
         for (uint32_t b0 = gwarp * 32u; b0 < a.n; b0 += nwarps * 32u) {
             const uint32_t v = b0 + lane;
             uint32_t s0 = 0, np = 0;
-            if (v < a.n) {
-                const double t = __ldcg(&a.r[v]);
-                const bool act = fabs(t) > a.acc;
-                if (a.accel) {
-                    const double tk = act ? t : 0.0;
-                    if (rho != 0.0) qs += fabs(tk - rho * a.taken[v]);
-                    a.taken[v] = tk;
-                    rs += fabs(tk);
-                }
-                if (act) {
-                    a.r[v] = (1.0 - alpha) * t;
-                    a.xv[v] = __ldcg(&a.xv[v]) + alpha * t;
-                    ++my_taken;
-                    const uint32_t d = __ldg(&a.deg[v]);
-                    if (d) {
-                        a.amt[v] = a.damping * (alpha * t) / (double)d;
-                        s0 = __ldg(&a.vstart[v]);
-                        np = __ldg(&a.vstart[v + 1]) - s0;
-                    }
-                }
-            }
-            append_parts(s0, np, &ctrl->plen[cur], a.pq, a.P, lane);
+            const uint32_t hb = a.nhot ? __ldg(&a.hbits[b0 >> 5]) : 0u;
+            if (v < a.n && !((hb >> lane) & 1u)) take(v, __ldcg(&a.r[v]), s0, np);
+            if (!ACC) append_parts(s0, np, &ctrl->plen[cur], a.pq, a.P, lane);
         }
-        if (a.accel) {
+        if (ACC) {
+            above = __any_sync(0xffffffffu, above);
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) {
                 rs += __shfl_down_sync(0xffffffffu, rs, off);
@@ -169,8 +207,9 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
                 s_red[0][threadIdx.x >> 5] = rs;
                 s_red[1][threadIdx.x >> 5] = qs;
             }
-            __syncthreads();
+            above = __syncthreads_or(above);
             if (threadIdx.x == 0) {
+                if (above) atomicAdd(&ctrl->plen[cur], 1u);
                 double r2 = 0.0, q2 = 0.0;
                 for (int w = 0; w < DD_TPB / 32; ++w) {
                     r2 += s_red[0][w];
@@ -183,7 +222,7 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
         if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) break;
         if (threadIdx.x == 0) {
             s_len = ld_relaxed(&ctrl->plen[cur]);
-            if (a.accel) {
+            if (ACC) {
                 const double rt = __ldcg(&ctrl->rsum[cur]);
                 if (alpha != 1.0) {  // this round takes the step: rt is the residual before it
                     s_ex.alpha = 1.f;
@@ -199,25 +238,32 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
         __syncthreads();
         uint32_t npq = s_len;
         __syncthreads();
-        if (npq == 0u) break;  // nothing pushes: every residual stays <= acc
-        if (npq > a.P) {
+        if (npq == 0u) {  // nothing pushes: every residual stays <= acc
+            undo = alpha;
+            break;
+        }
+        if (!ACC && npq > a.P) {
             if (blockIdx.x == 0 && threadIdx.x == 0)
                 atomicCAS(&ctrl->bw.status, (uint32_t)DEV_OK, (uint32_t)DEV_OVERFLOW);
             npq = a.P;
         }
         // ---- phase B: push the amounts along the queued parts (reductions: no value comes back)
-        for (uint32_t b0 = gwarp * 32u; b0 < npq; b0 += nwarps * 32u) {
-            const uint32_t i = b0 + lane;
-            if (i < npq) {
+        if (ACC) npq = a.P;
+        for (uint64_t b0 = (uint64_t)gwarp * 32u; b0 < npq; b0 += (uint64_t)nwarps * 32u) {
+            const uint32_t i = (uint32_t)b0 + lane;
+            if (b0 + lane < npq) {
                 uint32_t col[K];
-                const uint32_t p = __ldcg(&a.pq[i]);
+                const uint32_t p = ACC ? i : __ldcg(&a.pq[i]);
                 const double am = __ldcg(&a.amt[__ldg(&a.vowner[p])]);
+                if (ACC && am == 0.0) continue;
                 ld_part<K>(a.vcol + (size_t)p * K, col, pol);
                 ++my_parts;
 #pragma unroll
                 for (int k = 0; k < K; ++k)
                     if (col[k] != NO_EDGE) {
-                        atomicAdd(&a.r[col[k]], am);
+                        double* at = a.r + col[k];
+                        if (a.nhot && (col[k] & HOT)) at = a.rep + (size_t)(col[k] & ~HOT) * 32u + lane;
+                        atomicAdd(at, am);
                         ++my_pushes;
                     }
             }
@@ -229,10 +275,22 @@ finish:
         // the output, and what is left: residual mass (error bound resid / (1-d)) and the value norm
         double rs = 0.0, xs = 0.0;
         for (uint32_t v = gtid; v < a.n; v += gthreads) {
-            const double xv = __ldcg(&a.xv[v]);
+            double xv = __ldcg(&a.xv[v]);
+            double rv = __ldcg(&a.r[v]);
+            if (ACC && undo != 0.0) {
+                rv = __ldcg(&a.taken[v]);
+                xv -= undo * rv;
+            }
             a.x[v] = (float)xv;
-            rs += fabs(__ldcg(&a.r[v]));
+            if (a.nhot && ((__ldg(&a.hbits[v >> 5]) >> (v & 31u)) & 1u)) rv = 0.0;  // counted below
+            rs += fabs(rv);
             xs += xv;
+        }
+        for (uint32_t h = gtid; h < a.nhot; h += gthreads) {  // pushes not taken (the round cap) count too
+            const uint32_t v = __ldg(&a.hot[h]);
+            double rv = ACC && undo != 0.0 ? __ldcg(&a.taken[v]) : __ldcg(&a.r[v]);
+            for (uint32_t l = 0; l < 32u; ++l) rv += __ldcg(&a.rep[(size_t)h * 32u + l]);
+            rs += fabs(rv);
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -263,9 +321,37 @@ finish:
     }
 }
 
+// ---- hot targets (once per graph)
+__global__ void k_dd_indeg(uint64_t slots, const uint32_t* __restrict__ col, uint32_t* cnt) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t c = col[i];
+        if (c != NO_EDGE) atomicAdd(&cnt[c], 1u);
+    }
+}
+// cnt[v] (in-degree) -> v's private id; hot vertices listed in hot[1..], their number in hot[0], bits in hbits
+__global__ void k_dd_hot(uint32_t n, uint32_t limit, uint32_t* cnt, uint32_t* hot, uint32_t* hbits) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        uint32_t id = v;
+        if (cnt[v] > limit) {
+            const uint32_t h = atomicAdd(&hot[0], 1u);
+            hot[1u + h] = v;
+            atomicOr(&hbits[v >> 5], 1u << (v & 31u));
+            id = HOT | h;
+        }
+        cnt[v] = id;
+    }
+}
+__global__ void k_dd_cols(uint64_t slots, const uint32_t* __restrict__ col, const uint32_t* __restrict__ id,
+                          uint32_t* __restrict__ out) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t c = col[i];
+        out[i] = c == NO_EDGE ? NO_EDGE : id[c];
+    }
+}
+
 template <int K>
-eeg_status launch_dd(const DDArgs& a, int device, uint32_t bps, cudaStream_t st) {
-    auto kern = k_pagerank_dd<K>;
+eeg_status launch_dd(const DDArgs& a, bool acc, int device, uint32_t bps, cudaStream_t st) {
+    auto kern = acc ? k_pagerank_dd<K, true> : k_pagerank_dd<K, false>;
     int per_sm = 0;
     EEG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, DD_TPB, 0));
     if (per_sm <= 0) {
@@ -284,6 +370,42 @@ eeg_status launch_dd(const DDArgs& a, int device, uint32_t bps, cudaStream_t st)
 }
 
 }  // namespace
+
+static eeg_status ensure_dd_hot(eeg_vgraph* vg, cudaStream_t st) {
+    Workspace& ws = vg->ws;
+    if (ws.dd_hot_ready) return EEG_OK;
+    const uint64_t slots = vg->fwd.P * vg->K;
+    const uint64_t limit = std::max<uint64_t>(256, vg->m >> 12);  // sum of in-degrees = m: below 4096 hot vertices
+    ws.dd_nhot = 0;
+    if (slots && vg->n < HOT && vg->m > limit) {
+        const size_t words = ((size_t)vg->n + 31) / 32;
+        if (!ws.dd_hot) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_hot, sizeof(uint32_t) * (4097 + words)));
+        uint32_t* cnt = nullptr;
+        EEG_CUDA(cudaMallocAsync((void**)&cnt, sizeof(uint32_t) * vg->n, st));
+        EEG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * vg->n, st));
+        EEG_CUDA(cudaMemsetAsync(ws.dd_hot, 0, sizeof(uint32_t) * (4097 + words), st));
+        const uint64_t cap = (uint64_t)sm_count(vg->device) * 8;
+        const unsigned gs = (unsigned)std::min<uint64_t>((slots + 255) / 256, cap * 2);
+        const unsigned gv = (unsigned)std::min<uint64_t>(((uint64_t)vg->n + 255) / 256, cap);
+        k_dd_indeg<<<gs, 256, 0, st>>>(slots, vg->fwd.vcol, cnt);
+        k_dd_hot<<<gv, 256, 0, st>>>(vg->n, (uint32_t)limit, cnt, ws.dd_hot, ws.dd_hot + 4097);
+        uint32_t nhot = 0;
+        cudaError_t e = cudaMemcpyAsync(&nhot, ws.dd_hot, sizeof(nhot), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        eeg_status s = e == cudaSuccess ? EEG_OK : cuda_fail(e, "data-driven PageRank set-up", __FILE__, __LINE__);
+        if (s == EEG_OK && nhot) {
+            if (!ws.dd_col) s = vg_alloc(vg, (void**)&ws.dd_col, sizeof(uint32_t) * slots);
+            if (s == EEG_OK && !ws.dd_rep) s = vg_alloc(vg, (void**)&ws.dd_rep, sizeof(double) * 32 * (size_t)nhot);
+            if (s == EEG_OK) k_dd_cols<<<gs, 256, 0, st>>>(slots, vg->fwd.vcol, cnt, ws.dd_col);
+        }
+        cudaFreeAsync(cnt, st);
+        EEG_TRY(s);
+        EEG_CUDA(cudaGetLastError());
+        ws.dd_nhot = nhot;
+    }
+    ws.dd_hot_ready = true;
+    return EEG_OK;
+}
 
 eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_options& o, cudaStream_t st,
                            eeg_result* res) {
@@ -313,6 +435,7 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
         EEG_CUDA(cudaEventCreate(&ws.ev[0]));
         EEG_CUDA(cudaEventCreate(&ws.ev[1]));
     }
+    EEG_TRY(ensure_dd_hot(vg, st));
     EEG_CUDA(cudaMemsetAsync(ws.ddctrl, 0, sizeof(PRDDCtrl), st));
     const double damping = o.pr_damping > 0.f ? (double)o.pr_damping : 0.85;
     const double tol = o.pr_tolerance > 0.f ? (double)o.pr_tolerance : 1e-7;
@@ -321,13 +444,16 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
     a.P = (uint32_t)vg->fwd.P;
     a.vstart = vg->fwd.vstart;
     a.vowner = vg->fwd.vowner;
-    a.vcol = vg->fwd.vcol;
+    a.vcol = ws.dd_nhot ? ws.dd_col : vg->fwd.vcol;
     a.deg = vg->fwd.deg;
+    a.nhot = ws.dd_nhot;
+    a.hot = ws.dd_hot ? ws.dd_hot + 1 : nullptr;
+    a.hbits = ws.dd_hot ? ws.dd_hot + 4097 : nullptr;
+    a.rep = ws.dd_rep;
     a.r = ws.dd_r;
     a.xv = ws.dd_x;
     a.amt = ws.dd_amt;
     a.taken = ws.dd_taken;
-    a.accel = accel ? 1u : 0u;
     a.x = ws.x;
     a.pq = ws.dd_pq;
     a.ctrl = ws.ddctrl;
@@ -342,9 +468,9 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
     EEG_CUDA(cudaEventRecord(ws.ev[0], st));
     eeg_status s;
     switch (vg->K) {
-        case 4: s = launch_dd<4>(a, vg->device, o.blocks_per_sm, st); break;
-        case 8: s = launch_dd<8>(a, vg->device, o.blocks_per_sm, st); break;
-        case 16: s = launch_dd<16>(a, vg->device, o.blocks_per_sm, st); break;
+        case 4: s = launch_dd<4>(a, accel, vg->device, o.blocks_per_sm, st); break;
+        case 8: s = launch_dd<8>(a, accel, vg->device, o.blocks_per_sm, st); break;
+        case 16: s = launch_dd<16>(a, accel, vg->device, o.blocks_per_sm, st); break;
         default: set_last_error("K must be 4, 8 or 16"); return EEG_ERR_UNSUPPORTED;
     }
     if (s != EEG_OK) return s;
