@@ -35,7 +35,7 @@
 // another (about 4 ns each: 20 thousand on R-MAT s17's first vertex, 80 of a round's 84 us). Vertices with
 // more than m / 4096 in-edges (and more than 256) therefore collect in 32 places, one per lane, summed when
 // phase A reads the vertex; their ids in a private copy of the targets say so (built once per graph, like
-// the pull sweeps' ranks; none where no vertex is hot). R-MAT s17, K = 8: 2.34 -> HOTNEW ms.
+// the pull sweeps' ranks; none where no vertex is hot). R-MAT s17, K = 8: 2.34 -> 1.84 ms.
 // The reference's two DD kernels differ only in when a vertex's label is cleared (in the kernel that
 // processes it, or by clearLabel after it); with the residual taken once per round in a phase of its
 // own that makes no difference, so SYNC_PUSH_DD and ASYNC_PUSH_DD run these same rounds.

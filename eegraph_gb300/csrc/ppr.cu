@@ -479,19 +479,48 @@ __device__ __forceinline__ void finish_row(const SolveArgs& a, const SweepEnd& e
     }
 }
 
-// 3 CTAs per SM (<= 85 registers, a few spilled): the solve is latency-bound, and 24 warps per SM
-// instead of 16 measured 1.3x faster on R-MAT s20 x 64 columns. NQ = W/4 lanes per row.
-template <int K, int NQ, bool RES>
-__global__ void __launch_bounds__(PPR_TPB, 3) k_ppr_rows(SolveArgs a) {
+// A chunk's neighbour ids and weights (at most 128 each), staged in shared memory while the chunk before is
+// worked on: 16-byte asynchronous copies, four slots per lane and array (rows are 16-byte aligned).
+struct Stage {
+    uint32_t col[PPR_SLOTS];
+    float w[PPR_SLOTS];
+};
+__device__ __forceinline__ void stage_chunk(const DirTab& g, Stage* s, uint32_t p0, uint32_t slots, uint32_t K, uint32_t lane) {
+    if (4u * lane < slots) {
+        const size_t at = (size_t)p0 * K + 4u * lane;
+        const uint32_t dc = (uint32_t)__cvta_generic_to_shared(s->col + 4u * lane);
+        const uint32_t dw = (uint32_t)__cvta_generic_to_shared(s->w + 4u * lane);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dc), "l"(g.vcol + at) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dw), "l"(g.w + at) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The solve is latency-bound: nothing but the row gathers is left on a step's chain of loads -- the chunk's ids
+// and weights come from shared memory, and the next chunk's description, owners, ids and weights are fetched
+// while the current one is gathered; for 64 columns what is the same in the whole grid, and the FP64 sums,
+// are kept in shared memory (8 row gathers take 32 of a lane's registers; 32 columns, whose vertices end twice
+// as often per gather, keep them in registers: 125 against 147 us a sweep). R-MAT s18 x 64 columns, one sweep: 183 us with
+// the ids loaded step by step and 150 bytes spilled, 158 us so with 3 CTAs per SM (24 warps).
+//   CTAS = 4 (64 registers, rare spills): more rows in flight where they come from beyond L2 or its far half:
+// s18 158 -> 155 us, s20 625 -> 575; but s16 51 -> 53, 100 K vertices with K = 16 50 -> 55. So 4 is taken
+// for rows above 48 MB. NQ = W/4 lanes per row.
+constexpr size_t PPR_MANY_ROWS = (size_t)48 << 20;
+template <int K, int NQ, bool RES, int CTAS>
+__global__ void __launch_bounds__(PPR_TPB, CTAS) k_ppr_rows(SolveArgs a) {
     constexpr int G = 32 / NQ;               // lane groups (rows per gather instruction)
     constexpr int H = K / G;                 // slots per group per part
     constexpr int U = RowStep<K, G>::U;      // parts per step: 8 row gathers in flight per lane
+    constexpr bool KEEP = NQ == 8;           // sweep state and sums in registers
     static_assert(H >= 1 && H <= 8, "K must be at least the number of lane groups");
     const uint32_t lane = threadIdx.x & 31u, grp = lane / NQ, q = lane % NQ;
     __shared__ uint32_t s_next[2];  // per sweep (alternating): next of this CTA's chunks
+    __shared__ __align__(16) Stage s_stage[PPR_TPB / 32][2];
     if (threadIdx.x == 0) s_next[0] = s_next[1] = 0u;
     __syncthreads();
-    const uint64_t pol = l2_evict_first_policy();
+    Stage* stage = s_stage[threadIdx.x >> 5];
+    __shared__ SweepEnd s_end;            // this sweep's end of a vertex
+    __shared__ double s_sum[KEEP ? 1 : 3][KEEP ? 1 : PPR_TPB];  // each thread's residual, norm and probe of the sweep
     const float4* b = reinterpret_cast<const float4*>(a.b);
     __shared__ Extrapolation s_ex;
     uint32_t epoch = 0, s = 0;
@@ -522,7 +551,7 @@ __global__ void __launch_bounds__(PPR_TPB, 3) k_ppr_rows(SolveArgs a) {
         }
         if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) goto finish;
         for (; s < a.max_iters || tail; ++s) {
-            SweepEnd e;
+            SweepEnd e;  // the same in every thread; kept in shared memory for the vertices' ends
             e.mode = SW_VALUE;
             e.alpha = 1.f;
             e.out = (s & 1u) ? y0 : y1;
@@ -540,26 +569,49 @@ __global__ void __launch_bounds__(PPR_TPB, 3) k_ppr_rows(SolveArgs a) {
             }
             // the rows whose old values a vertex's end reads; the other sweeps skip the load
             const bool want_old = !RES || e.mode == SW_PROBE || e.mode == SW_STEP;
+            const int mode = e.mode;
             double dr = 0.0, dn = 0.0, dq = 0.0;
+            if (!KEEP) {
+                s_sum[0][threadIdx.x] = s_sum[1][threadIdx.x] = s_sum[2][threadIdx.x] = 0.0;
+                if (threadIdx.x == 0) s_end = e;
+                __syncthreads();
+            }
+            const SweepEnd& end = KEEP ? e : s_end;
             if (threadIdx.x == 0) s_next[(s + 1u) & 1u] = 0u;  // next sweep's; ordered by the sweep's grid barrier
-            for (uint32_t c; (c = next_chunk(&s_next[s & 1u], a.g.nchunks, lane)) != NONE;) {
-                const Chunk ch = a.g.chunk[c];
-                const uint32_t np = ch.p1 - ch.p0;
-                const uint32_t own_l = lane < np ? ld_nc(a.g.vowner + ch.p0 + lane) : NONE;
+            // the next chunk: its parts and hub index (z); no parts when the share is used up
+            auto draw = [&](uint32_t& c, uint3& parts) {
+                c = next_chunk(&s_next[s & 1u], a.g.nchunks, lane);
+                const Chunk h = c != NONE ? a.g.chunk[c] : Chunk{0u, 0u, NONE, 0u};
+                parts = make_uint3(h.p0, h.p1, h.hub);
+            };
+            auto fetch = [&](uint3 parts, uint32_t st) -> uint32_t {  // its rows into stage st; its owners
+                stage_chunk(a.g, stage + st, parts.x, (parts.y - parts.x) * K, K, lane);
+                return lane < parts.y - parts.x ? ld_nc(a.g.vowner + parts.x + lane) : NONE;
+            };
+            uint32_t c, c_next;
+            uint3 parts, parts_next;
+            draw(c, parts);
+            uint32_t sid = 0;
+            uint32_t own_l = fetch(parts, sid);
+            draw(c_next, parts_next);
+            for (; c != NONE; c = c_next, parts = parts_next, draw(c_next, parts_next)) {
+                const uint32_t own_next = fetch(parts_next, sid ^ 1u);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");  // this chunk's stage has landed
+                __syncwarp();
+                const Stage& sg = stage[sid];
+                const uint32_t np = parts.y - parts.x;
                 uint32_t cur = __shfl_sync(FULL, own_l, 0);
                 float4 bv = own[(size_t)cur * NQ + q];
                 float4 ov = want_old ? in[(size_t)cur * NQ + q] : f4(0.f);
                 float4 acc = f4(0.f);
                 float rr = 0.f, nn = 0.f, qq = 0.f;
                 for (uint32_t pp = 0; pp < np; pp += U) {
-                    uint32_t colg[U][H], wbg[U][H];
-                    load_group_slots<K, G>(a.g, ch.p0, pp, np, grp, pol, colg, wbg);
                     float4 xv[U][H];
 #pragma unroll
                     for (int u = 0; u < U; ++u)
 #pragma unroll
                         for (int j = 0; j < H; ++j) {
-                            const uint32_t id = colg[u][j];
+                            const uint32_t id = pp + u < np ? sg.col[(pp + u) * K + j * G + grp] : NONE;
                             xv[u][j] = id != NONE ? in[(size_t)id * NQ + q] : f4(0.f);
                         }
 #pragma unroll
@@ -567,36 +619,46 @@ __global__ void __launch_bounds__(PPR_TPB, 3) k_ppr_rows(SolveArgs a) {
                         if (pp + u < np) {
                             const uint32_t o = __shfl_sync(FULL, own_l, pp + u);
                             if (o != cur) {
-                                finish_row<NQ, RES>(a, e, cur, across_groups<NQ>(acc), bv, ov, grp, q, rr, nn, qq);
+                                finish_row<NQ, RES>(a, end, cur, across_groups<NQ>(acc), bv, ov, grp, q, rr, nn, qq);
                                 acc = f4(0.f);
                                 cur = o;
                                 bv = own[(size_t)cur * NQ + q];
                                 if (want_old) ov = in[(size_t)cur * NQ + q];
                             }
 #pragma unroll
-                            for (int j = 0; j < H; ++j) fma4(acc, __uint_as_float(wbg[u][j]), xv[u][j]);
+                            for (int j = 0; j < H; ++j) fma4(acc, sg.w[(pp + u) * K + j * G + grp], xv[u][j]);
                         }
                     }
                 }
                 const float4 tot = across_groups<NQ>(acc);
-                if (ch.hub == NONE) {
-                    finish_row<NQ, RES>(a, e, cur, tot, bv, ov, grp, q, rr, nn, qq);
+                if (parts.z == NONE) {
+                    finish_row<NQ, RES>(a, end, cur, tot, bv, ov, grp, q, rr, nn, qq);
                 } else {
                     float4 full;
                     uint32_t v;
-                    if (hub_rows<NQ>(a.g, ch, tot, s + 1, lane, full, v))
-                        finish_row<NQ, RES>(a, e, v, full, own[(size_t)v * NQ + q],
+                    if (hub_rows<NQ>(a.g, a.g.chunk[c], tot, s + 1, lane, full, v))
+                        finish_row<NQ, RES>(a, end, v, full, own[(size_t)v * NQ + q],
                                             want_old ? in[(size_t)v * NQ + q] : f4(0.f), grp, q, rr, nn, qq);
                 }
-                dr += (double)rr;
-                dn += (double)nn;
-                if (RES) dq += (double)qq;
+                if (KEEP) {
+                    dr += (double)rr;
+                    dn += (double)nn;
+                    if (RES) dq += (double)qq;
+                } else {
+                    s_sum[0][threadIdx.x] += (double)rr;
+                    s_sum[1][threadIdx.x] += (double)nn;
+                    if (RES) s_sum[2][threadIdx.x] += (double)qq;
+                }
+                own_l = own_next;
+                sid ^= 1u;
+                __syncwarp();  // every lane has read the stage before it is filled again
             }
+            asm volatile("cp.async.wait_all;" ::: "memory");
             if (RES && tail) {  // rows without parts: the value is s b
                 for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < tot;
                      i += (uint64_t)gridDim.x * blockDim.x) {
                     const uint32_t v = (uint32_t)(i / NQ);
-                    if (a.g.vstart[v + 1] == a.g.vstart[v]) e.out[i] = yy[i];
+                    if (a.g.vstart[v + 1] == a.g.vstart[v]) end.out[i] = yy[i];
                 }
                 if (--tail) {
                     if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) goto finish;
@@ -606,7 +668,12 @@ __global__ void __launch_bounds__(PPR_TPB, 3) k_ppr_rows(SolveArgs a) {
                 ++s;
                 break;
             }
-            const int st = end_sweep<RES>(a, s, dr, dn, dq, e.mode, &s_ex, epoch);
+            if (!KEEP) {
+                dr = s_sum[0][threadIdx.x];
+                dn = s_sum[1][threadIdx.x];
+                dq = s_sum[2][threadIdx.x];
+            }
+            const int st = end_sweep<RES>(a, s, dr, dn, dq, mode, &s_ex, epoch);
             if (st == 2) goto finish;
             if (st == 1) {
                 if (RES) {
@@ -938,29 +1005,67 @@ __global__ void k_ppr_scale(uint64_t count, float f, const float* __restrict__ i
 }
 
 // ------------------------------------------------------------------ weights
-// s_u = sum of u's raw out-weights (warp per vertex, fixed order); flags negative / non-finite weights.
-__global__ void k_ppr_out_sums(uint32_t n, uint32_t K, const uint32_t* __restrict__ vstart,
-                               const uint32_t* __restrict__ veid, const float* __restrict__ w, float* __restrict__ s,
-                               uint32_t* bad) {
+// s_u = sum of u's raw out-weights over the forward chunks (a lane owns a slot, as in k_ppr_grad_scalar; a
+// hub's chunks deliver partials: with a warp per vertex, R-MAT s18's first vertex alone took 0.27 ms), in a
+// fixed order; vertices without out-edges keep the zero they were set to. Flags negative / non-finite weights.
+template <int K>
+__global__ void __launch_bounds__(PPR_TPB, 4) k_ppr_out_sums(DirTab g, const uint32_t* __restrict__ veid,
+                                                             const float* __restrict__ w, float* __restrict__ s, uint32_t* bad) {
+    constexpr int PPS = 32 / K;
+    constexpr int STEPS = (int)PPR_SLOTS / 32;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t v = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += nw) {
-        const size_t a0 = (size_t)vstart[v] * K, a1 = (size_t)vstart[v + 1] * K;
-        float acc = 0.f;
-        uint32_t b = 0;
-        for (size_t i = a0 + lane; i < a1; i += 32) {
-            const uint32_t e = veid[i];
-            if (e != NONE) {
-                const float x = w[e];
-                if (!(x >= 0.f) || !isfinite(x)) b = 1;
-                acc += x;
-            }
+    __shared__ uint32_t s_next;
+    if (threadIdx.x == 0) s_next = 0u;
+    __syncthreads();
+    uint32_t wrong = 0;
+    for (uint32_t c; (c = next_chunk(&s_next, g.nchunks, lane)) != NONE;) {
+        const Chunk ch = g.chunk[c];
+        const uint32_t np = ch.p1 - ch.p0, nsl = np * K;
+        const size_t base = (size_t)ch.p0 * K;
+        const uint32_t own_l = lane < np ? ld_nc(g.vowner + ch.p0 + lane) : NONE;
+        uint32_t e[STEPS];
+        float x[STEPS];
+#pragma unroll
+        for (int st = 0; st < STEPS; ++st) {
+            const uint32_t idx = (uint32_t)st * 32u + lane;
+            e[st] = idx < nsl ? ld_nc(veid + base + idx) : NONE;
         }
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
-        if (__any_sync(FULL, b) && lane == 0) atomicOr(bad, 1u);
-        if (lane == 0) s[v] = acc;
+        for (int st = 0; st < STEPS; ++st) x[st] = e[st] != NONE ? __ldg(w + e[st]) : 0.f;
+        float psum = 0.f;
+#pragma unroll
+        for (int st = 0; st < STEPS; ++st) {
+            if (!(x[st] >= 0.f) || !isfinite(x[st])) wrong = 1u;
+            if ((uint32_t)st * 32u < nsl) {
+                float v = x[st];
+#pragma unroll
+                for (int o = K / 2; o >= 1; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+#pragma unroll
+                for (int i = 0; i < PPS; ++i) {
+                    const float t = __shfl_sync(FULL, v, i * K);
+                    if (lane == (uint32_t)(st * PPS + i)) psum = t;
+                }
+            }
+        }
+        const uint32_t prev = __shfl_up_sync(FULL, own_l, 1);
+        const uint32_t hm = __ballot_sync(FULL, lane == 0 || own_l != prev);
+        const uint32_t start = 31u - __clz(hm & (((lane == 31u) ? 0u : (2u << lane)) - 1u));
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_up_sync(FULL, psum, o);
+            if (lane >= (uint32_t)o && lane - (uint32_t)o >= start) psum += t;
+        }
+        if (ch.hub == NONE) {
+            const uint32_t next = __shfl_down_sync(FULL, own_l, 1);
+            if (lane < np && (lane == np - 1 || next != own_l)) s[own_l] = psum;
+        } else {
+            const float tot = __shfl_sync(FULL, psum, np - 1);
+            float full;
+            uint32_t v;
+            if (hub_scalar(g, ch, tot, 1u, lane, full, v) && lane == 0) s[v] = full;
+        }
     }
+    if (__any_sync(FULL, wrong) && lane == 0) atomicOr(bad, 1u);
 }
 // Normalised weight per slot. Forward: the slot's source is the part owner; transposed: the slot's
 // neighbour.
@@ -1141,8 +1246,10 @@ template <int K, bool RES>
 eeg_status launch_solve(eeg_ppr* p, SolveArgs& a, uint32_t bps, cudaStream_t st) {
     const uint64_t work = std::max<uint64_t>(a.g.nchunks, ((uint64_t)a.n * 16 + 31) / 32);
     if (p->W == 1) return launch_coop(k_ppr_scalar<K, RES>, &a, p->vg->device, bps, work, st);
-    if (p->W == 32) return launch_coop(k_ppr_rows<K, 8, RES>, &a, p->vg->device, bps, work, st);
-    return launch_coop(k_ppr_rows<K, 16, RES>, &a, p->vg->device, bps, work, st);
+    if (p->W == 32) return launch_coop(k_ppr_rows<K, 8, RES, 3>, &a, p->vg->device, bps, work, st);
+    if (RES && (size_t)a.n * PPR_W * sizeof(float) > PPR_MANY_ROWS)
+        return launch_coop(k_ppr_rows<K, 16, RES, RES ? 4 : 3>, &a, p->vg->device, bps, work, st);
+    return launch_coop(k_ppr_rows<K, 16, RES, 3>, &a, p->vg->device, bps, work, st);
 }
 
 template <int K>
@@ -1335,8 +1442,15 @@ EEG_API eeg_status eeg_ppr_set_weights(eeg_ppr* p, const float* w, int on_device
     if (vg->m > 0)
         EEG_CUDA(cudaMemcpy(p->w_raw, w, sizeof(float) * vg->m, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
     EEG_CUDA(cudaMemset(p->bad, 0, sizeof(uint32_t)));
-    k_ppr_out_sums<<<grid_1d((uint64_t)vg->n * 32, vg->device), PPR_TPB>>>(vg->n, K, vg->fwd.vstart, vg->fwd.veid,
-                                                                           p->w_raw, p->s, p->bad);
+    EEG_CUDA(cudaMemset(p->s, 0, sizeof(float) * vg->n));
+    EEG_TRY(reset_counters(p->fwd, 0));
+    if (p->fwd.nchunks) {
+        const DirTab g = tab(vg->fwd, p->fwd);
+        const unsigned blocks = grid_1d((uint64_t)p->fwd.nchunks * 32, vg->device);
+        if (K == 4) k_ppr_out_sums<4><<<blocks, PPR_TPB>>>(g, vg->fwd.veid, p->w_raw, p->s, p->bad);
+        else if (K == 8) k_ppr_out_sums<8><<<blocks, PPR_TPB>>>(g, vg->fwd.veid, p->w_raw, p->s, p->bad);
+        else k_ppr_out_sums<16><<<blocks, PPR_TPB>>>(g, vg->fwd.veid, p->w_raw, p->s, p->bad);
+    }
     const uint64_t fs = (uint64_t)vg->fwd.P * K, rs = (uint64_t)vg->rev.P * K;
     if (fs)
         k_ppr_norm<<<grid_1d(fs, vg->device), PPR_TPB>>>(fs, K, 0, vg->fwd.veid, vg->fwd.vowner, vg->fwd.vcol, p->w_raw,
