@@ -302,7 +302,7 @@ __device__ __forceinline__ bool round_barrier(unsigned long long* w, BarrierWord
     return s_ok3 != 0;
 }
 
-// BK (SSSP/SSWP, SYNC_PUSH_DD, delta > 0): bucketed rounds. A claimed vertex whose key (SSSP: distance,
+// Bucketed rounds (SSSP/SSWP, SYNC_PUSH_DD, delta > 0). A claimed vertex whose key (SSSP: distance,
 // SSWP: INF - width; smaller is closer in both) is not below the threshold T waits in a far pile (one
 // entry per vertex, marked by its flag) instead of entering the next queue. When the queue runs empty,
 // a far round sets T = smallest recorded far key + delta and moves every far vertex below T back.
@@ -310,13 +310,16 @@ __device__ __forceinline__ bool round_barrier(unsigned long long* w, BarrierWord
 // current pile travel in control words keyed by round parity, so every CTA (and every host-loop
 // launch) reads the value the previous round settled; three piles rotate so that a pile's length is
 // reset two far rounds before it is written again.
-template <int OP, int K, bool TD, bool BK = false>
+// MODE: SSSP and SSWP, bucketed rounds; BFS, pull rounds. Kernels of their own: either takes registers that the
+// plain rounds need (with the pull code in it, push-only BFS spilled at K = 16 and pull BFS at K = 8).
+template <int OP, int K, bool TD, bool MODE = false>
 __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
     constexpr int T_TPB = trav_tpb<OP>();
+    constexpr bool BKT = MODE && OP != OP_BFS, BFSBU = MODE && OP == OP_BFS;
     __shared__ uint32_t s_buf[TD ? 1 : T_TPB / 32][TD ? 1 : WCAP];
     __shared__ uint2 s_tot[TD ? 1 : T_TPB / 32];
-    __shared__ uint32_t s_far[BK ? T_TPB / 32 : 1][BK ? FCAP : 1];
-    __shared__ uint32_t s_fbase[BK ? T_TPB / 32 : 1], s_fkey[BK ? T_TPB / 32 : 1];
+    __shared__ uint32_t s_far[BKT ? T_TPB / 32 : 1][BKT ? FCAP : 1];
+    __shared__ uint32_t s_fbase[BKT ? T_TPB / 32 : 1], s_fkey[BKT ? T_TPB / 32 : 1];
     __shared__ uint32_t s_next[2];  // per round (alternating): next of this CTA's 32-entry chunks
     __shared__ uint32_t s_ctl[6];   // this round's control words, read once per CTA
 
@@ -326,7 +329,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lanemask_lt = (1u << lane) - 1u;
     uint32_t* wbuf = s_buf[TD ? 0 : threadIdx.x >> 5];
-    uint32_t* fbuf = s_far[BK ? threadIdx.x >> 5 : 0];
+    uint32_t* fbuf = s_far[BKT ? threadIdx.x >> 5 : 0];
     const uint64_t pol = l2_evict_first_policy();
     uint32_t epoch = 0;
 
@@ -358,7 +361,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
     // edges scanned per reached edge 2.03 -> 1.20 and 1.33 -> 1.22 ms on R-MAT s22 (symmetrised).
     // SSSP and SSWP rescan less for it too (1.59 -> 1.21, 1.65 -> 1.19) but take the same time, and the
     // per-part values cost them 15 % more DRAM traffic, so their kernels leave the check out, as does BFS.
-    const bool use_push = OP == OP_CC && !TD && !BK && a.pushed != nullptr;
+    const bool use_push = OP == OP_CC && !TD && !BKT && a.pushed != nullptr;
     constexpr uint32_t PSENT = OP == OP_SSWP ? 0u : 0xFFFFFFFFu;  // no part ever pushes with it
     // Direction-optimising BFS (source-seeded, one persistent launch): when the frontier's parts are many
     // against the parts of the vertices not yet reached (14x), a round pulls instead of pushing -- every
@@ -369,10 +372,9 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
     // lists the ones with in-edges that it left unreached; a later pull round walks the last list only
     // (a superset of the unreached vertices with in-edges, whatever rounds came between). Same levels;
     // R-MAT s22 from the hub pulls in its two large rounds, the second over 6.5 % of the vertices.
-    constexpr bool BFSBU = OP == OP_BFS && !TD && !BK;
     constexpr int KH = K > 8 && trav_tpb<OP>() == 512 ? 8 : K;  // slots of a part expanded at a time
     constexpr int PVL = K <= 8 ? 4 : 2;  // vertices per lane in a pull round, their loads issued together
-    const bool can_bu = BFSBU && bfs_levels && a.rvstart != nullptr && a.rounds_limit == 0;
+    const bool can_bu = BFSBU;  // source-seeded, transposed parts, one persistent launch
     uint32_t seen_parts = 0;  // forward parts of the vertices reached so far
     bool bu = false;          // this round pulls
     uint32_t pj = 0;          // pull rounds so far
@@ -385,11 +387,11 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
         for (uint32_t v = gtid; v < a.n; v += gthreads) {
             a.dist[v] = init_value<OP>(v, a.source);
             if (!TD && !bfs_levels) a.stamp[v] = 0u;
-            if (BK) a.fflag[v] = 0u;
+            if (BKT) a.fflag[v] = 0u;
         }
         if (use_push)
             for (uint32_t q = gtid; q < a.P; q += gthreads) a.pushed[q] = PSENT;
-        if (BK && blockIdx.x == 0 && threadIdx.x == 0) {
+        if (BKT && blockIdx.x == 0 && threadIdx.x == 0) {
             for (int i = 0; i < 3; ++i) {
                 ctrl->fcnt[i] = 0u;
                 ctrl->fmin[i] = 0xFFFFFFFFu;
@@ -424,7 +426,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
             if (first) s_ctl[0] = (uint32_t)ld_relaxed64(&ctrl->queued[cur]);
             if (can_bu || a.activity) s_ctl[5] = ld_relaxed(&ctrl->qverts[cur]);
             if (can_bu) s_ctl[1] = ld_relaxed(&ctrl->lcnt[(pj + 2u) % 3u]);  // the last pull round's list
-            if (BK) {
+            if (BKT) {
                 const uint32_t f = ld_relaxed(&ctrl->fcsel[it & 1u]);
                 uint32_t c[3], m[3];  // every pile's words, not those of pile f after it is known
 #pragma unroll
@@ -438,9 +440,9 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                 s_ctl[4] = f == 0u ? m[0] : (f == 1u ? m[1] : m[2]);
             }
         }
-        if (first || can_bu || a.activity || BK) __syncthreads();
+        if (first || can_bu || a.activity || BKT) __syncthreads();
         uint32_t fc = 0, T = 0xFFFFFFFFu, fcount = 0;
-        if (BK) {
+        if (BKT) {
             fc = s_ctl[1];
             T = s_ctl[2];
             fcount = s_ctl[3];
@@ -472,7 +474,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
         if (BFSBU && bu) len = (uint32_t)(((uint64_t)pcnt + 32u * PVL - 1u) / (32u * PVL) * 32u);
         bool far_round = false;
         if (frontier_empty) {
-            if (!BK || fcount == 0u) break;
+            if (!BKT || fcount == 0u) break;
             if (fcount > a.n) {  // one entry per flagged vertex; never read past the pile
                 if (blockIdx.x == 0 && threadIdx.x == 0)
                     atomicCAS(&ctrl->bw.status, (uint32_t)DEV_OK, (uint32_t)DEV_OVERFLOW);
@@ -491,7 +493,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
             ctrl->queued[old] = 0ull;
             ctrl->qverts[old] = 0u;
             if (BFSBU && bu) ctrl->lcnt[(pj + 1u) % 3u] = 0u;  // the next pull round's list
-            if (BK) {  // what the next round reads; the pile two far rounds back is free again
+            if (BKT) {  // what the next round reads; the pile two far rounds back is free again
                 ctrl->fcsel[(it + 1u) & 1u] = fdst;
                 ctrl->tsel[(it + 1u) & 1u] = T;
                 if (far_round) {
@@ -500,8 +502,8 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                 }
             }
         }
-        const uint32_t* pile_src = BK ? a.fpile + (size_t)fc * a.n : nullptr;
-        uint32_t* pile_dst = BK ? a.fpile + (size_t)fdst * a.n : nullptr;
+        const uint32_t* pile_src = BKT ? a.fpile + (size_t)fc * a.n : nullptr;
+        uint32_t* pile_dst = BKT ? a.fpile + (size_t)fdst * a.n : nullptr;
         uint32_t fcnt = 0, fkmin = 0xFFFFFFFFu;  // fill of the far buffer (warp-uniform); this lane's smallest key
         // Warp-collective: the lanes with `fl` send vertex t (key `key`) to the far pile, through a per-warp
         // buffer: one flag exchange, one reservation and one minimum per slot and warp (each with its
@@ -540,7 +542,12 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
         // A round of at most two chunks per warp is a chain of dependent loads: the part ranges of the
         // claimed vertices are fetched while the chunk is still expanded (BFS on the 2047^2 grid 1.28 ->
         // 1.21 ms). In large rounds the fetches only take L1 from the filter reads (R-MAT s22 BFS +2 %).
-        const bool small = (OP == OP_BFS || BK) && items <= 2u * gthreads;
+        const bool small = ((OP == OP_BFS && !BFSBU) || BKT) && items <= 2u * gthreads;
+        // In such a round of a low-degree graph (about one part per vertex) BFS leaves the filter reads out of
+        // the chain: atomicMin finds out itself, for three or four targets per part, whether one improves
+        // (2047^2 grid 1.07 -> 1.00 ms). In the small rounds of a power-law graph nearly all of a part's eight
+        // targets are reached already, and the filter spares their atomics (R-MAT s22 0.203 ms, 0.211 without).
+        const bool unfiltered = OP == OP_BFS && !TD && bfs_levels && small && a.P - a.P / 8u <= a.n;
         // A pull round's chunks are vertex ranges, and a vertex id's low bits set its degree on R-MAT-like
         // graphs: with chunk b + i * grid (grid = 304 = 16 * 19) a CTA saw the same low bits in every
         // chunk, and CTAs took 115 to 360 thousand cycles over the same chunk counts (R-MAT s22). In a
@@ -579,7 +586,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
             if (ci_next >= my_chunks) break;
             const uint32_t p = p_next;
             ci_next = draw(p_next);
-            if (BK && far_round) {  // far round: p is a far vertex; move it back when below T
+            if (BKT && far_round) {  // far round: p is a far vertex; move it back when below T
                 bool move = false, stay = false;
                 uint32_t key = 0;
                 if (p < a.n && atomicExch(&a.fflag[p], 0u) == 1u) {
@@ -775,7 +782,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                 // almost always live, so their filter reads do not wait for the owner's value.
                 uint32_t cd[KH];
 #pragma unroll
-                for (int i = 0; i < KH; ++i) cd[i] = (fetch && col[i] != NO_EDGE) ? a.dist[col[i]] : 0u;
+                for (int i = 0; i < KH; ++i) cd[i] = unfiltered ? INF : ((fetch && col[i] != NO_EDGE) ? a.dist[col[i]] : 0u);
                 // What each slot would push, in the place of its weight, and the slots that pass the filter: the
                 // filter values and the owner's value are dead before the first atomic (7 % of SSSP's time on
                 // R-MAT s22, where they spilled).
@@ -797,7 +804,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                 // appends the target, whoever improved it, and a target improved in a round is appended
                 // exactly once.
                 // the 384-thread shape has room for a whole part
-                constexpr int ATG = BK ? 2 : (trav_tpb<OP>() == 384 ? 8 : ATOMIC_GROUP);
+                constexpr int ATG = BKT ? 2 : (trav_tpb<OP>() == 384 ? 8 : ATOMIC_GROUP);
                 constexpr int ATB = KH < ATG ? KH : ATG;
 #pragma unroll
                 for (int i0 = 0; i0 < KH; i0 += ATB) {
@@ -831,7 +838,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                             } else {
                                 claim = ex[j] != tag;
                             }
-                            if (BK && claim) {
+                            if (BKT && claim) {
                                 const uint32_t now = imp ? nd : prev[j];  // the target's value after this atomic
                                 const uint32_t key = OP == OP_SSWP ? INF - now : now;
                                 if (key >= T) {  // not in this bucket: wait in the far pile
@@ -841,7 +848,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                                 }
                             }
                         }
-                        if (BK) to_far(far, t, fkey);
+                        if (BKT) to_far(far, t, fkey);
                         if (!TD) {
                             const uint32_t mask = __ballot_sync(0xffffffffu, claim);
                             if (mask) {
@@ -864,7 +871,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
         if (TD) {
             if (__syncthreads_or(changed) && threadIdx.x == 0) atomicAdd(&ctrl->queued[nxt], 1ull);
         } else {
-            if (BK) {  // the far buffers, one reservation per CTA
+            if (BKT) {  // the far buffers, one reservation per CTA
                 constexpr int NW = T_TPB / 32;
                 const uint32_t warp = threadIdx.x >> 5;
                 uint32_t bits = 0, before = 0, tot = 0;
@@ -1002,15 +1009,17 @@ __global__ void __launch_bounds__(512) k_finish(const uint32_t* __restrict__ dis
 
 template <int OP, int K, bool TD>
 eeg_status launch_one(const TravArgs& args, int device, uint32_t blocks_per_sm_req, cudaStream_t st) {
-    constexpr bool CAN_BK = !TD && (OP == OP_SSSP || OP == OP_SSWP);
-    auto kern = (CAN_BK && args.delta && !args.seed_all) ? k_traverse<OP, K, TD, CAN_BK> : k_traverse<OP, K, TD, false>;
+    constexpr bool CAN_MODE = !TD && (OP == OP_SSSP || OP == OP_SSWP || OP == OP_BFS);
+    // bucketed rounds; BFS: pull rounds, from the source in one launch on a graph with transposed parts
+    const bool mode = CAN_MODE && !args.seed_all && (OP == OP_BFS ? args.rvstart && args.rounds_limit == 0 : args.delta != 0u);
+    auto kern = mode ? k_traverse<OP, K, TD, CAN_MODE> : k_traverse<OP, K, TD, false>;
     constexpr int T_TPB = trav_tpb<OP>();
     // The filter reads of dist[] are L1 hits in part, and L1 is what shared memory leaves: ask for the
     // smallest carveout that still holds the two CTAs per SM the kernel is built for (R-MAT s22: SSSP
     // 0.725 -> 0.706 ms, SSWP 0.726 -> 0.709, CC 1.215 -> 1.193 against the CUDA driver's default). The hint
     // and the occupancy belong to the kernel and the device: asked for once (four runtime calls less per run).
     static std::atomic<int> resident[2][64];
-    std::atomic<int>& slot = resident[args.delta && !args.seed_all ? 1 : 0][device & 63];
+    std::atomic<int>& slot = resident[mode ? 1 : 0][device & 63];
     int per_sm = slot.load(std::memory_order_acquire);
     if (per_sm == 0) {
         EEG_TRY(prefer_l1(kern, 2, device));
