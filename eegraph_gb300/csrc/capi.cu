@@ -525,6 +525,18 @@ EEG_API void eeg_vgraph_destroy(eeg_vgraph* vg) {
     delete vg;
 }
 
+// A driver function by name, or null.
+static void* driver_entry(const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion(name, &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+        (void)cudaGetLastError();
+        f = nullptr;
+    }
+    return f;
+}
+
 // True when [p, p + bytes) lies within one 4-byte aligned allocation of `device` that its kernels can
 // write: what a device-to-device copy would accept, checked without making one.
 static bool writable_on(int device, const void* p, size_t bytes) {
@@ -535,18 +547,15 @@ static bool writable_on(int device, const void* p, size_t bytes) {
     }
     if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
     using RangeFn = CUresult(CUDAAPI*)(CUdeviceptr*, size_t*, CUdeviceptr);
-    static const RangeFn range = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            (void)cudaGetLastError();
-            f = nullptr;
-        }
-        return (RangeFn)f;
-    }();
+    using AttrFn = CUresult(CUDAAPI*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const RangeFn range = (RangeFn)driver_entry("cuMemGetAddressRange");
+    static const AttrFn attr = (AttrFn)driver_entry("cuPointerGetAttribute");
     CUdeviceptr base = 0;
     size_t size = 0;
+    unsigned access = 0;  // a mapping may be read-only
+    if (!attr || attr(&access, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, (CUdeviceptr)p) != CUDA_SUCCESS ||
+        access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE)
+        return false;
     if (!range || range(&base, &size, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
     return (CUdeviceptr)p + bytes <= base + size;
 }
