@@ -118,6 +118,7 @@ static void free_ws(eeg_vgraph* vg) {
     vg_free(vg, w.dd_x);
     vg_free(vg, w.dd_amt);
     vg_free(vg, w.dd_taken);
+    vg_free(vg, w.dd_share);
     vg_free(vg, w.dd_pq);
     vg_free(vg, w.dd_hot);
     vg_free(vg, w.dd_col);

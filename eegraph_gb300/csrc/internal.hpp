@@ -126,6 +126,7 @@ struct Workspace {
     double* dd_x = nullptr;       // n: values (FP64 accumulation; the output is written to x)
     double* dd_amt = nullptr;     // n: push amount of each vertex activated in the current round
     double* dd_taken = nullptr;   // n: residual each vertex took in the last round (long steps)
+    double* dd_share = nullptr;   // n: d / outdeg (long steps)
     uint32_t* dd_pq = nullptr;    // P: part queue of the current round
     uint32_t* dd_hot = nullptr;   // hot targets: their number, up to 4096 of them, a bit per vertex
     uint32_t* dd_col = nullptr;   // the targets with hot ones marked (P * K; none without hot targets)

@@ -30,12 +30,20 @@
 // as residual and pushes alpha times the amount. Every residual takes part until none exceeds acc (|r|: they
 // may be negative): with only those above acc, the last decade lost its single mode and some graphs took 60
 // rounds instead of 22-26. So the rounds need no queue: phase A walks the vertices, phase B all parts. A phase
-// A that finds nothing above acc is undone from the recorded residuals. R-MAT s17, K = 8: 10.5 -> 1.2 ms (with the hot targets below).
-// Hot targets: a vertex that takes a large share of the edges receives its pushes on one address, one after
-// another (about 4 ns each: 20 thousand on R-MAT s17's first vertex, 80 of a round's 84 us). Vertices with
-// more than m / 4096 in-edges (and more than 256) therefore collect in 32 places, one per lane, summed when
-// phase A reads the vertex; their ids in a private copy of the targets say so (built once per graph, like
-// the pull sweeps' ranks; none where no vertex is hot). R-MAT s17, K = 8: 2.34 -> 1.84 ms.
+// A that finds nothing above acc is undone from the recorded residuals. R-MAT s17, K = 8:
+// 10.5 -> 0.66 ms (with the hot targets below).
+// Hot targets: reductions to one 128-byte line are done one after another (4 ns each on one address, 1 to 1.5 ns
+// within a line by the times below; on lines of their own 175 G/s), so the pushes to an R-MAT graph's first vertices, which share
+// lines, set the round's time. Vertices with more than m / 32768 in-edges (and more than 64) therefore
+// collect in 32 places, one per lane and each in a line of its own, summed when phase A reads the vertex;
+// their ids in a private copy of the targets say so (built once per graph, like the pull sweeps' ranks;
+// none where no vertex is hot). R-MAT s17, K = 8: 2.34 -> 1.84 ms with a vertex's 32 places side by side and
+// m / 4096; a line each 0.90 -> 0.74 ms, m / 32768 0.66 ms (s20: 4.9 -> 4.3 -> 3.4 ms; m / 8192 and m / 16384
+// lie between; graphs of even degree have no hot vertex and do not change).
+// Phase A of the long steps was bound by FP64 instructions (the unit takes a warp's in about 16 cycles): a
+// division per vertex and round, and ten adds per warp for the two sums. d / outdeg is kept (computed once
+// per run), the CTA's sums are added by two warps, and loads that do not depend on each other go out
+// together: with one-load barrier polls 1.19 -> 0.98 ms (s17), 0.65 -> 0.43 ms (100003 x 12, even degrees).
 // The reference's two DD kernels differ only in when a vertex's label is cleared (in the kernel that
 // processes it, or by clearLabel after it); with the residual taken once per round in a phase of its
 // own that makes no difference, so SYNC_PUSH_DD and ASYNC_PUSH_DD run these same rounds.
@@ -48,6 +56,7 @@ namespace {
 
 constexpr int DD_TPB = 512;
 constexpr uint32_t HOT = 0x80000000u;  // private target ids: index of a hot vertex (graphs below 2^31 vertices)
+constexpr uint32_t HOT_CAP = 32768;
 
 struct DDArgs {
     uint32_t n;
@@ -59,11 +68,13 @@ struct DDArgs {
     const uint32_t* __restrict__ hot;    // nhot hot vertices
     const uint32_t* __restrict__ hbits;  // bit per vertex: hot
     uint32_t nhot;
-    double* rep;                         // nhot x 32 partial residuals
+    uint32_t hstride;                    // nhot rounded up to whole 128-byte lines
+    double* rep;                         // 32 x hstride partial residuals
     double* r;
     double* xv;
     double* amt;
     double* taken;  // long steps: each vertex's residual in the last round
+    double* share;  // long steps: d / outdeg (0 without out-edges)
     float* x;
     uint32_t* pq;
     PRDDCtrl* ctrl;
@@ -108,6 +119,7 @@ template <int K, bool ACC>
 __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
     __shared__ uint32_t s_len;
     __shared__ double s_red[2][DD_TPB / 32];
+    __shared__ double s_sum[2][ACC ? DD_TPB : 1];
     PRDDCtrl* ctrl = a.ctrl;
     const uint32_t gtid = blockIdx.x * DD_TPB + threadIdx.x;
     const uint32_t gthreads = gridDim.x * DD_TPB;
@@ -125,9 +137,13 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
     for (uint32_t v = gtid; v < a.n; v += gthreads) {
         a.r[v] = a.base;
         a.xv[v] = 0.0;
+        if (ACC) {
+            const uint32_t d = __ldg(&a.deg[v]);
+            a.share[v] = d ? a.damping / (double)d : 0.0;
+        }
     }
-    for (uint32_t i = gtid; i < a.nhot * 32u; i += gthreads) a.rep[i] = 0.0;
-    if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) goto finish;
+    for (uint32_t i = gtid; i < a.hstride * 32u; i += gthreads) a.rep[i] = 0.0;
+    if (!grid_barrier_sync(&ctrl->bw, epoch, a.timeout_ns)) goto finish;
 
     for (;; ++it) {
         const uint32_t cur = it % 3u, nxt = (it + 1u) % 3u;
@@ -146,22 +162,8 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
         double rs = 0.0, qs = 0.0;
         // ---- phase A: every vertex whose residual exceeds acc takes it (a dense scan of the residuals)
         uint32_t above = 0;  // ACC: this thread saw a residual above acc
-        // vertex v with residual t: taken when it exceeds acc (ACC: always); its parts [s0, s0 + np) then push
+        // vertex v with residual t: taken when it exceeds acc; its parts [s0, s0 + np) then push
         auto take = [&](uint32_t v, double t, uint32_t& s0, uint32_t& np) {
-            if (ACC) {
-                if (rho != 0.0) qs += fabs(t - rho * a.taken[v]);
-                a.taken[v] = t;
-                rs += fabs(t);
-                above |= fabs(t) > a.acc ? 1u : 0u;
-                const uint32_t d = __ldg(&a.deg[v]);
-                a.amt[v] = d && t != 0.0 ? a.damping * (alpha * t) / (double)d : 0.0;
-                a.r[v] = (1.0 - alpha) * t;
-                if (t != 0.0) {
-                    a.xv[v] = __ldcg(&a.xv[v]) + alpha * t;
-                    ++my_taken;
-                }
-                return true;
-            }
             const bool act = t > a.acc;
             if (act) {
                 a.r[v] = 0.0;
@@ -176,16 +178,37 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
             }
             return act;
         };
-        for (uint32_t h = gwarp; h < a.nhot; h += nwarps) {  // a warp sums a hot vertex's partial residuals
-            double sum = __ldcg(&a.rep[(size_t)h * 32u + lane]);
-            a.rep[(size_t)h * 32u + lane] = 0.0;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+        // ACC: every vertex is taken. Value, share and last residual are loaded beside t.
+        auto step = [&](uint32_t v, double t, double xo, double share, double last) {
+            const double at = alpha != 1.0 ? alpha * t : t;
+            if (rho != 0.0) qs += fabs(t - rho * last);
+            rs += fabs(t);
+            above |= fabs(t) > a.acc ? 1u : 0u;
+            a.taken[v] = t;
+            a.amt[v] = at * share;
+            a.r[v] = alpha != 1.0 ? (1.0 - alpha) * t : 0.0;
+            a.xv[v] = xo + at;
+            my_taken += t != 0.0 ? 1u : 0u;
+        };
+        // hot vertices: a lane sums one vertex's partial residuals (32 vertices per warp, spread over the CTAs)
+        for (uint32_t h0 = (threadIdx.x / 32u * gridDim.x + blockIdx.x) * 32u; h0 < a.nhot; h0 += nwarps * 32u) {
+            const uint32_t h = h0 + lane;
             uint32_t s0 = 0, np = 0;
-            if (lane == 0) {
+            if (h < a.nhot) {
                 const uint32_t v = __ldg(&a.hot[h]);
-                const double t = __ldcg(&a.r[v]) + sum;
-                if (!take(v, t, s0, np)) a.r[v] = t;
+                const double r0 = __ldcg(&a.r[v]), xo = __ldcg(&a.xv[v]);
+                const double share = ACC ? __ldcg(&a.share[v]) : 0.0;
+                const double last = ACC && rho != 0.0 ? __ldcg(&a.taken[v]) : 0.0;
+                double sum = 0.0;
+#pragma unroll 8
+                for (uint32_t l = 0; l < 32u; ++l) sum += __ldcg(&a.rep[(size_t)l * a.hstride + h]);
+#pragma unroll 8
+                for (uint32_t l = 0; l < 32u; ++l) a.rep[(size_t)l * a.hstride + h] = 0.0;
+                const double t = r0 + sum;
+                if (ACC)
+                    step(v, t, xo, share, last);
+                else if (!take(v, t, s0, np))
+                    a.r[v] = t;
             }
             if (!ACC) append_parts(s0, np, &ctrl->plen[cur], a.pq, a.P, lane);
         }
@@ -193,33 +216,38 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
             const uint32_t v = b0 + lane;
             uint32_t s0 = 0, np = 0;
             const uint32_t hb = a.nhot ? __ldg(&a.hbits[b0 >> 5]) : 0u;
-            if (v < a.n && !((hb >> lane) & 1u)) take(v, __ldcg(&a.r[v]), s0, np);
-            if (!ACC) append_parts(s0, np, &ctrl->plen[cur], a.pq, a.P, lane);
-        }
-        if (ACC) {
-            above = __any_sync(0xffffffffu, above);
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                rs += __shfl_down_sync(0xffffffffu, rs, off);
-                qs += __shfl_down_sync(0xffffffffu, qs, off);
-            }
-            if (lane == 0) {
-                s_red[0][threadIdx.x >> 5] = rs;
-                s_red[1][threadIdx.x >> 5] = qs;
-            }
-            above = __syncthreads_or(above);
-            if (threadIdx.x == 0) {
-                if (above) atomicAdd(&ctrl->plen[cur], 1u);
-                double r2 = 0.0, q2 = 0.0;
-                for (int w = 0; w < DD_TPB / 32; ++w) {
-                    r2 += s_red[0][w];
-                    q2 += s_red[1][w];
+            if (ACC) {
+                double t = 0.0, xo = 0.0, share = 0.0, last = 0.0;
+                if (v < a.n) {
+                    t = __ldcg(&a.r[v]);
+                    xo = __ldcg(&a.xv[v]);
+                    share = __ldcg(&a.share[v]);
+                    if (rho != 0.0) last = __ldcg(&a.taken[v]);
                 }
-                atomicAdd(&ctrl->rsum[cur], r2);
-                if (rho != 0.0) atomicAdd(&ctrl->probe[cur], q2);
+                if (v < a.n && !((hb >> lane) & 1u)) step(v, t, xo, share, last);
+            } else {
+                if (v < a.n && !((hb >> lane) & 1u)) take(v, __ldcg(&a.r[v]), s0, np);
+                append_parts(s0, np, &ctrl->plen[cur], a.pq, a.P, lane);
             }
         }
-        if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) break;
+        if (ACC) {  // two warps add the CTA's sums
+            s_sum[0][threadIdx.x] = rs;
+            s_sum[1][threadIdx.x] = qs;
+            above = __syncthreads_or(above);
+            if (threadIdx.x < 64u) {
+                const uint32_t which = threadIdx.x >> 5;
+                double sum = 0.0;
+                if (which == 0u || rho != 0.0) {
+#pragma unroll 4
+                    for (int w = 0; w < DD_TPB / 32; ++w) sum += s_sum[which][w * 32 + lane];
+#pragma unroll
+                    for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+                    if (lane == 0u) atomicAdd(which ? &ctrl->probe[cur] : &ctrl->rsum[cur], sum);
+                }
+                if (threadIdx.x == 0 && above) atomicAdd(&ctrl->plen[cur], 1u);
+            }
+        }
+        if (!grid_barrier_sync(&ctrl->bw, epoch, a.timeout_ns)) break;
         if (threadIdx.x == 0) {
             s_len = ld_relaxed(&ctrl->plen[cur]);
             if (ACC) {
@@ -249,26 +277,36 @@ __global__ void __launch_bounds__(DD_TPB, 2) k_pagerank_dd(DDArgs a) {
         }
         // ---- phase B: push the amounts along the queued parts (reductions: no value comes back)
         if (ACC) npq = a.P;
-        for (uint64_t b0 = (uint64_t)gwarp * 32u; b0 < npq; b0 += (uint64_t)nwarps * 32u) {
-            const uint32_t i = (uint32_t)b0 + lane;
-            if (b0 + lane < npq) {
-                uint32_t col[K];
-                const uint32_t p = ACC ? i : __ldcg(&a.pq[i]);
-                const double am = __ldcg(&a.amt[__ldg(&a.vowner[p])]);
-                if (ACC && am == 0.0) continue;
-                ld_part<K>(a.vcol + (size_t)p * K, col, pol);
+        constexpr int U = K >= 16 ? 1 : 2;  // chunks in flight per warp
+        for (uint64_t b0 = (uint64_t)gwarp * 32u; b0 < npq; b0 += (uint64_t)nwarps * 32u * U) {
+            uint32_t col[U][K];
+            double am[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint64_t i = b0 + (uint64_t)u * nwarps * 32u + lane;
+                am[u] = 0.0;
+                if (i < npq) {
+                    const uint32_t p = ACC ? (uint32_t)i : __ldcg(&a.pq[i]);
+                    const uint32_t owner = __ldg(&a.vowner[p]);
+                    ld_part<K>(a.vcol + (size_t)p * K, col[u], pol);
+                    am[u] = __ldcg(&a.amt[owner]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (am[u] == 0.0) continue;  // past the end, or nothing to push
                 ++my_parts;
 #pragma unroll
                 for (int k = 0; k < K; ++k)
-                    if (col[k] != NO_EDGE) {
-                        double* at = a.r + col[k];
-                        if (a.nhot && (col[k] & HOT)) at = a.rep + (size_t)(col[k] & ~HOT) * 32u + lane;
-                        atomicAdd(at, am);
+                    if (col[u][k] != NO_EDGE) {
+                        double* at = a.r + col[u][k];
+                        if (a.nhot && (col[u][k] & HOT)) at = a.rep + (size_t)lane * a.hstride + (col[u][k] & ~HOT);
+                        atomicAdd(at, am[u]);
                         ++my_pushes;
                     }
             }
         }
-        if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) break;
+        if (!grid_barrier_sync(&ctrl->bw, epoch, a.timeout_ns)) break;
     }
 finish:
     {
@@ -289,7 +327,7 @@ finish:
         for (uint32_t h = gtid; h < a.nhot; h += gthreads) {  // pushes not taken (the round cap) count too
             const uint32_t v = __ldg(&a.hot[h]);
             double rv = ACC && undo != 0.0 ? __ldcg(&a.taken[v]) : __ldcg(&a.r[v]);
-            for (uint32_t l = 0; l < 32u; ++l) rv += __ldcg(&a.rep[(size_t)h * 32u + l]);
+            for (uint32_t l = 0; l < 32u; ++l) rv += __ldcg(&a.rep[(size_t)l * a.hstride + h]);
             rs += fabs(rv);
         }
 #pragma unroll
@@ -371,31 +409,33 @@ eeg_status launch_dd(const DDArgs& a, bool acc, int device, uint32_t bps, cudaSt
 
 }  // namespace
 
+static uint32_t hot_stride(uint32_t nhot) { return (nhot + 15u) / 16u * 16u; }
+
 static eeg_status ensure_dd_hot(eeg_vgraph* vg, cudaStream_t st) {
     Workspace& ws = vg->ws;
     if (ws.dd_hot_ready) return EEG_OK;
     const uint64_t slots = vg->fwd.P * vg->K;
-    const uint64_t limit = std::max<uint64_t>(256, vg->m >> 12);  // sum of in-degrees = m: below 4096 hot vertices
+    const uint64_t limit = std::max<uint64_t>(64, vg->m >> 15);  // sum of in-degrees = m: below HOT_CAP hot vertices
     ws.dd_nhot = 0;
     if (slots && vg->n < HOT && vg->m > limit) {
         const size_t words = ((size_t)vg->n + 31) / 32;
-        if (!ws.dd_hot) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_hot, sizeof(uint32_t) * (4097 + words)));
+        if (!ws.dd_hot) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_hot, sizeof(uint32_t) * (HOT_CAP + 1 + words)));
         uint32_t* cnt = nullptr;
         EEG_CUDA(cudaMallocAsync((void**)&cnt, sizeof(uint32_t) * vg->n, st));
         EEG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * vg->n, st));
-        EEG_CUDA(cudaMemsetAsync(ws.dd_hot, 0, sizeof(uint32_t) * (4097 + words), st));
+        EEG_CUDA(cudaMemsetAsync(ws.dd_hot, 0, sizeof(uint32_t) * (HOT_CAP + 1 + words), st));
         const uint64_t cap = (uint64_t)sm_count(vg->device) * 8;
         const unsigned gs = (unsigned)std::min<uint64_t>((slots + 255) / 256, cap * 2);
         const unsigned gv = (unsigned)std::min<uint64_t>(((uint64_t)vg->n + 255) / 256, cap);
         k_dd_indeg<<<gs, 256, 0, st>>>(slots, vg->fwd.vcol, cnt);
-        k_dd_hot<<<gv, 256, 0, st>>>(vg->n, (uint32_t)limit, cnt, ws.dd_hot, ws.dd_hot + 4097);
+        k_dd_hot<<<gv, 256, 0, st>>>(vg->n, (uint32_t)limit, cnt, ws.dd_hot, ws.dd_hot + HOT_CAP + 1);
         uint32_t nhot = 0;
         cudaError_t e = cudaMemcpyAsync(&nhot, ws.dd_hot, sizeof(nhot), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         eeg_status s = e == cudaSuccess ? EEG_OK : cuda_fail(e, "data-driven PageRank set-up", __FILE__, __LINE__);
         if (s == EEG_OK && nhot) {
             if (!ws.dd_col) s = vg_alloc(vg, (void**)&ws.dd_col, sizeof(uint32_t) * slots);
-            if (s == EEG_OK && !ws.dd_rep) s = vg_alloc(vg, (void**)&ws.dd_rep, sizeof(double) * 32 * (size_t)nhot);
+            if (s == EEG_OK && !ws.dd_rep) s = vg_alloc(vg, (void**)&ws.dd_rep, sizeof(double) * 32 * (size_t)hot_stride(nhot));
             if (s == EEG_OK) k_dd_cols<<<gs, 256, 0, st>>>(slots, vg->fwd.vcol, cnt, ws.dd_col);
         }
         cudaFreeAsync(cnt, st);
@@ -429,6 +469,7 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
     // long steps: the threshold and the schedule are the library's own (no --accuracy, no round cap)
     const bool accel = !(o.pr_accuracy > 0.f) && o.max_iterations == 0;
     if (accel && !ws.dd_taken) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_taken, sizeof(double) * n));
+    if (accel && !ws.dd_share) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_share, sizeof(double) * n));
     if (!ws.dd_pq) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_pq, sizeof(uint32_t) * P));
     if (!ws.ddctrl) EEG_CUDA(cudaMalloc((void**)&ws.ddctrl, sizeof(PRDDCtrl)));
     if (!ws.ev[0]) {
@@ -447,13 +488,15 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
     a.vcol = ws.dd_nhot ? ws.dd_col : vg->fwd.vcol;
     a.deg = vg->fwd.deg;
     a.nhot = ws.dd_nhot;
+    a.hstride = hot_stride(ws.dd_nhot);
     a.hot = ws.dd_hot ? ws.dd_hot + 1 : nullptr;
-    a.hbits = ws.dd_hot ? ws.dd_hot + 4097 : nullptr;
+    a.hbits = ws.dd_hot ? ws.dd_hot + HOT_CAP + 1 : nullptr;
     a.rep = ws.dd_rep;
     a.r = ws.dd_r;
     a.xv = ws.dd_x;
     a.amt = ws.dd_amt;
     a.taken = ws.dd_taken;
+    a.share = ws.dd_share;
     a.x = ws.x;
     a.pq = ws.dd_pq;
     a.ctrl = ws.ddctrl;
