@@ -806,8 +806,8 @@ def bench_ppr(args, emit: bool = True):
                      "traffic": traffic,
                      "dram_achieved": round(traffic / (fkm * 1e-3) / 1e9, 1) if traffic else None,
                      "dram_frac": round(traffic / (fkm * 1e-3) / 1e9 / peak, 4) if traffic else None,
-                     "note": "algorithmic bytes count every row gather as DRAM traffic; at 64 columns about "
-                             "79 % of them hit L2 (traffic = measured DRAM bytes per launch), so frac can exceed 1; "
+                     "note": "algorithmic bytes count every row gather as DRAM traffic; at 64 columns over "
+                             "80 % of them hit L2 (traffic = measured DRAM bytes per launch), so frac can exceed 1; "
                              "dram_frac = measured DRAM bytes per launch / kernel time / peak"},
         "e2e": {"value": round(C_all / (e2e_med * 1e-3), 2) if e2e_med else None, "unit": "PR-grad/s",
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

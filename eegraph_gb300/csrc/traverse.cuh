@@ -10,12 +10,13 @@
 //
 // One cooperative launch runs the whole traversal. Rounds are separated by a bounded grid barrier
 // (common.cuh) instead of a host round trip. A thread expands one part (<= K out-edges of one vertex)
-// with K/4 aligned 128-bit streaming loads of targets and weights.
+// with aligned 128- or 256-bit streaming loads of targets and weights.
 //   TD (topology driven): every round expands every part, as the reference's *_push_td kernels do.
 //      SYNC_PUSH_TD keeps the reference's odd/even partner permutation (src/bfs.cu:196-272).
 //   DD (data driven): the frontier is a queue of PART ids. A vertex whose value improved is claimed
-//      once per round through a round stamp. Each CTA then appends the parts of its claimed vertices
-//      with one atomic reservation per CTA chunk (hub vertices are written by the whole CTA). This
+//      once per round through a round stamp. Claimed vertices collect in per-warp
+//      buffers; what is left at a round's end is appended with one reservation per CTA (a hub's parts are
+//      written by a whole warp). This
 //      replaces label1/label2 + clearLabel; the queue-length counters give --activity (sumLabels).
 //      SYNC_PUSH_DD seeds {source}; ASYNC_PUSH_DD seeds every vertex (src/eegraph.cu:41-49).
 // Values are updated in place with atomicMin/atomicMax, as in the reference; a vertex whose value is
@@ -32,10 +33,11 @@
 namespace eeg {
 namespace trav {
 
-// CTA size per operator, two CTAs per SM: 384 threads (85 registers) for BFS, whose group of atomics
-// then covers a whole 8-slot part; 512 threads (64 registers) for the others. Measured with K = 8:
-// BFS 0.385 against 0.395 ms on R-MAT s22 and 2.2 against 2.6 ms on the 4096^2 grid; CC 1.35 against
-// 1.33 ms, SSSP 0.80 against 0.75 ms and SSWP 0.74 against 0.73 ms at 384 and 512 respectively.
+// CTA size per operator, two CTAs per SM: 384 threads (80 registers) for BFS, whose group of atomics
+// then covers a whole 8-slot part; 512 threads (64 registers) for the others. Measured with K = 8: BFS on
+// the 2047^2 grid 1.00 ms, at 512 threads 1.04; SSSP on R-MAT s22 0.634 ms and BFS on the grid within 1 %
+// with 768 or 1024 threads and one CTA per SM, more at three CTAs of 384 (56 registers); bucketed rounds
+// 5.95 ms on the 4096^2 grid, at 384 threads with 4 or 8 slots in flight 5.85 to 5.90.
 template <int OP>
 __host__ __device__ constexpr int trav_tpb() {
     return OP == OP_BFS ? 384 : 512;
