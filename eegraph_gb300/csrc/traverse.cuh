@@ -202,8 +202,20 @@ __device__ __forceinline__ void warp_flush(const TravArgs& a, const uint32_t* bu
     warp_write(a.vstart, buf, cnt, base + before, qnext, lane, a.P);
 }
 
+// The same vertices' part total, without the parts (a round whose queue is not written).
+__device__ __forceinline__ void warp_count(const TravArgs& a, const uint32_t* buf, uint32_t cnt, uint32_t nxt,
+                                           uint32_t lane) {
+    uint32_t before;
+    const uint32_t total = warp_parts(a.vstart, buf, cnt, lane, &before);
+    if (lane == 0) {
+        atomicAdd(&a.ctrl->queued[nxt], (unsigned long long)total);
+        atomicAdd(&a.ctrl->qverts[nxt], cnt);
+    }
+}
+
 // End of a round: what the CTA's warps still hold, in one reservation per CTA (with one per warp, and the
-// vertices counted always, BFS on the 4096^2 grid took 2.24 ms, against 2.07). Called by all threads.
+// vertices counted always, BFS on the 4096^2 grid took 2.24 ms, against 2.07). Called by all threads; qnext
+// null: counted only.
 template <int NW>
 __device__ __forceinline__ void cta_flush(const TravArgs& a, const uint32_t* buf, uint32_t cnt, uint32_t* qnext,
                                           uint32_t nxt, bool count_verts, uint32_t lane, uint2* s_tot) {
@@ -230,7 +242,7 @@ __device__ __forceinline__ void cta_flush(const TravArgs& a, const uint32_t* buf
         if (lane < NW) s_tot[lane].x = base + inc - t.x;
     }
     __syncthreads();
-    if (cnt) warp_write(a.vstart, buf, cnt, s_tot[warp].x + before, qnext, lane, a.P);
+    if (cnt && qnext) warp_write(a.vstart, buf, cnt, s_tot[warp].x + before, qnext, lane, a.P);
 }
 
 // Bucketed rounds, a warp's buffered far vertices: all flag exchanges go out together; a vertex enters the
@@ -368,8 +380,8 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
     // Direction-optimising BFS (source-seeded, one persistent launch): when the frontier's parts are many
     // against the parts of the vertices not yet reached (14x), a round pulls instead of pushing -- every
     // unreached vertex reads the levels of its in-neighbours from the transposed parts, part by part, and
-    // takes level it+1 at the first one found at level it (its forward parts are appended, so a push
-    // round can follow); rounds push again once the frontier holds fewer than n/12 vertices. Every CTA
+    // takes level it+1 at the first one found at level it (its forward parts are counted and, after the
+    // first pull round, appended, so a push round can follow); rounds push again once the frontier holds fewer than n/12 vertices. Every CTA
     // takes the same decision from the same control words. The first pull round walks every vertex and
     // lists the ones with in-edges that it left unreached; a later pull round walks the last list only
     // (a superset of the unreached vertices with in-edges, whatever rounds came between). Same levels;
@@ -401,7 +413,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
             ctrl->fcsel[0] = 0u;  // round 0 (the source's parts) sends every claim to pile 0 (T = 0)
             ctrl->tsel[0] = 0u;
         }
-        if (BFSBU && blockIdx.x == 0 && threadIdx.x == 0) ctrl->lcnt[0] = ctrl->lcnt[1] = ctrl->lcnt[2] = 0u;
+        if (BFSBU && blockIdx.x == 0 && threadIdx.x == 0) ctrl->lcnt[0] = ctrl->lcnt[1] = ctrl->lcnt[2] = ctrl->fcnt[0] = 0u;
         if (!TD && !a.seed_all && blockIdx.x == 0) {
             const uint32_t s0 = a.vstart[a.source], s1 = a.vstart[a.source + 1];
             for (uint32_t j = threadIdx.x; j < s1 - s0; j += T_TPB) a.q0[j] = s0 + j;
@@ -455,6 +467,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                 a.activity[it - 1] = TD ? produced : s_ctl[5];
             if (produced == 0u && fcount == 0u) break;
         }
+        const bool was_bu = bu;
         if (can_bu) {
             const uint32_t fparts = s_ctl[0], fverts = s_ctl[5];
             seen_parts += fparts;
@@ -503,6 +516,41 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                     ctrl->fmin[(fc + 2u) % 3u] = 0xFFFFFFFFu;
                 }
             }
+        }
+        // The first pull round claims most of the graph, and as a rule the next round pulls too: it counts its
+        // claims' parts but does not write them (R-MAT s22 0.199 -> 0.181 ms; s21 to s16, ef 8 to 32: 1 to 13 %
+        // less). A push round that follows it all the same collects the vertices at its level here: a scan of the levels and one more barrier, once
+        // per run.
+        if (BFSBU && was_bu && !bu && pj == 1u) {
+            uint32_t* q = (it & 1u) ? a.q1 : a.q0;
+            uint32_t cnt = 0;
+            auto put = [&]() {
+                uint32_t before, base = 0;
+                const uint32_t total = warp_parts(a.vstart, wbuf, cnt, lane, &before);
+                if (lane == 0) base = atomicAdd(&ctrl->fcnt[0], total);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                warp_write(a.vstart, wbuf, cnt, base + before, q, lane, a.P);
+                cnt = 0;
+            };
+            for (uint64_t b0 = (uint64_t)(gtid - lane) * 4u; b0 < a.n; b0 += (uint64_t)gthreads * 4u) {
+                bool hit[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint64_t v = b0 + 32u * u + lane;
+                    hit[u] = v < a.n && a.dist[v] == it;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t mask = __ballot_sync(0xffffffffu, hit[u]);
+                    if (!mask) continue;
+                    const uint32_t c = __popc(mask);
+                    if (cnt + c > (uint32_t)WCAP) put();
+                    if (hit[u]) wbuf[cnt + __popc(mask & lanemask_lt)] = (uint32_t)b0 + 32u * u + lane;
+                    cnt += c;
+                }
+            }
+            if (cnt) put();
+            if (!grid_barrier(&ctrl->bw, epoch, a.timeout_ns)) break;
         }
         const uint32_t* pile_src = BKT ? a.fpile + (size_t)fc * a.n : nullptr;
         uint32_t* pile_dst = BKT ? a.fpile + (size_t)fdst * a.n : nullptr;
@@ -706,7 +754,8 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                     if (mask) {
                         const uint32_t cn = __popc(mask);
                         if (wcnt + cn > (uint32_t)WCAP) {
-                            warp_flush(a, wbuf, wcnt, qnext, nxt, can_bu || a.activity, lane);
+                            if (pj > 0u) warp_flush(a, wbuf, wcnt, qnext, nxt, true, lane);
+                            else warp_count(a, wbuf, wcnt, nxt, lane);
                             wcnt = 0;
                         }
                         if (claim[k]) wbuf[wcnt + __popc(mask & lanemask_lt)] = vv[k];
@@ -902,7 +951,7 @@ __global__ void __launch_bounds__(trav_tpb<OP>(), 2) k_traverse(TravArgs a) {
                 __syncthreads();
                 if (fcnt) far_write(a, fbuf, bits, s_fbase[warp] + before, pile_dst, lane);
             }
-            cta_flush<T_TPB / 32>(a, wbuf, wcnt, qnext, nxt, can_bu || a.activity, lane, s_tot);
+            cta_flush<T_TPB / 32>(a, wbuf, wcnt, BFSBU && bu && pj == 0u ? nullptr : qnext, nxt, can_bu || a.activity, lane, s_tot);
         }
         if ((it & 63u) == 63u) stat_round();
         if (BFSBU && bu) ++pj;

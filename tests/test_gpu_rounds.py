@@ -55,3 +55,26 @@ def test_wide_parts(gpu, algo, degree):
         for variant in ("async_push_dd", "async_push_td", "sync_push_td"):
             got, _ = vg.run(algo, variant, 3)
             assert np.array_equal(got, oracle.expected(algo, variant, n, s, d, w, 3)), variant
+
+
+@pytest.mark.parametrize("K", [4, 8, 16])
+@pytest.mark.parametrize("b", [1, 31, 257, 3000])
+def test_push_after_the_first_pull_round(gpu, b, K):
+    """BFS's first pull round only counts its claims' parts; when a push round follows, the queue is collected
+    from the levels. Vertex 0 reaches 4000 vertices with many parts, b of them lead on (too few to pull
+    again: 12 b < n), the first through a vertex of more than 32 parts; two more levels follow. The
+    vertices are numbered at random, so the ones collected lie anywhere."""
+    a, rng = 4000, np.random.default_rng(b)
+    n = 1 + a + 3 * b + 12 * b + 1003
+    A, B, C, D = 1 + np.arange(a), 1 + a + np.arange(b), 1 + a + b + np.arange(b), 1 + a + 2 * b + np.arange(b)
+    pairs = [(np.zeros(a), A), (np.repeat(A, 9), np.zeros(9 * a)), (A[:b], B), (B, C),
+             (np.full(40 * K + 3, B[0]), C[np.arange(40 * K + 3) % b]), (C, D)]
+    name = rng.permutation(n)
+    s, d = (name[np.concatenate([p[i] for p in pairs]).astype(np.int64)].astype(np.uint32) for i in (0, 1))
+    src = int(name[0])
+    want = oracle.bfs(n, s, d, src)
+    with gpu.VirtualGraph.build(n, s, d, None, K=K, reverse=True) as vg:
+        got, res, act = vg.run("bfs", "sync_push_dd", src, activity_cap=16)
+        assert np.array_equal(got, want) and res["pull_rounds"] >= 1
+        ref, res2, act2 = vg.run("bfs", "sync_push_dd", src, activity_cap=16, bfs_push_only=True)
+        assert np.array_equal(ref, want) and res2["pull_rounds"] == 0 and np.array_equal(act, act2)
