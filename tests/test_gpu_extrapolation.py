@@ -131,3 +131,26 @@ def test_ppr_capped_runs_keep_the_plain_iterates(gpu):
             for _ in range(k):
                 want = 0.15 * T + 0.85 * np.stack([np.bincount(d, weights=wn * want[s, c], minlength=n) for c in range(3)], 1)
             assert np.abs(X - want).sum() <= 8 * 2.0 ** -24 / 0.15 * want.sum()
+
+
+@pytest.mark.parametrize("K", [4, 8, 16])
+@pytest.mark.parametrize("hot", [1, 15, 16, 17, 31, 32, 33, 5000])
+def test_pagerank_dd_hot_targets(gpu, hot, K):
+    """Vertices with more than 64 in-edges (here: 70, `hot` of them, anywhere) collect their pushes in 32 places
+    each. The counts lie around a line of places (16), around a warp's vertices (32), and far above. With a
+    threshold the rounds stop at |r|_1 / (1-d) of the fixed point; without one, as above."""
+    rng = np.random.default_rng(hot)
+    n = 20011
+    hubs = rng.permutation(n)[:hot]
+    s = np.concatenate((rng.integers(0, n, 70 * hot), rng.integers(0, n, 2 * n))).astype(np.uint32)
+    d = np.concatenate((np.repeat(hubs, 70), np.repeat(np.arange(n), 2))).astype(np.uint32)
+    dd = 0.85
+    want, _ = oracle.pagerank(n, s, d, damping=dd)
+    with gpu.VirtualGraph.build(n, s, d, None, K=K) as vg:
+        for variant, acc in (("sync_push_dd", 0.0), ("async_push_dd", 0.0), ("sync_push_dd", 1e-4), ("sync_push_dd", 1e-7)):
+            x, res = vg.run("pr", variant, pr_accuracy=acc)
+            err = np.abs(x.astype(np.float64) - want).sum()
+            # 2^-24: the output's rounding; 1e-9: the oracle's own stop and the FP64 sums
+            bound = res["pr_residual"] / (1 - dd) + (2.0 ** -24 + 1e-9) * np.abs(want).sum()
+            assert err <= bound, (variant, acc, err, bound)
+            assert acc > 0 or res["pr_residual"] <= n * 1e-7 * (1 - dd) ** 2 * 1.0001
