@@ -6,6 +6,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include <string>
 
@@ -232,12 +233,13 @@ struct Extrapolation {
     uint32_t steps;   // long steps so far
     uint32_t wait, gap;
     uint32_t off;     // a step failed (the adjoint's estimate can be wrong): plain sweeps from here on
+    uint32_t looks;   // looks at the vertices that found one off (VertexBound)
 };
 __device__ __forceinline__ void extrapolation_init(Extrapolation& e) {
     e.r_prev = e.r_before = 0.0;
     e.alpha = 1.0f;
     e.cand = 0.0f;
-    e.steps = e.wait = e.off = 0u;
+    e.steps = e.wait = e.off = e.looks = 0u;
     e.gap = 1u;
 }
 // After a sweep: its residual norm r, its q (when e.cand was set) and the factor d.
@@ -265,6 +267,55 @@ __device__ __forceinline__ void extrapolation_next(Extrapolation& e, double r, d
     }
     if (e.wait) --e.wait;
     else if (!e.off && rho > 0.3 && rho < 1.0 - 1.0 / 4096.0) e.cand = (float)(rint(64.0 / (1.0 - rho)) / 64.0);
+}
+
+// The bound on single vertices of a run with long steps. Plain sweeps shrink every part of the error alike: when
+// they meet the L1 test, each vertex of a graph whose mass circulates is within about twice the tolerance of its
+// own value. A long step takes out one mode and multiplies what lies far from it by up to
+// 1 + 2d/(1-d) (the alternating modes of small components, stars and paths), and those vertices' share of the
+// L1 norm is too small for its test to see: symmetrised R-MAT s14-s18 ended with vertices 1e-6 to 1e-4 off at
+// tol 1e-7 (plain sweeps: 1.3e-7), and 0.6 % off at 1e-4. So such a run also needs, at every vertex, an error of
+// at most 8 tol |x_v|, estimated from the residual f of its last plain sweep and the one before, fo, as
+//     |f| rho / (1 - rho),    rho = min(|f| / |fo|, d),
+// which overstates it (10 to 100 times on directed R-MAT graphs, where 8 tol is met at once or a sweep later). A run
+// that is not there at the first look has something left of its long steps, and has to come to 3 tol: after a plain
+// sweep, a short step and a plain sweep before each look. A step of length 1 / (1 + z d) takes out what changes by
+// -z d per sweep, and z goes through four values spread over what long steps leave. 1e-8 to 4e-7 was left (64-bit
+// model; directed and symmetrised R-MAT s14-s19, grids, paths), for 5 to 15 more sweeps on symmetrised R-MAT graphs
+// (of 98 plain ones; without the short steps 5 to 34). Past log(tol) / log(d) sweeps, where plain ones would have
+// ended, the L1 test decides alone.
+struct VertexBound {
+    float tol, d;     // the tolerance and the factor
+    uint32_t sweeps;  // asked for up to here
+};
+inline VertexBound vertex_bound(double tol, double d) {
+    VertexBound b{(float)tol, (float)d, 0u};
+    if (tol < 1.0 && d > 0.0 && d < 1.0) {
+        const double s = ceil(log(tol) / log(d));
+        b.sweeps = s < 4e9 ? (uint32_t)s : 0xFFFFFFFFu;
+    }
+    return b;
+}
+// most: the part of |x| that is allowed. fo() is asked for where rho = d does not settle it.
+__device__ __forceinline__ float vertex_part(const VertexBound& b, const Extrapolation& e) {
+    return (e.looks ? 3.f : 8.f) * b.tol;
+}
+template <class Before>
+__device__ __forceinline__ bool vertex_off(float most, float d, float f, float x, Before fo) {
+    f = fabsf(f);
+    most *= fabsf(x);
+    if (f * d <= most * (1.f - d)) return false;
+    const float before = fabsf(fo());
+    return !(f < d * before) || f * f > most * (before - f);
+}
+
+// After a look that found a vertex off: a plain sweep the first time, then a short step.
+__device__ __forceinline__ void vertices_off(Extrapolation& e, double d) {
+    const uint32_t k = e.looks++;
+    const float z = (k & 3u) == 1u ? 0.95f : ((k & 3u) == 2u ? 0.6f : ((k & 3u) == 3u ? 0.1f : -0.4f));
+    e.alpha = k ? 1.f / (1.f + z * (float)d) : 1.f;
+    e.cand = 0.f;
+    e.r_before = 1e300;  // the longest of them (z < 0) may raise the norm: no failed step
 }
 
 // Exclusive CTA-wide sum scan of one uint32 per thread. `s_warp` needs 33 entries.

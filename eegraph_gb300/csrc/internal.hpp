@@ -77,11 +77,10 @@ struct PRCtrl {
     double resid[3];     // ||x_{k+1}-x_k||_1 per sweep (rotating)
     double norm[3];      // ||x_{k+1}||_1 per sweep (rotating)
     double probe[3];     // residual form: ||f_{k+1} - rho f_k||_1 of a measuring sweep (rotating)
+    uint32_t far[3];     // residual form: a value is further from its end than VertexBound allows (rotating)
     uint32_t iterations;
-    uint32_t pad;
     double last_resid;
     double last_norm;
-    unsigned long long edges_scanned;
     unsigned long long zero_in;  // vertices without in-edges (value stays 1-d)
 };
 

@@ -26,8 +26,9 @@
 //   error against 64 bits 1.0e-7 -> 4.7e-8. In value form the same
 //   steps would meet FP32's rounding of x (on a grid the alternating mode then never settles below the
 //   stop test); the residual shrinks, and its rounding with it. The iterate is an FP32 pair
-//   (value, compensation), and after a step the sweeps stop at a quarter of the tolerance, so the result
-//   is closer to the 64-bit fixed point than the plain sweeps leave it.
+//   (value, compensation), and after a step the sweeps stop at a quarter of the tolerance and when every
+//   vertex is within the bound of common.cuh, so the result is as close to the 64-bit fixed point as the
+//   plain sweeps leave it, in the norm and vertex by vertex.
 //   Value form (runs with an explicit sweep cap, whose result after k sweeps is the k-th Jacobi iterate):
 //   SYNC variants double-buffer contrib, ASYNC variants update it in place (values of this sweep are used
 //   as soon as written; order-dependent rounding).
@@ -69,6 +70,7 @@ struct PRArgs {
     double base64;
     float d_hi, d_lo;
     double tol;
+    VertexBound bound;
     uint64_t timeout_ns;
     uint32_t inplace;
 };
@@ -136,6 +138,32 @@ __device__ __forceinline__ void settle_spanning(const PRArgs& a, const uint2* xb
     __syncwarp();
 }
 
+// Looks at every vertex once the L1 test is met (see VertexBound): 0 = some vertex is off, and the control's next
+// step is set for it; 1 = none is; 2 = the grid is aborting. One grid barrier. A pass of its own, 50 us on R-MAT s22
+// (1.6 % of the run; the test in the sweeps themselves cost 3.4 %), and not inlined: that spilled in the gather loop
+// (K = 8: a sweep 246 -> 282 us; so, and without counting the gathered edges there, 249, K = 16 197 -> 195).
+static __device__ __noinline__ int look(uint32_t n, const uint2* __restrict__ info, const float* cnext, const float* ccur,
+                                        const float2* y, VertexBound bound, PRCtrl* ctrl, uint32_t slot, uint32_t epoch,
+                                        uint64_t timeout_ns, Extrapolation* ex, double d) {
+    const float most = vertex_part(bound, *ex);
+    uint32_t far = 0;
+    for (uint32_t v = blockIdx.x * PR_TPB + threadIdx.x; v < n; v += gridDim.x * PR_TPB) {
+        const uint2 inf = __ldg(&info[v]);
+        const float w = inf.y ? (float)inf.y : 1.f;
+        far |= vertex_off(most, bound.d, cnext[inf.x] * w, __ldcg(&y[v]).x, [&]() { return ccur[inf.x] * w; }) ? 1u : 0u;
+    }
+    far = __syncthreads_or(far);
+    if (threadIdx.x == 0 && far) atomicOr(&ctrl->far[slot], 1u);
+    if (!grid_barrier_sync(&ctrl->bw, epoch, timeout_ns)) return 2;
+    __shared__ uint32_t s_far;
+    if (threadIdx.x == 0) {
+        s_far = *(volatile uint32_t*)&ctrl->far[slot];
+        if (s_far) vertices_off(*ex, d);
+    }
+    __syncthreads();
+    return s_far ? 0 : 1;
+}
+
 template <int K, bool RES>
 __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
     constexpr int PR_U = InFlight<K>::U;
@@ -188,7 +216,6 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
     __syncthreads();
     if (threadIdx.x == 0 && s_zero) atomicAdd(&ctrl->zero_in, s_zero);
     uint32_t s = 0;
-    unsigned long long my_edges = 0;
     if (!grid_barrier_sync(&ctrl->bw, epoch, a.timeout_ns)) goto finish;
     {
         const double zero_norm = (double)*(volatile unsigned long long*)&ctrl->zero_in * (double)a.base;
@@ -202,7 +229,10 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 ctrl->resid[(s + 1u) % 3u] = 0.0;
                 ctrl->norm[(s + 1u) % 3u] = 0.0;
-                if (RES) ctrl->probe[(s + 1u) % 3u] = 0.0;
+                if (RES) {
+                    ctrl->probe[(s + 1u) % 3u] = 0.0;
+                    ctrl->far[(s + 1u) % 3u] = 0u;
+                }
             }
             // ccur is read through L1 (plain loads): the grid barrier's acquire makes the previous sweep's
             // values visible, and within a sweep they do not change (SYNC) or may be stale (ASYNC, allowed)
@@ -264,16 +294,13 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
                 // padding slots gather 0 (adding an exact zero leaves the compensated sum unchanged),
                 // so the id registers die here
                 float y[PR_U][K];
-                uint32_t nvalid = 0;
 #pragma unroll
                 for (int u = 0; u < PR_U; ++u)
 #pragma unroll
                     for (int i = 0; i < K; ++i) {
                         const bool ok = valid[u] && col[u][i] != NO_EDGE;
-                        nvalid += ok ? 1u : 0u;
                         y[u][i] = ok ? (col[u][i] < a.hot ? s_hot[col[u][i]] : ccur[col[u][i]]) : 0.f;
                     }
-                my_edges += nvalid;
                 // segment ends: prefetch what finalisation needs while the gathers are in flight
                 bool last[PR_U];
                 float2 xo[PR_U];  // the old value (residual form: its pair)
@@ -384,11 +411,15 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
                     ctrl->last_resid = resid;
                     ctrl->last_norm = norm;
                 }
-                if (step.x == 1.f && a.damping64 / (1.0 - a.damping64) * resid <= tol * norm) {
-                    ++s;
-                    break;
+                if (step.x != 1.f || !(a.damping64 / (1.0 - a.damping64) * resid <= tol * norm)) continue;
+                if (s_ex.steps && s + 1u < a.bound.sweeps) {
+                    const int seen = look(a.n, a.info, cnext, ccur, a.y, a.bound, ctrl, slot, epoch++, a.timeout_ns, &s_ex,
+                                          a.damping64);
+                    if (seen == 0) continue;
+                    if (seen == 2) break;
                 }
-                continue;
+                ++s;
+                break;
             }
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 ctrl->last_resid = resid;
@@ -406,9 +437,6 @@ finish:
             const float2 y = __ldcg(&a.y[v]);
             a.x[v] = __fadd_rn(y.x, y.y);
         }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) my_edges += __shfl_down_sync(0xffffffffu, my_edges, off);
-    if (lane == 0 && my_edges) atomicAdd(&ctrl->edges_scanned, my_edges);
     if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->iterations = s;
 }
 
@@ -605,6 +633,7 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
     a.d_hi = (float)a.damping64;
     a.d_lo = (float)(a.damping64 - (double)a.d_hi);
     a.tol = o.pr_tolerance > 0.f ? (double)o.pr_tolerance : 1e-7;
+    a.bound = vertex_bound(a.tol, a.damping64);
     a.timeout_ns = wait_limit_ns(o);
     a.inplace = (variant == EEG_ASYNC_PUSH_TD || variant == EEG_ASYNC_PUSH_DD) ? 1u : 0u;
 
@@ -626,7 +655,7 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
     if (res) {
         res->kernel_ms = ms;
         res->iterations = hc.iterations;
-        res->edges_scanned = hc.edges_scanned;
+        res->edges_scanned = (uint64_t)hc.iterations * vg->m;  // a sweep gathers along every edge
         res->parts_processed = (uint64_t)hc.iterations * vg->rev.P;
         res->pr_residual = hc.last_resid;
         res->pr_l1_norm = hc.last_norm;
