@@ -285,11 +285,12 @@ __device__ __forceinline__ void extrapolation_next(Extrapolation& e, double r, d
 // (of 98 plain ones; without the short steps 5 to 34). Past log(tol) / log(d) sweeps, where plain ones would have
 // ended, the L1 test decides alone.
 struct VertexBound {
-    float tol, d;     // the tolerance and the factor
-    uint32_t sweeps;  // asked for up to here
+    float first, later;  // the part of |x| that is allowed, at the first look and at the others
+    float d;
+    uint32_t sweeps;     // asked for up to here
 };
-inline VertexBound vertex_bound(double tol, double d) {
-    VertexBound b{(float)tol, (float)d, 0u};
+inline VertexBound vertex_bound(double tol, double d, double first, double later) {
+    VertexBound b{(float)(first * tol), (float)(later * tol), (float)d, 0u};
     if (tol < 1.0 && d > 0.0 && d < 1.0) {
         const double s = ceil(log(tol) / log(d));
         b.sweeps = s < 4e9 ? (uint32_t)s : 0xFFFFFFFFu;
@@ -297,16 +298,16 @@ inline VertexBound vertex_bound(double tol, double d) {
     return b;
 }
 // most: the part of |x| that is allowed. fo() is asked for where rho = d does not settle it.
-__device__ __forceinline__ float vertex_part(const VertexBound& b, const Extrapolation& e) {
-    return (e.looks ? 3.f : 8.f) * b.tol;
-}
-template <class Before>
+// TAIL: two plain sweeps follow, whatever is found here (the estimate shrinks by rho^2).
+template <bool TAIL, class Before>
 __device__ __forceinline__ bool vertex_off(float most, float d, float f, float x, Before fo) {
     f = fabsf(f);
     most *= fabsf(x);
-    if (f * d <= most * (1.f - d)) return false;
+    if (f * (TAIL ? d * d * d : d) <= most * (1.f - d)) return false;
     const float before = fabsf(fo());
-    return !(f < d * before) || f * f > most * (before - f);
+    if (!(f < d * before)) return true;
+    const float rho = f / before;
+    return f * (TAIL ? rho * rho * rho : rho) > most * (1.f - rho);
 }
 
 // After a look that found a vertex off: a plain sweep the first time, then a short step.

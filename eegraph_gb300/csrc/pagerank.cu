@@ -145,12 +145,12 @@ __device__ __forceinline__ void settle_spanning(const PRArgs& a, const uint2* xb
 static __device__ __noinline__ int look(uint32_t n, const uint2* __restrict__ info, const float* cnext, const float* ccur,
                                         const float2* y, VertexBound bound, PRCtrl* ctrl, uint32_t slot, uint32_t epoch,
                                         uint64_t timeout_ns, Extrapolation* ex, double d) {
-    const float most = vertex_part(bound, *ex);
+    const float most = ex->looks ? bound.later : bound.first;
     uint32_t far = 0;
     for (uint32_t v = blockIdx.x * PR_TPB + threadIdx.x; v < n; v += gridDim.x * PR_TPB) {
         const uint2 inf = __ldg(&info[v]);
         const float w = inf.y ? (float)inf.y : 1.f;
-        far |= vertex_off(most, bound.d, cnext[inf.x] * w, __ldcg(&y[v]).x, [&]() { return ccur[inf.x] * w; }) ? 1u : 0u;
+        far |= vertex_off<false>(most, bound.d, cnext[inf.x] * w, __ldcg(&y[v]).x, [&]() { return ccur[inf.x] * w; }) ? 1u : 0u;
     }
     far = __syncthreads_or(far);
     if (threadIdx.x == 0 && far) atomicOr(&ctrl->far[slot], 1u);
@@ -633,7 +633,7 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
     a.d_hi = (float)a.damping64;
     a.d_lo = (float)(a.damping64 - (double)a.d_hi);
     a.tol = o.pr_tolerance > 0.f ? (double)o.pr_tolerance : 1e-7;
-    a.bound = vertex_bound(a.tol, a.damping64);
+    a.bound = vertex_bound(a.tol, a.damping64, 8.0, 3.0);
     a.timeout_ns = wait_limit_ns(o);
     a.inplace = (variant == EEG_ASYNC_PUSH_TD || variant == EEG_ASYNC_PUSH_DD) ? 1u : 0u;
 

@@ -28,6 +28,8 @@
 //   The iterate is accumulated in FP32, so two last value-form sweeps (x = s b + d sum) replace the
 //   rounding of the additions by that of one sweep: relative L2 error of the adjoint at R-MAT s18 in a
 //   CPU model 9.1e-8 without them, 5.2e-8 with one, 2.8e-8 with two (plain sweeps: 1.0e-7).
+//   After long steps a forward solve also ends only when no element is further from its end than the bound of
+//   common.cuh allows (see look()).
 //   Value form (runs with an explicit cap, whose result after k sweeps is the k-th Jacobi iterate).
 // Stop test: d/(1-d) * ||Y_{k+1}-Y_k||_1 <= tol * ||Y_{k+1}||_1 over all columns, reduced in FP64
 // (FP32 per-chunk partials, FP64 per lane and across the grid); everything else is FP32.
@@ -94,6 +96,7 @@ struct SolveArgs {
     PRCtrl* ctrl;
     uint32_t max_iters;
     double tol;
+    VertexBound bound;  // residual form, forward
     uint64_t timeout_ns;
 };
 
@@ -412,13 +415,56 @@ __device__ __forceinline__ int end_sweep(const SolveArgs& a, uint32_t s, double 
         // slot (s+2)%3 was last read before barrier s and is next accumulated after barrier s+1
         ctrl->resid[(s + 2) % 3] = 0.0;
         ctrl->norm[(s + 2) % 3] = 0.0;
-        if (RES) ctrl->probe[(s + 2) % 3] = 0.0;
+        if (RES) {
+            ctrl->probe[(s + 2) % 3] = 0.0;
+            ctrl->far[(s + 2) % 3] = 0u;
+        }
         ctrl->last_resid = resid;
         ctrl->last_norm = norm;
     }
     if (RES && mode == SW_STEP) return 0;  // its residual is that of the step's start
     const double tol = RES && ex->steps ? 0.25 * a.tol : a.tol;
     return ((double)a.d / (1.0 - (double)a.d) * resid <= tol * norm) ? 1 : 0;
+}
+
+// A solve with long steps whose L1 test is met after sweep s looks at every element of its iterate (see
+// VertexBound): 0 = one is off, and the control's next step is set for it; 1 = none is; 2 = the grid is aborting.
+// Forward solves only: their values are sums of one sign, so each has a size of its own to be measured by.
+// (Adjoints, whose values cancel, came out as close as from plain sweeps, element by element, in the same 64-bit
+// model.) Symmetrised R-MAT s14-s17, 32 seeds a column: elements 1e-4 to 1e-3 off without it, 8e-7 with it, 3e-7 to
+// 2e-6 with plain sweeps; 15 to 25 more sweeps. The estimate (before two more plain sweeps) is there 1e-3 and more, on
+// directed graphs mostly below 6e-6 with elements 1e-9 to 6e-8 off: 64 tol at the first look, then 8 tol (at 8 tol
+// from the start directed graphs took one sweep more). The look takes 35 us of 3.4 ms (R-MAT s18, 64 columns). Not
+// inlined: the gather loop needs the registers.
+constexpr double PPR_FIRST = 64.0, PPR_LATER = 8.0;
+static __device__ __noinline__ int look(const SolveArgs& a, uint32_t width, uint32_t s, uint32_t epoch, Extrapolation* ex) {
+    const float most = ex->looks ? a.bound.later : a.bound.first;
+    const float *f = (s & 1u) ? a.y0 : a.y1, *fo = (s & 1u) ? a.y1 : a.y0, *y = a.y;
+    const uint64_t count = (uint64_t)a.n * width;
+    uint32_t far = 0;
+    auto one = [&](float fv, float yv, uint64_t i) {
+        far |= vertex_off<true>(most, a.bound.d, fv, yv, [&]() { return fo[i]; }) ? 1u : 0u;
+    };
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+#pragma unroll 2
+    for (uint64_t i = t0; i < count / 4u; i += step) {
+        const float4 fv = reinterpret_cast<const float4*>(f)[i], yv = reinterpret_cast<const float4*>(y)[i];
+        one(fv.x, yv.x, 4u * i);
+        one(fv.y, yv.y, 4u * i + 1u);
+        one(fv.z, yv.z, 4u * i + 2u);
+        one(fv.w, yv.w, 4u * i + 3u);
+    }
+    for (uint64_t i = count / 4u * 4u + t0; i < count; i += step) one(f[i], y[i], i);
+    far = __syncthreads_or(far);
+    if (threadIdx.x == 0 && far) atomicOr(&a.ctrl->far[s % 3u], 1u);
+    if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) return 2;
+    __shared__ uint32_t s_far;
+    if (threadIdx.x == 0) {
+        s_far = __ldcg(&a.ctrl->far[s % 3u]);
+        if (s_far) vertices_off(*ex, (double)a.d);
+    }
+    __syncthreads();
+    return s_far ? 0 : 1;
 }
 
 // One element of a vertex's end in residual form: yv the iterate's (FIRST: the source row's) old value, fo
@@ -507,7 +553,7 @@ __device__ __forceinline__ void stage_chunk(const DirTab& g, Stage* s, uint32_t 
 // for rows above 48 MB. NQ = W/4 lanes per row.
 constexpr size_t PPR_MANY_ROWS = (size_t)48 << 20;
 template <int K, int NQ, bool RES, int CTAS>
-__global__ void __launch_bounds__(PPR_TPB, CTAS) k_ppr_rows(SolveArgs a) {
+__global__ void __launch_bounds__(PPR_TPB, CTAS) k_ppr_rows(const __grid_constant__ SolveArgs a) {
     constexpr int G = 32 / NQ;               // lane groups (rows per gather instruction)
     constexpr int H = K / G;                 // slots per group per part
     constexpr int U = RowStep<K, G>::U;      // parts per step: 8 row gathers in flight per lane
@@ -677,7 +723,9 @@ __global__ void __launch_bounds__(PPR_TPB, CTAS) k_ppr_rows(SolveArgs a) {
             if (st == 2) goto finish;
             if (st == 1) {
                 if (RES) {
-                    tail = 2u;
+                    const int seen = s_ex.steps && s + 1u < a.bound.sweeps ? look(a, 4u * NQ, s, epoch++, &s_ex) : 1;
+                    if (seen == 2) goto finish;
+                    if (seen == 1) tail = 2u;
                 } else {
                     ++s;
                     conv = true;
@@ -693,7 +741,7 @@ finish:
 
 // ------------------------------------------------------------------ single column: solve
 template <int K, bool RES>
-__global__ void __launch_bounds__(PPR_TPB, 4) k_ppr_scalar(SolveArgs a) {
+__global__ void __launch_bounds__(PPR_TPB, 4) k_ppr_scalar(const __grid_constant__ SolveArgs a) {
     constexpr int PPS = 32 / K;                   // parts per 32-slot step
     constexpr int STEPS = (int)PPR_SLOTS / 32;    // steps per chunk
     const uint32_t lane = threadIdx.x & 31u;
@@ -823,7 +871,9 @@ __global__ void __launch_bounds__(PPR_TPB, 4) k_ppr_scalar(SolveArgs a) {
         if (st == 2) goto finish;
         if (st == 1) {
             if (RES) {
-                tail = 2u;
+                const int seen = s_ex.steps && s + 1u < a.bound.sweeps ? look(a, 1u, s, epoch++, &s_ex) : 1;
+                if (seen == 2) goto finish;
+                if (seen == 1) tail = 2u;
             } else {
                 ++s;
                 conv = true;
@@ -1331,6 +1381,7 @@ eeg_status solve(eeg_ppr* p, bool adjoint, const float* bsrc, const eeg_options&
     a.ctrl = p->ctrl;
     a.max_iters = o.max_iterations ? o.max_iterations : 10000u;
     a.tol = o.pr_tolerance > 0.f ? (double)o.pr_tolerance : 1e-7;
+    if (!adjoint) a.bound = vertex_bound(a.tol, (double)a.d, PPR_FIRST, PPR_LATER);
     a.timeout_ns = wait_limit_ns(o);
     EEG_CUDA(cudaMemsetAsync(p->ctrl, 0, sizeof(PRCtrl), st));
     EEG_TRY(reset_counters(d, st));

@@ -1,4 +1,4 @@
-"""Every vertex's value, not their norm alone: PageRank on graphs with small components, stars and paths, whose
+"""Every vertex's value, not their norm alone: PageRank and personalised PageRank on graphs with small components, stars and paths, whose
 share of the L1 norm is far below the tolerance.
 
 Plain sweeps leave each vertex within about the tolerance of its own value; a run that takes long steps has to
@@ -49,3 +49,32 @@ def test_pagerank_vertex_by_vertex(gpu, name, K):
             assert res["status"] == gpu.OK
             off = np.abs(x.astype(np.float64) - want) / want
             assert off.max() <= 8 * (tol or 1e-7) + 3e-6, (tol, off.max(), res["iterations"])
+
+
+@pytest.mark.parametrize("C,K", [(1, 8), (5, 4), (32, 16), (64, 8)])
+@pytest.mark.parametrize("name", [(12, 16), (16, 16)], ids=str)
+def test_ppr_element_by_element(gpu, name, C, K):
+    """A chunk's row is added up in at most 128 steps and a weight is rounded once per edge of a path: 1e-5."""
+    sp = pytest.importorskip("scipy.sparse")
+    n, s, d = _graph(gpu, name)
+    rng = np.random.default_rng(3)
+    w = (rng.random(len(s)) + 0.05).astype(np.float32)
+    T = np.zeros((n, C), np.float32)
+    for c in range(C):
+        T[rng.integers(0, n, 32), c] += 1 / 32
+    cols = min(C, 5)
+    w64 = w.astype(np.float64)
+    A = sp.csr_matrix((0.85 * w64 / np.bincount(s, w64, n)[s], (d, s)), (n, n))
+    f = want = 0.15 * T[:, :cols].astype(np.float64)
+    while np.abs(f).sum() > 1e-16 * want.sum():
+        f = A @ f
+        want = want + f
+    with gpu.VirtualGraph.build(n, s.astype(np.uint32), d.astype(np.uint32), None, K=K, reverse=True, edge_ids=True) as vg:
+        with gpu.PPR(vg, C) as p:
+            p.set_weights(w)
+            for tol in (0.0, 1e-4):
+                x, _ = p.forward(T, tol=tol)
+                x = x[:, :cols].astype(np.float64)
+                assert np.array_equal(x == 0, want == 0)
+                off = (np.abs(x - want)[want > 0] / want[want > 0]).max()
+                assert off <= 8 * (tol or 1e-7) + 1e-5, (tol, off)
