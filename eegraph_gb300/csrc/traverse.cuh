@@ -285,7 +285,9 @@ __device__ __forceinline__ void far_write(const TravArgs& a, const uint32_t* buf
 // arrivals brings the queue length along, so a round starts without reading control words (one L2 round
 // trip and one CTA barrier less), and the arrival is a release-ordered reduction instead of a fence and an
 // atomic. R-MAT s22 SSSP 0.707 -> 0.667 ms, s20 0.250 -> 0.233, s16 97 -> 91 us. Bounded like grid_barrier
-// (common.cuh); a CTA that gives up sets the word's top bit for the others. Returns false when aborting.
+// (common.cuh); a CTA that gives up sets the word's top bit for the others that wait there and, for those that have
+// gone on to another barrier, the abort word (looked at with the timer, so the common poll costs nothing more).
+// Returns false when aborting.
 __device__ __forceinline__ bool round_barrier(unsigned long long* w, BarrierWords* bw, uint64_t timeout_ns,
                                               uint32_t* s_len) {
     __shared__ uint32_t s_ok3;
@@ -302,11 +304,15 @@ __device__ __forceinline__ bool round_barrier(unsigned long long* w, BarrierWord
             if (arrived & 0x80000000u) { ok = 0; break; }
             if (arrived == gridDim.x) break;
             __nanosleep(32);
-            if ((++spins & 7u) == 0 && global_timer_ns() - t0 > timeout_ns) {
-                atomicCAS(&bw->status, (uint32_t)DEV_OK, (uint32_t)DEV_TIMEOUT);
-                atomicOr(w, 1ull << 63);
-                ok = 0;
-                break;
+            if ((++spins & 7u) == 0) {
+                if (ld_relaxed(&bw->abort)) { ok = 0; break; }
+                if (global_timer_ns() - t0 > timeout_ns) {
+                    atomicCAS(&bw->status, (uint32_t)DEV_OK, (uint32_t)DEV_TIMEOUT);
+                    atomicExch(&bw->abort, 1u);
+                    atomicOr(w, 1ull << 63);
+                    ok = 0;
+                    break;
+                }
             }
         }
         *s_len = (uint32_t)v;
