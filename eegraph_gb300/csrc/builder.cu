@@ -399,6 +399,9 @@ __host__ __device__ constexpr size_t place_tile(bool payload) {
 constexpr size_t partition_smem(uint32_t bins, bool payload) { return partition_tile(bins, payload) + (size_t)bins * (4 + 2); }
 constexpr size_t place_smem(bool payload) { return place_tile(payload) + (size_t)S_BINS * (8 + 2); }
 static_assert(S_WARPS * 4 * 2 % 16 == 0 && S_TILE * 6 % 16 == 0, "16-byte aligned counters");
+// What the kernels are allowed to be launched with belongs to the process: the largest that any build asks for,
+// always, so that builds in several threads do not take it from each other.
+constexpr size_t PARTITION_SMEM = partition_smem(S_BINS, true), PLACE_SMEM = place_smem(true);
 
 // Partition, scatter of one tile: a key's place = its bin's start + the bin's keys in earlier tiles + its rank
 // in the tile. The tile goes through shared memory in bin order, so a bin's run is written by consecutive
@@ -865,7 +868,7 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
             const size_t smem = partition_smem(bins, payload);
             const uint32_t* kin = p == 0 ? copy : in_key;
             auto go = [&](auto kern, auto* kout) -> eeg_status {
-                EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PARTITION_SMEM));
                 kern<<<(unsigned)nt, S_TPB, smem, st>>>(s, kin, in_nb, in_pay, m, lo, bins, hist, csum, start, kout,
                                                             out_nb, out_pay);
                 return EEG_OK;
@@ -932,7 +935,7 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
         k_owners<<<grid_for(n, vg->device), B_TPB, 0, st>>>(n, K, d->vstart, d->deg, d->vowner, d->vcol, d->vw, d->veid);
         const size_t psm = place_smem(payload);
         auto go = [&](auto kern, auto* k) -> eeg_status {
-            EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+            EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PLACE_SMEM));
             kern<<<(unsigned)vtiles, S_TPB, psm, st>>>(k, nb, pay, bstart, tstart, tbucket, nb_buckets, n, K, vcnt,
                                                              d->vstart, d->vcol, d->vw, with_w ? d_w : nullptr, d->veid,
                                                              sym ? m_in : 0);
