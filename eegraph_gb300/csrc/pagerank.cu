@@ -456,7 +456,8 @@ eeg_status launch_pr(const PRArgs& args, bool res, int device, uint32_t bps, uin
     hot = std::min<size_t>(hot, hot_limit ? hot_limit : PR_HOT_DEFAULT);
     a.hot = (uint32_t)(hot & ~(size_t)3);
     const size_t dyn = (size_t)a.hot * sizeof(float);
-    EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    // the limit belongs to the process: always the largest, so that runs in several threads do not lower it for each other
+    EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
     int per_sm = 0;
     EEG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PR_TPB, dyn));
     if (per_sm <= 0) {

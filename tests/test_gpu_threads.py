@@ -42,3 +42,24 @@ def test_builds_with_and_without_weights(gpu):
         return go
 
     _in_threads([job(500, True), job(700, False), job(5000, True), job(40000, False)])
+
+
+def test_pagerank_of_small_and_large_graphs(gpu):
+    """The sweeps' shared memory follows the number of vertices."""
+    def job(n, reps=150):
+        rng = np.random.default_rng(n)
+        s, d = rng.integers(0, n, 4 * n, dtype=np.uint32), rng.integers(0, n, 4 * n, dtype=np.uint32)
+        vg = gpu.VirtualGraph.build(n, s, d, None, K=8, reverse_only=True)
+
+        def go():
+            gpu.lib().eeg_set_device(0)
+            first = None
+            for _ in range(reps):
+                x, res = vg.run("pr", "sync_push_td")
+                assert res["status"] == gpu.OK
+                first = x if first is None else first
+                assert np.allclose(x, first, rtol=1e-5)
+            vg.close()
+        return go
+
+    _in_threads([job(300), job(3000), job(50000)])
