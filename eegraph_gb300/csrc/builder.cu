@@ -12,6 +12,8 @@
 //   3. part counts  np[v] = ceil(deg[v] / K); vstart = exclusive scan; vstart[n] = P
 //   4. owners       vowner of every part, unused slots of a vertex's last part
 //   5. placement    stable, each tile: edge of rank r of vertex v -> slot vstart[v]*K + r (part r/K)
+// A sparse graph (see sorted_by_vertex) is partitioned by all bits of the owner id instead: 2. is then the runs of
+// equal owners, and 5. an edge's place in its run.
 // What bounds it is memory traffic: 8-bit radix passes over all 22 bits, a preparing copy, run detection,
 // cleared slots and a separate placement moved 9.7 GB for 67 M weighted edges; this moves 4 GB (2.95 ->
 // 1.98 ms from device arrays; now the tile kernels' shared-memory and store throughput, 0.65 ms each).
@@ -572,6 +574,65 @@ __global__ void __launch_bounds__(256) k_degrees(uint32_t* cnt, const uint32_t* 
     if (lane == 0u && mine) atomicMax(best, mine);
 }
 
+// Edges sorted by vertex: first[v] = v's first edge, end[v] = one past its last; vertices without edges keep the zero
+// that end was cleared to.
+__global__ void k_runs(const uint32_t* __restrict__ key, uint64_t m, uint32_t* __restrict__ first, uint32_t* __restrict__ end) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t v = key[i];
+        if (i == 0 || key[i - 1] != v) first[v] = (uint32_t)i;
+        if (i + 1 == m || key[i + 1] != v) end[v] = (uint32_t)i + 1u;
+    }
+}
+// end[v] -> deg[v] (in place), np[v] = ceil(deg/K) (np[n] = 0) and the max-degree vertex (lowest id among ties). Four
+// vertices per thread; where they have no edges, nothing but np is written.
+__global__ void __launch_bounds__(256) k_run_degrees(const uint32_t* __restrict__ first, uint32_t n, uint32_t K,
+                                                     uint32_t* __restrict__ deg, uint32_t* __restrict__ np,
+                                                     unsigned long long* __restrict__ best) {
+    unsigned long long mine = 0;
+    auto one = [&](uint32_t v, uint32_t e) {
+        if (!e) return 0u;
+        const uint32_t d = e - first[v];
+        deg[v] = d;
+        const unsigned long long key = ((unsigned long long)d << 32) | (unsigned long long)(0xFFFFFFFFu - v);
+        mine = key > mine ? key : mine;
+        return (d + K - 1) / K;
+    };
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = t0; i < n / 4u; i += step) {  // both arrays are 256-byte aligned
+        const uint4 e = reinterpret_cast<const uint4*>(deg)[i];
+        const uint32_t v = (uint32_t)i * 4u;
+        uint4 p = make_uint4(0u, 0u, 0u, 0u);
+        if (e.x | e.y | e.z | e.w) p = make_uint4(one(v, e.x), one(v + 1u, e.y), one(v + 2u, e.z), one(v + 3u, e.w));
+        reinterpret_cast<uint4*>(np)[i] = p;
+    }
+    for (uint64_t v = n / 4u * 4u + t0; v < n; v += step) np[v] = one((uint32_t)v, deg[v]);
+    if (t0 == 0) np[n] = 0;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_down_sync(0xffffffffu, mine, off);
+        mine = o > mine ? o : mine;
+    }
+    if ((threadIdx.x & 31u) == 0u && mine) atomicMax(best, mine);
+}
+// Placement from edges sorted by vertex (payloads as in k_place).
+__global__ void k_place_runs(const uint32_t* __restrict__ key, const uint32_t* __restrict__ nb, const uint32_t* __restrict__ pay,
+                             uint64_t m, uint32_t K, const uint32_t* __restrict__ first, const uint32_t* __restrict__ vstart,
+                             uint32_t* __restrict__ vcol, uint32_t* __restrict__ vw, const uint32_t* __restrict__ w_in,
+                             uint32_t* __restrict__ veid, uint64_t m_in) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t v = key[i];
+        const size_t slot = (size_t)vstart[v] * K + (uint32_t)((uint32_t)i - first[v]);
+        vcol[slot] = nb[i];
+        if (veid) {
+            const uint32_t e = pay[i];
+            veid[slot] = e;
+            if (vw) vw[slot] = w_in ? w_in[(m_in && e >= m_in) ? e - m_in : e] : 1u;
+        } else if (vw) {
+            vw[slot] = pay[i];
+        }
+    }
+}
+
 // Owner of every part, and the unused slots of each vertex's last part (targets and edge indices NO_EDGE,
 // weights 0). A vertex of more than 32 parts is written by its whole warp. The unused slots end a row aligned
 // to its size, so they are written in at most one store each of 4, 8 and 16 bytes (and one more 16 for K =
@@ -788,6 +849,15 @@ eeg_status build_out_degrees(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, con
     return EEG_OK;
 }
 
+// Sparse graphs are sorted down to the vertex instead of into buckets: a bucket costs its tile (64 KB of counters
+// cleared twice, 8 KB of counts written and read), however few edges it has. Device arrays, forward and weighted, ms:
+// 2^26 vertices with 1 M edges 4.19 -> 1.02, with 8 M 5.1 -> 1.8, with 64 M 7.8 -> 5.7 (128 M: 9.8, 9.2 this way); 2^24
+// with 8 M 1.62 -> 1.00, with 32 M 2.50 (2.39 this way, symmetrised 3.15 and 3.21); 2^22 with 2 M 0.43 -> 0.35, with
+// 4 M 0.51 (0.51); 2^20 with 0.5 M 0.21 (0.21). Up to 2^22 vertices the buckets take one pass, this two.
+static bool sorted_by_vertex(uint32_t n, uint64_t m) {
+    return m > 0 && n > (1u << 20) && (n > (1u << 22) ? 2 * m < 3ull * n : 4 * m < 3ull * n);
+}
+
 // Build one direction. reverse: edges (s,t) are inserted as (t,s) -- the transposed graph. Each vertex's
 // edges keep the input order (the order the reference's MakeGraph gives them) and the layout is
 // deterministic. With EEG_VG_SYMMETRIZE the vg->m arcs are the vg->m / 2 input edges followed by their
@@ -802,7 +872,9 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
     const bool eid = (vg->flags & EEG_VG_EDGE_IDS) != 0;
     const bool payload = with_w || eid;  // a third word per edge: weight, or edge index
     const uint32_t bits = n > 1 ? 32u - (uint32_t)__builtin_clz(n - 1) : 1u;
-    const uint32_t high = bits > (uint32_t)S_BITS ? bits - (uint32_t)S_BITS : 0u;  // bucket bits
+    const bool by_vertex = sorted_by_vertex(n, m);
+    const uint32_t low = by_vertex ? 0u : (uint32_t)S_BITS;
+    const uint32_t high = bits > low ? bits - low : 0u;  // bits to partition by
     const uint32_t passes = std::max<uint32_t>(1u, (high + S_BITS - 1) / S_BITS);
     const uint32_t nb_buckets = n ? ((n - 1) >> S_BITS) + 1u : 1u;
     // the first pass's tiles have one direction each (later passes have no more of them)
@@ -810,6 +882,7 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
     const uint64_t ntiles2 = (m + S_TILE - 1) / S_TILE;
     const uint64_t nchunks = (ntiles + S_CHUNK - 1) / S_CHUNK;
     const uint64_t vtiles = m / S_TILE + std::min<uint64_t>(nb_buckets, m);  // most tiles the buckets can have
+    const bool low_keys = passes == 1 && !by_vertex;  // the partition keeps the low bits only
 
     EEG_TRY(vg_alloc(vg, (void**)&d->deg, sizeof(uint32_t) * (size_t)(n + 1)));
     EEG_TRY(vg_alloc(vg, (void**)&d->vstart, sizeof(uint32_t) * (size_t)(n + 1)));
@@ -824,7 +897,7 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
     // ---- partition by bucket
     void* key = nullptr;                       // uint16_t low bits (one pass) or the uint32_t owners
     uint32_t *nb = nullptr, *pay = nullptr;    // partitioned
-    uint32_t *bstart = nullptr, *tstart = nullptr, *tbucket = nullptr, *vcnt = nullptr;
+    uint32_t *bstart = nullptr, *tstart = nullptr, *tbucket = nullptr, *vcnt = nullptr, *first = nullptr;
     if (m > 0) {
         Arcs s{};
         s.a = reverse ? d_dst : d_src;
@@ -846,7 +919,7 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
         if (host_in) EEG_TRY(T.get((void**)&copy, sizeof(uint32_t) * m));
         uint32_t* in_key = nullptr;  // null: the arcs
         uint32_t *in_nb = nullptr, *in_pay = nullptr;
-        uint32_t lo = (uint32_t)S_BITS;
+        uint32_t lo = low;
         for (uint32_t p = 0; p < passes; ++p) {
             const bool last = p + 1 == passes;
             // bits of this pass (at least 2: the tile kernels take four bins per thread)
@@ -854,7 +927,7 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
             const uint32_t bins = 1u << pbits;
             void* out_key = nullptr;
             uint32_t *out_nb = nullptr, *out_pay = nullptr;
-            EEG_TRY(T.get(&out_key, (passes == 1 ? sizeof(uint16_t) : sizeof(uint32_t)) * m));
+            EEG_TRY(T.get(&out_key, (low_keys ? sizeof(uint16_t) : sizeof(uint32_t)) * m));
             EEG_TRY(T.get((void**)&out_nb, sizeof(uint32_t) * m));
             if (payload) EEG_TRY(T.get((void**)&out_pay, sizeof(uint32_t) * m));
             const uint64_t nt = p == 0 ? ntiles : ntiles2, nc = (nt + S_CHUNK - 1) / S_CHUNK;
@@ -873,11 +946,11 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
                                                             out_nb, out_pay);
                 return EEG_OK;
             };
-            if (passes == 1) EEG_TRY(go(k_partition<true, uint16_t>, (uint16_t*)out_key));
+            if (low_keys) EEG_TRY(go(k_partition<true, uint16_t>, (uint16_t*)out_key));
             else if (p == 0) EEG_TRY(go(k_partition<true, uint32_t>, (uint32_t*)out_key));
             else EEG_TRY(go(k_partition<false, uint32_t>, (uint32_t*)out_key));
             EEG_CUDA(cudaGetLastError());
-            in_key = passes == 1 ? nullptr : (uint32_t*)out_key;
+            in_key = low_keys ? nullptr : (uint32_t*)out_key;
             in_nb = out_nb;
             in_pay = out_pay;
             key = out_key;
@@ -885,28 +958,37 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
         }
         nb = in_nb;
         pay = in_pay;
-        // ---- tiles of the buckets, counts per vertex
-        EEG_TRY(T.get((void**)&tstart, sizeof(uint32_t) * ((size_t)nb_buckets + 1)));
-        EEG_TRY(T.get((void**)&tbucket, sizeof(uint32_t) * vtiles));
-        EEG_TRY(T.get((void**)&vcnt, sizeof(uint32_t) * vtiles * S_BINS));
-        if (passes == 1) {
-            bstart = start;  // bins at least the buckets; their starts run on to m
+        if (by_vertex) {
+            EEG_TRY(T.get((void**)&first, sizeof(uint32_t) * (size_t)n));
+            EEG_CUDA(cudaMemsetAsync(d->deg, 0, sizeof(uint32_t) * (size_t)n, st));
+            k_runs<<<grid_for(m, vg->device), B_TPB, 0, st>>>((const uint32_t*)key, m, first, d->deg);
         } else {
-            EEG_TRY(T.get((void**)&bstart, sizeof(uint32_t) * ((size_t)nb_buckets + 1)));
-            k_bucket_starts<<<grid_for(m + 1, vg->device), B_TPB, 0, st>>>((const uint32_t*)key, m, nb_buckets, bstart);
+            // ---- tiles of the buckets, counts per vertex
+            EEG_TRY(T.get((void**)&tstart, sizeof(uint32_t) * ((size_t)nb_buckets + 1)));
+            EEG_TRY(T.get((void**)&tbucket, sizeof(uint32_t) * vtiles));
+            EEG_TRY(T.get((void**)&vcnt, sizeof(uint32_t) * vtiles * S_BINS));
+            if (low_keys) {
+                bstart = start;  // bins at least the buckets; their starts run on to m
+            } else {
+                EEG_TRY(T.get((void**)&bstart, sizeof(uint32_t) * ((size_t)nb_buckets + 1)));
+                k_bucket_starts<<<grid_for(m + 1, vg->device), B_TPB, 0, st>>>((const uint32_t*)key, m, nb_buckets, bstart);
+            }
+            k_bucket_tiles<<<1, SCAN_TPB, 0, st>>>(bstart, nb_buckets, tstart, tbucket);
+            if (low_keys)
+                k_vertex_counts<uint16_t><<<(unsigned)vtiles, S_TPB, 0, st>>>((const uint16_t*)key, bstart, tstart, tbucket,
+                                                                              nb_buckets, vcnt);
+            else
+                k_vertex_counts<uint32_t><<<(unsigned)vtiles, S_TPB, 0, st>>>((const uint32_t*)key, bstart, tstart, tbucket,
+                                                                              nb_buckets, vcnt);
         }
-        k_bucket_tiles<<<1, SCAN_TPB, 0, st>>>(bstart, nb_buckets, tstart, tbucket);
-        if (passes == 1)
-            k_vertex_counts<uint16_t><<<(unsigned)vtiles, S_TPB, 0, st>>>((const uint16_t*)key, bstart, tstart, tbucket,
-                                                                          nb_buckets, vcnt);
-        else
-            k_vertex_counts<uint32_t><<<(unsigned)vtiles, S_TPB, 0, st>>>((const uint32_t*)key, bstart, tstart, tbucket,
-                                                                          nb_buckets, vcnt);
-    } else {  // no edges: no tile in any bucket
+    } else if (!by_vertex) {  // no edges: no tile in any bucket
         EEG_TRY(T.get((void**)&tstart, sizeof(uint32_t) * ((size_t)nb_buckets + 1)));
         EEG_CUDA(cudaMemsetAsync(tstart, 0, sizeof(uint32_t) * ((size_t)nb_buckets + 1), st));
     }
-    k_degrees<<<dim3(grid_for((uint64_t)n, vg->device), 8), 256, 0, st>>>(vcnt, tstart, n, K, d->deg, np, best);
+    if (by_vertex)
+        k_run_degrees<<<grid_for((uint64_t)n, vg->device), 256, 0, st>>>(first, n, K, d->deg, np, best);
+    else
+        k_degrees<<<dim3(grid_for((uint64_t)n, vg->device), 8), 256, 0, st>>>(vcnt, tstart, n, K, d->deg, np, best);
     EEG_TRY(device_scan_u32(np, d->vstart, (uint64_t)n + 1, false, SCAN_ADD, tmp, st));
 
     uint32_t hbuf[4] = {0, 0, 0, 0};
@@ -933,16 +1015,21 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
 
     if (P > 0) {
         k_owners<<<grid_for(n, vg->device), B_TPB, 0, st>>>(n, K, d->vstart, d->deg, d->vowner, d->vcol, d->vw, d->veid);
-        const size_t psm = place_smem(payload);
-        auto go = [&](auto kern, auto* k) -> eeg_status {
-            EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PLACE_SMEM));
-            kern<<<(unsigned)vtiles, S_TPB, psm, st>>>(k, nb, pay, bstart, tstart, tbucket, nb_buckets, n, K, vcnt,
-                                                             d->vstart, d->vcol, d->vw, with_w ? d_w : nullptr, d->veid,
-                                                             sym ? m_in : 0);
-            return EEG_OK;
-        };
-        if (passes == 1) EEG_TRY(go(k_place<uint16_t>, (const uint16_t*)key));
-        else EEG_TRY(go(k_place<uint32_t>, (const uint32_t*)key));
+        if (by_vertex) {
+            k_place_runs<<<grid_for(m, vg->device), B_TPB, 0, st>>>((const uint32_t*)key, nb, pay, m, K, first, d->vstart, d->vcol,
+                                                                    d->vw, with_w ? d_w : nullptr, d->veid, sym ? m_in : 0);
+        } else {
+            const size_t psm = place_smem(payload);
+            auto go = [&](auto kern, auto* k) -> eeg_status {
+                EEG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PLACE_SMEM));
+                kern<<<(unsigned)vtiles, S_TPB, psm, st>>>(k, nb, pay, bstart, tstart, tbucket, nb_buckets, n, K, vcnt,
+                                                                 d->vstart, d->vcol, d->vw, with_w ? d_w : nullptr, d->veid,
+                                                                 sym ? m_in : 0);
+                return EEG_OK;
+            };
+            if (low_keys) EEG_TRY(go(k_place<uint16_t>, (const uint16_t*)key));
+            else EEG_TRY(go(k_place<uint32_t>, (const uint32_t*)key));
+        }
     }
     EEG_CUDA(cudaGetLastError());
     vg->bytes += sizeof(uint32_t) * ((size_t)(n + 1) * 2 + (size_t)P + slots * (1 + (with_w ? 1 : 0) + (eid ? 1 : 0)));
