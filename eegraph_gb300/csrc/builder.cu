@@ -310,8 +310,21 @@ __global__ void __launch_bounds__(SCAN_TPB) k_bucket_tiles(const uint32_t* __res
                                                            uint32_t* tstart, uint32_t* tbucket) {
     scan_to([&](uint32_t i) { return (bstart[i + 1] - bstart[i] + (uint32_t)S_TILE - 1u) / (uint32_t)S_TILE; }, nb, tstart);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < nb; i += SCAN_TPB)
-        for (uint32_t t = tstart[i]; t < tstart[i + 1]; ++t) tbucket[t] = i;
+    // a bucket of many tiles (2048 of them: 70 us by one thread) is written by the whole CTA
+    __shared__ uint32_t s_many[SCAN_TPB], s_count;
+    for (uint32_t base = 0; base < nb; base += SCAN_TPB) {
+        if (threadIdx.x == 0) s_count = 0u;
+        __syncthreads();
+        const uint32_t i = base + threadIdx.x;
+        const uint32_t t0 = i < nb ? tstart[i] : 0u, t1 = i < nb ? tstart[i + 1] : 0u;
+        if (t1 - t0 > 16u) s_many[atomicAdd(&s_count, 1u)] = i;
+        else
+            for (uint32_t t = t0; t < t1; ++t) tbucket[t] = i;
+        __syncthreads();
+        for (uint32_t k = 0; k < s_count; ++k)
+            for (uint32_t t = tstart[s_many[k]] + threadIdx.x; t < tstart[s_many[k] + 1]; t += SCAN_TPB) tbucket[t] = s_many[k];
+        __syncthreads();
+    }
 }
 // Bucket starts from keys sorted by bucket (more than one partition pass): entry i closes every bucket up to its own
 __global__ void k_bucket_starts(const uint32_t* __restrict__ key, uint64_t m, uint32_t nb, uint32_t* __restrict__ bstart) {
@@ -634,7 +647,9 @@ __global__ void k_place_runs(const uint32_t* __restrict__ key, const uint32_t* _
 }
 
 // Owner of every part, and the unused slots of each vertex's last part (targets and edge indices NO_EDGE,
-// weights 0). A vertex of more than 32 parts is written by its whole warp. The unused slots end a row aligned
+// weights 0). The owners of a vertex of more than 32 parts are written by its whole warp, those of one of more than
+// HUB_PARTS (on hubs: their number, then their ids) by k_hub_owners' whole grid: a vertex of 2 M parts took its warp
+// 340 us. The unused slots end a row aligned
 // to its size, so they are written in at most one store each of 4, 8 and 16 bytes (and one more 16 for K =
 // 16): a store of 32 lanes here touches 32 sectors whatever its width, 0.16 ms on R-MAT s22 word by word.
 __device__ __forceinline__ void pad_row(uint32_t* p, size_t i, size_t end, uint32_t x) {
@@ -645,9 +660,10 @@ __device__ __forceinline__ void pad_row(uint32_t* p, size_t i, size_t end, uint3
     }
     for (; i < end; i += 4) *reinterpret_cast<uint4*>(p + i) = make_uint4(x, x, x, x);
 }
+constexpr uint32_t HUB_PARTS = 4096;
 __global__ void k_owners(uint32_t n, uint32_t K, const uint32_t* __restrict__ vstart, const uint32_t* __restrict__ deg,
                          uint32_t* __restrict__ vowner, uint32_t* __restrict__ vcol, uint32_t* __restrict__ vw,
-                         uint32_t* __restrict__ veid) {
+                         uint32_t* __restrict__ veid, uint32_t* __restrict__ hubs) {
     const uint32_t lane = threadIdx.x & 31u;
     for (uint64_t v0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; v0 < n;
          v0 += (uint64_t)gridDim.x * blockDim.x) {
@@ -664,15 +680,24 @@ __global__ void k_owners(uint32_t n, uint32_t K, const uint32_t* __restrict__ vs
                 if (veid) pad_row(veid, used, end, NO_EDGE);
                 if (np <= 32u)
                     for (uint32_t j = 0; j < np; ++j) vowner[s0 + j] = (uint32_t)v;
+                else if (np > HUB_PARTS) hubs[1u + atomicAdd(&hubs[0], 1u)] = (uint32_t)v;
             }
         }
-        uint32_t big = __ballot_sync(0xffffffffu, np > 32u);
+        uint32_t big = __ballot_sync(0xffffffffu, np > 32u && np <= HUB_PARTS);
         while (big) {
             const int l = __ffs(big) - 1;
             big &= big - 1u;
             const uint32_t bs = __shfl_sync(0xffffffffu, s0, l), bn = __shfl_sync(0xffffffffu, np, l);
             for (uint32_t j = lane; j < bn; j += 32u) vowner[bs + j] = (uint32_t)v0 + (uint32_t)l;
         }
+    }
+}
+
+__global__ void k_hub_owners(const uint32_t* __restrict__ hubs, const uint32_t* __restrict__ vstart, uint32_t* __restrict__ vowner) {
+    for (uint32_t h = 0; h < hubs[0]; ++h) {
+        const uint32_t v = hubs[1u + h], end = vstart[v + 1];
+        for (uint64_t p = (uint64_t)vstart[v] + blockIdx.x * blockDim.x + threadIdx.x; p < end; p += gridDim.x * blockDim.x)
+            vowner[p] = v;
     }
 }
 
@@ -1000,8 +1025,8 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
         set_last_error("edge endpoint outside [0, num_nodes)");
         return EEG_ERR_INVALID;
     }
+    const unsigned long long kbest = ((unsigned long long)hbuf[3] << 32) | hbuf[2];
     if (!reverse) {
-        unsigned long long kbest = ((unsigned long long)hbuf[3] << 32) | hbuf[2];
         vg->max_deg = (uint32_t)(kbest >> 32);
         vg->max_deg_vertex = kbest ? 0xFFFFFFFFu - (uint32_t)(kbest & 0xFFFFFFFFu) : 0u;
     }
@@ -1014,7 +1039,13 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
     if (eid) EEG_TRY(vg_alloc(vg, (void**)&d->veid, sizeof(uint32_t) * std::max<size_t>(slots, 4)));
 
     if (P > 0) {
-        k_owners<<<grid_for(n, vg->device), B_TPB, 0, st>>>(n, K, d->vstart, d->deg, d->vowner, d->vcol, d->vw, d->veid);
+        uint32_t* hubs = nullptr;
+        if ((kbest >> 32) > (uint64_t)HUB_PARTS * K) {  // each of them has more edges than that
+            EEG_TRY(T.get((void**)&hubs, sizeof(uint32_t) * (m / ((uint64_t)HUB_PARTS * K) + 2)));
+            EEG_CUDA(cudaMemsetAsync(hubs, 0, sizeof(uint32_t), st));
+        }
+        k_owners<<<grid_for(n, vg->device), B_TPB, 0, st>>>(n, K, d->vstart, d->deg, d->vowner, d->vcol, d->vw, d->veid, hubs);
+        if (hubs) k_hub_owners<<<(unsigned)sm_count(vg->device) * 2, B_TPB, 0, st>>>(hubs, d->vstart, d->vowner);
         if (by_vertex) {
             k_place_runs<<<grid_for(m, vg->device), B_TPB, 0, st>>>((const uint32_t*)key, nb, pay, m, K, first, d->vstart, d->vcol,
                                                                     d->vw, with_w ? d_w : nullptr, d->veid, sym ? m_in : 0);
