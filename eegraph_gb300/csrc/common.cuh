@@ -303,7 +303,7 @@ template <bool TAIL, class Before>
 __device__ __forceinline__ bool vertex_off(float most, float d, float f, float x, Before fo) {
     f = fabsf(f);
     most *= fabsf(x);
-    if (f * (TAIL ? d * d * d : d) <= most * (1.f - d)) return false;
+    if (!(f * (TAIL ? d * d * d : d) > most * (1.f - d))) return false;
     const float before = fabsf(fo());
     if (!(f < d * before)) return true;
     const float rho = f / before;

@@ -7,12 +7,13 @@
 // over-counts vertices with more than K out-edges; here each vertex is updated exactly once per sweep.
 //
 // GB300 form: Jacobi sweeps that PULL over the transposed virtual graph (parts of <= K in-edges).
-//  * A warp owns chunks of 32 consecutive parts and keeps two chunks in flight: their part rows
+//  * A warp owns chunks of 32 consecutive parts and keeps one or two chunks in flight: their part rows
 //    (256-bit loads) and then all 2*K gathers of contrib[u] = x_u / outdeg(u) are issued before any
 //    of them is consumed; the old value and out-degree of each chunk's segment ends are prefetched
 //    alongside the gathers.
 //  * Each lane sums its part's K values by a pairwise tree; parts of one vertex are combined by a
 //    segmented warp scan of compensated (hi, lo) pairs.
+//  * What the sweeps start from, and the values at the end, are written by kernels of their own.
 //  * A vertex whose parts all sit in one chunk is finalised in place. A vertex whose parts span chunks
 //    gets one FP64 atomic partial per chunk plus an arrival count; the warp that brings the count to
 //    the number of chunks spanned finalises it. So a sweep needs ONE grid barrier.
@@ -42,10 +43,11 @@ namespace {
 
 constexpr int PR_TPB = 1024;  // one CTA per SM: its shared memory holds the hot contributions
 constexpr uint32_t PR_HOT_DEFAULT = 32768;
-// chunks in flight per warp (K = 16 keeps one: its 16 ids + 16 gathered values already fill the registers)
-template <int K>
+// chunks in flight per warp (K = 16 keeps one: its 16 ids + 16 gathered values already fill the registers; so does
+// K = 8 in residual form, where two spill 72 bytes: 260 us a sweep on R-MAT s22, one 224)
+template <int K, bool RES>
 struct InFlight {
-    static constexpr int U = K >= 16 ? 1 : 2;
+    static constexpr int U = K >= (RES ? 8 : 16) ? 1 : 2;
 };
 
 struct PRArgs {
@@ -140,83 +142,132 @@ __device__ __forceinline__ void settle_spanning(const PRArgs& a, const uint2* xb
 
 // Looks at every vertex once the L1 test is met (see VertexBound): 0 = some vertex is off, and the control's next
 // step is set for it; 1 = none is; 2 = the grid is aborting. One grid barrier. A pass of its own, 50 us on R-MAT s22
-// (1.6 % of the run; the test in the sweeps themselves cost 3.4 %), and not inlined: that spilled in the gather loop
-// (K = 8: a sweep 246 -> 282 us; so, and without counting the gathered edges there, 249, K = 16 197 -> 195).
-static __device__ __noinline__ int look(uint32_t n, const uint2* __restrict__ info, const float* cnext, const float* ccur,
-                                        const float2* y, VertexBound bound, PRCtrl* ctrl, uint32_t slot, uint32_t epoch,
-                                        uint64_t timeout_ns, Extrapolation* ex, double d) {
-    const float most = ex->looks ? bound.later : bound.first;
+// (1.6 % of the run; the test in the sweeps themselves cost 3.4 %), and not inlined: that spilled in the gather loop.
+static __device__ __noinline__ int look(const PRArgs& a, uint32_t s, uint32_t epoch, Extrapolation* ex) {
+    const float *cnext = (s & 1u) ? a.c0 : a.c1, *ccur = (s & 1u) ? a.c1 : a.c0;
+    PRCtrl* ctrl = a.ctrl;
+    const float most = ex->looks ? a.bound.later : a.bound.first;
     uint32_t far = 0;
-    for (uint32_t v = blockIdx.x * PR_TPB + threadIdx.x; v < n; v += gridDim.x * PR_TPB) {
-        const uint2 inf = __ldg(&info[v]);
+    for (uint32_t v = blockIdx.x * PR_TPB + threadIdx.x; v < a.n; v += gridDim.x * PR_TPB) {
+        const uint2 inf = __ldg(&a.info[v]);
         const float w = inf.y ? (float)inf.y : 1.f;
-        far |= vertex_off<false>(most, bound.d, cnext[inf.x] * w, __ldcg(&y[v]).x, [&]() { return ccur[inf.x] * w; }) ? 1u : 0u;
+        far |= vertex_off<false>(most, a.bound.d, cnext[inf.x] * w, __ldcg(&a.y[v]).x, [&]() { return ccur[inf.x] * w; }) ? 1u : 0u;
     }
     far = __syncthreads_or(far);
-    if (threadIdx.x == 0 && far) atomicOr(&ctrl->far[slot], 1u);
-    if (!grid_barrier_sync(&ctrl->bw, epoch, timeout_ns)) return 2;
+    if (threadIdx.x == 0 && far) atomicOr(&ctrl->far[s % 3u], 1u);
+    if (!grid_barrier_sync(&ctrl->bw, epoch, a.timeout_ns)) return 2;
     __shared__ uint32_t s_far;
     if (threadIdx.x == 0) {
-        s_far = *(volatile uint32_t*)&ctrl->far[slot];
-        if (s_far) vertices_off(*ex, d);
+        s_far = *(volatile uint32_t*)&ctrl->far[s % 3u];
+        if (s_far) vertices_off(*ex, a.damping64);
     }
     __syncthreads();
     return s_far ? 0 : 1;
 }
 
+// The passes over the vertices before and after the sweeps are kernels of their own, with four vertices per thread at
+// a time, their loads first: in the sweeps' kernel (one CTA per SM, a chain of two loads per vertex) they took most of
+// a run on a graph of many vertices and few edges (2^26 and 1 M, 2 sweeps: 1.59 ms, 1.17 so).
+constexpr int PASS_TPB = 256;
+struct Vertices4 {
+    uint2 info[4];
+    bool in[4], none[4];  // a vertex; without in-edges: its value stays the base
+};
+__device__ __forceinline__ Vertices4 fetch_vertices(const PRArgs& a, uint64_t v0, uint64_t step) {
+    Vertices4 r;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const uint64_t v = v0 + (uint64_t)u * step;
+        r.in[u] = v < a.n;
+        r.none[u] = false;
+        r.info[u] = make_uint2(0u, 0u);
+        if (r.in[u]) {
+            r.info[u] = __ldg(&a.info[v]);
+            r.none[u] = __ldg(&a.rvstart[v + 1]) == __ldg(&a.rvstart[v]);
+        }
+    }
+    return r;
+}
+// x0 = 1-d, its contributions, partial slots; counts the vertices without in-edges.
+template <bool RES>
+__global__ void __launch_bounds__(PASS_TPB) k_set_up(const PRArgs a) {
+    const uint64_t t0 = (uint64_t)blockIdx.x * PASS_TPB + threadIdx.x, step = (uint64_t)gridDim.x * PASS_TPB;
+    uint32_t zero_in = 0;
+    for (uint64_t v0 = t0; v0 < a.n; v0 += 4ull * step) {
+        const Vertices4 r = fetch_vertices(a, v0, step);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (!r.in[u]) break;
+            const uint64_t v = v0 + (uint64_t)u * step;
+            const uint32_t rk = r.info[u].x, od = r.info[u].y;
+            if (RES) {  // the first sweep gathers the base's contributions from x; its residual is d P base
+                const float b = (float)a.base64;
+                a.x[rk] = od ? b / (float)od : 0.f;
+                if (r.none[u]) a.c0[rk] = a.c1[rk] = 0.f;  // no sweep writes them
+                else a.y[v] = make_float2(b, (float)(a.base64 - (double)b));
+            } else {
+                const float c = od ? a.base / (float)od : 0.f;
+                a.x[v] = a.base;
+                a.c0[rk] = c;
+                a.c1[rk] = c;
+            }
+            a.acc[v] = 0.0;
+            a.arrive[v] = 0u;
+            zero_in += r.none[u] ? 1u : 0u;
+        }
+    }
+    const uint32_t warp = __reduce_add_sync(0xffffffffu, zero_in);
+    __shared__ uint32_t s_zero;
+    if (threadIdx.x == 0) s_zero = 0u;
+    __syncthreads();
+    if ((threadIdx.x & 31u) == 0u && warp) atomicAdd(&s_zero, warp);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_zero) atomicAdd(&a.ctrl->zero_in, (unsigned long long)s_zero);
+}
+// Residual form: the result.
+__global__ void __launch_bounds__(PASS_TPB) k_values(const PRArgs a) {
+    const uint64_t t0 = (uint64_t)blockIdx.x * PASS_TPB + threadIdx.x, step = (uint64_t)gridDim.x * PASS_TPB;
+    const float b = (float)a.base64;
+    for (uint64_t v0 = t0; v0 < a.n; v0 += 4ull * step) {
+        float2 y[4];
+        bool none[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t v = v0 + (uint64_t)u * step;
+            none[u] = true;
+            if (v < a.n) {
+                none[u] = __ldg(&a.rvstart[v + 1]) == __ldg(&a.rvstart[v]);
+                y[u] = a.y[v];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t v = v0 + (uint64_t)u * step;
+            if (v < a.n) a.x[v] = none[u] ? b : __fadd_rn(y[u].x, y[u].y);
+        }
+    }
+}
+
 template <int K, bool RES>
-__global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
-    constexpr int PR_U = InFlight<K>::U;
+__global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(const __grid_constant__ PRArgs a) {
+    constexpr int PR_U = InFlight<K, RES>::U;
     extern __shared__ float4 s_hot4[];  // contributions of the `hot` highest out-degree vertices
     const float* s_hot = reinterpret_cast<const float*>(s_hot4);
     __shared__ double s_red[RES ? 3 : 2][PR_TPB / 32];
-    __shared__ unsigned long long s_zero;
     __shared__ uint2 s_span[PR_TPB / 32][XCAP];
     __shared__ uint32_t s_next;  // next of this CTA's chunks to hand out in the current sweep
     __shared__ double s_rn[2];   // the last sweep's residual and norm
     __shared__ Extrapolation s_ex;  // residual form: step lengths (thread 0; the same in every CTA)
     uint2* xbuf = s_span[threadIdx.x >> 5];
     PRCtrl* ctrl = a.ctrl;
-    const uint32_t gtid = blockIdx.x * PR_TPB + threadIdx.x;
-    const uint32_t gthreads = gridDim.x * PR_TPB;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t nchunks = (a.RP + 31u) / 32u;
     const uint64_t pol = l2_evict_first_policy();
     uint32_t epoch = 0;
 
-    // ---- set-up: x0 = 1-d, contrib0, partial slots; count vertices without in-edges
-    if (threadIdx.x == 0) {
-        s_zero = 0;
-        extrapolation_init(s_ex);
-    }
+    if (threadIdx.x == 0) extrapolation_init(s_ex);
     __syncthreads();
-    unsigned long long zero_in = 0;
-    for (uint32_t v = gtid; v < a.n; v += gthreads) {
-        const uint2 inf = a.info[v];
-        const uint32_t od = inf.y;
-        const uint32_t rk = inf.x;
-        if (RES) {  // y0 = base; the first sweep's residual is d P base, zero where there is no in-edge
-            const float b = (float)a.base64;
-            a.y[v] = make_float2(b, (float)(a.base64 - (double)b));
-            a.c0[rk] = od ? b / (float)od : 0.f;
-            a.c1[rk] = 0.f;
-        } else {
-            const float c = od ? a.base / (float)od : 0.f;
-            a.x[v] = a.base;
-            a.c0[rk] = c;
-            a.c1[rk] = c;
-        }
-        a.acc[v] = 0.0;
-        a.arrive[v] = 0u;
-        zero_in += (a.rvstart[v + 1] == a.rvstart[v]) ? 1ull : 0ull;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) zero_in += __shfl_down_sync(0xffffffffu, zero_in, off);
-    if (lane == 0 && zero_in) atomicAdd(&s_zero, zero_in);
-    __syncthreads();
-    if (threadIdx.x == 0 && s_zero) atomicAdd(&ctrl->zero_in, s_zero);
     uint32_t s = 0;
-    if (!grid_barrier_sync(&ctrl->bw, epoch, a.timeout_ns)) goto finish;
     {
         const double zero_norm = (double)*(volatile unsigned long long*)&ctrl->zero_in * (double)a.base;
         for (;; ++s) {
@@ -237,12 +288,9 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
             // ccur is read through L1 (plain loads): the grid barrier's acquire makes the previous sweep's
             // values visible, and within a sweep they do not change (SYNC) or may be stale (ASYNC, allowed)
             const bool inplace = !RES && a.inplace;
-            const float* ccur = (s & 1u) && !inplace ? a.c1 : a.c0;
+            const float* ccur = RES && s == 0u ? a.x : ((s & 1u) && !inplace ? a.c1 : a.c0);
             float* cnext = inplace ? a.c0 : ((s & 1u) ? a.c0 : a.c1);
             const float2 step = RES ? make_float2(s_ex.alpha, s_ex.cand) : make_float2(1.f, 0.f);
-            if (RES && s == 1u)  // c0 still holds the base's contributions where no sweep writes
-                for (uint32_t v = gtid; v < a.n; v += gthreads)
-                    if (a.rvstart[v + 1] == a.rvstart[v]) a.c0[a.info[v].x] = 0.f;
             double r = 0.0, nrm = 0.0, q = 0.0;
             uint32_t nx = 0;  // warp-uniform fill of xbuf
             auto fin = [&](uint32_t vv, double sum) {
@@ -273,6 +321,11 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
                 uint32_t i0 = 0;
                 if (lane == 0) i0 = atomicAdd(&s_next, (uint32_t)PR_U);
                 i0 = __shfl_sync(0xffffffffu, i0, 0);
+                // a chunk adds at most two vertices to the list: the first and the last
+                if (nx && (i0 >= my_chunks || nx + 2u * PR_U > (uint32_t)XCAP)) {
+                    settle_spanning(a, xbuf, nx, lane, fin);
+                    nx = 0;
+                }
                 if (i0 >= my_chunks) break;
                 uint32_t v[PR_U], col[PR_U][K], vb[PR_U];
                 bool valid[PR_U];
@@ -356,17 +409,11 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
                     }
                     const uint32_t m = __ballot_sync(0xffffffffu, spans);
                     if (m) {
-                        const uint32_t c = __popc(m);
-                        if (nx + c > (uint32_t)XCAP) {
-                            settle_spanning(a, xbuf, nx, lane, fin);
-                            nx = 0;
-                        }
                         if (spans) xbuf[nx + __popc(m & ((1u << lane) - 1u))] = make_uint2(v[u], need);
-                        nx += c;
+                        nx += __popc(m);
                     }
                 }
             }
-            if (nx) settle_spanning(a, xbuf, nx, lane, fin);
             // CTA reduction of the FP64 residual / norm, one atomic per CTA
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) {
@@ -413,8 +460,7 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
                 }
                 if (step.x != 1.f || !(a.damping64 / (1.0 - a.damping64) * resid <= tol * norm)) continue;
                 if (s_ex.steps && s + 1u < a.bound.sweeps) {
-                    const int seen = look(a.n, a.info, cnext, ccur, a.y, a.bound, ctrl, slot, epoch++, a.timeout_ns, &s_ex,
-                                          a.damping64);
+                    const int seen = look(a, s, epoch++, &s_ex);
                     if (seen == 0) continue;
                     if (seen == 2) break;
                 }
@@ -431,12 +477,6 @@ __global__ void __launch_bounds__(PR_TPB, 1) k_pagerank(PRArgs a) {
             }
         }
     }
-finish:
-    if (RES)  // the result; every CTA's values are settled (the last sweep's barrier, or an abort)
-        for (uint32_t v = gtid; v < a.n; v += gthreads) {
-            const float2 y = __ldcg(&a.y[v]);
-            a.x[v] = __fadd_rn(y.x, y.y);
-        }
     if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->iterations = s;
 }
 
@@ -469,8 +509,13 @@ eeg_status launch_pr(const PRArgs& args, bool res, int device, uint32_t bps, uin
     const uint64_t work = std::max<uint64_t>(args.RP, args.n);
     const uint64_t need = (work + PR_TPB - 1) / PR_TPB;
     if (need < blocks) blocks = std::max<uint64_t>(need, 1);
+    const unsigned passes = (unsigned)std::min<uint64_t>((args.n + 4ull * PASS_TPB - 1) / (4ull * PASS_TPB), (uint64_t)sm_count(device) * 8);
+    if (res) k_set_up<true><<<passes, PASS_TPB, 0, st>>>(a);
+    else k_set_up<false><<<passes, PASS_TPB, 0, st>>>(a);
     void* params[] = {(void*)&a};
     EEG_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)blocks), dim3(PR_TPB), params, dyn, st));
+    if (res) k_values<<<passes, PASS_TPB, 0, st>>>(a);
+    EEG_CUDA(cudaGetLastError());
     return EEG_OK;
 }
 
@@ -660,7 +705,7 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
         res->parts_processed = (uint64_t)hc.iterations * vg->rev.P;
         res->pr_residual = hc.last_resid;
         res->pr_l1_norm = hc.last_norm;
-        res->launches = 1;
+        res->launches = res_form ? 3 : 2;
     }
     if (hc.bw.status == DEV_TIMEOUT) {
         set_last_error("grid barrier wait exceeded the timeout");
