@@ -23,7 +23,7 @@
 // would not hold the 1e-6 L1 bound); the output is FP32. Tracking which pushes lift a residual past acc
 // instead of scanning needs the atomics' old values: 25 % slower on R-MAT s22 (154.6 against 123.4 ms),
 // every returning FP64 atomic a long-scoreboard wait.
-// Long steps (ACC; runs without --accuracy and without a round cap): with the threshold derived from the
+// Long steps (ACC; runs without --accuracy and without a round cap, on graphs of at least a part per four vertices): with the threshold derived from the
 // tolerance nearly every vertex stays active for ~135 rounds of 0.84 each, and a round is a Jacobi sweep in
 // residual form. So these runs take the step lengths of the control in common.cuh (its evidence is one round
 // old when the step is taken): a round with step length alpha adds alpha t to the value, keeps (1 - alpha) t
@@ -467,7 +467,11 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
     if (!ws.dd_x) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_x, sizeof(double) * n));
     if (!ws.dd_amt) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_amt, sizeof(double) * n));
     // long steps: the threshold and the schedule are the library's own (no --accuracy, no round cap)
-    const bool accel = !(o.pr_accuracy > 0.f) && o.max_iterations == 0;
+    // and phase A is not most of the work: where few vertices have out-edges (fewer parts than n/4), nearly all of them are
+    // idle after the first round, and a queue's scan of the residuals takes a seventh of a long step's phase A (2^26
+    // vertices, 1 M edges: 3.1 ms, 11.5 with long steps; a cycle with 4 M leaves 0.33, 0.65. A tree, two vertices per
+    // part, still loses, 0.62 and 0.95 in 20 and 23 rounds; R-MAT graphs, whose mass circulates, gain from there on)
+    const bool accel = !(o.pr_accuracy > 0.f) && o.max_iterations == 0 && vg->fwd.P * 4u >= vg->n;
     if (accel && !ws.dd_taken) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_taken, sizeof(double) * n));
     if (accel && !ws.dd_share) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_share, sizeof(double) * n));
     if (!ws.dd_pq) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_pq, sizeof(uint32_t) * P));
