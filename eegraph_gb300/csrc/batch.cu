@@ -476,7 +476,9 @@ eeg_status configure(eeg_batch* b, uint32_t csize) {
 // for, and many small queries pay their rounds once per CTA. Measured against 4 for every batch: 64 graphs of
 // up to 2^18 vertices 4.0 -> 2.8 ms (8), 3 graphs of 2^18-2^20 8.6 -> 4.3 (8), 900 queries on graphs of up
 // to 2^12 0.75 -> 0.40 (1). 4 stays unless another size promises 15 % (between close ones the model is no
-// guide: 148 queries, 8 predicted 4 % faster, 0.28 -> 0.39 ms).
+// guide: 148 queries, 8 predicted 4 % faster, 0.28 -> 0.39 ms). The two constants are measured on a GB300 (152 SMs), as
+// is everything here: 14 batches of 1 to 900 queries, 2^10 to 2^20 vertices.
+//   More clusters need more working memory: one of 4 is not left for a size that needs over a sixteenth of the device's.
 uint32_t choose_cluster(const eeg_batch* b, const std::vector<BQuery>& queries) {
     const double ctas = 2.0 * sm_count(b->device);
     auto model = [&](uint32_t c) {
@@ -488,9 +490,15 @@ uint32_t choose_cluster(const eeg_batch* b, const std::vector<BQuery>& queries) 
         }
         return std::max(longest, total / ctas);
     };
+    auto scratch = [&](uint32_t c) {
+        return (double)std::min<size_t>((size_t)(ctas / c), queries.size()) * 4.0 * (2.0 * (double)b->qcap + (double)b->scap);
+    };
+    size_t free_bytes = 0, total_bytes = 0;
+    if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) (void)cudaGetLastError();
     uint32_t best = 4;
     double t = 0.85 * model(4);
     for (uint32_t c : {1u, 2u, 8u}) {
+        if (scratch(c) > std::max(scratch(4), (double)total_bytes / 16.0)) continue;
         const double tc = model(c);
         if (tc < t) {
             t = tc;
@@ -611,7 +619,13 @@ EEG_API eeg_status eeg_batch_set_queries(eeg_batch* b, const eeg_query* queries,
     b->out_words = off;
     b->max_rounds = max_n + 2u;
     if (out_words) *out_words = off;
-    return configure(b, cluster_size ? cluster_size : choose_cluster(b, hq));
+    const uint32_t size = cluster_size ? cluster_size : choose_cluster(b, hq);
+    eeg_status s = configure(b, size);
+    if (s != EEG_OK && cluster_size == 0 && size != 4) {  // the choice was ours: 4 if that fits
+        (void)cudaGetLastError();
+        s = configure(b, 4);
+    }
+    return s;
 }
 
 EEG_API eeg_status eeg_batch_query_offset(const eeg_batch* b, uint32_t query, unsigned long long* offset) {
