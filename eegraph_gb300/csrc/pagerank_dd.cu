@@ -411,6 +411,7 @@ eeg_status launch_dd(const DDArgs& a, bool acc, int device, uint32_t bps, cudaSt
 
 static uint32_t hot_stride(uint32_t nhot) { return (nhot + 15u) / 16u * 16u; }
 
+// A graph whose private targets (as many words as its own) do not fit runs without hot targets.
 static eeg_status ensure_dd_hot(eeg_vgraph* vg, cudaStream_t st) {
     Workspace& ws = vg->ws;
     if (ws.dd_hot_ready) return EEG_OK;
@@ -419,29 +420,42 @@ static eeg_status ensure_dd_hot(eeg_vgraph* vg, cudaStream_t st) {
     ws.dd_nhot = 0;
     if (slots && vg->n < HOT && vg->m > limit) {
         const size_t words = ((size_t)vg->n + 31) / 32;
-        if (!ws.dd_hot) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_hot, sizeof(uint32_t) * (HOT_CAP + 1 + words)));
         uint32_t* cnt = nullptr;
-        EEG_CUDA(cudaMallocAsync((void**)&cnt, sizeof(uint32_t) * vg->n, st));
-        EEG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * vg->n, st));
-        EEG_CUDA(cudaMemsetAsync(ws.dd_hot, 0, sizeof(uint32_t) * (HOT_CAP + 1 + words), st));
-        const uint64_t cap = (uint64_t)sm_count(vg->device) * 8;
-        const unsigned gs = (unsigned)std::min<uint64_t>((slots + 255) / 256, cap * 2);
-        const unsigned gv = (unsigned)std::min<uint64_t>(((uint64_t)vg->n + 255) / 256, cap);
-        k_dd_indeg<<<gs, 256, 0, st>>>(slots, vg->fwd.vcol, cnt);
-        k_dd_hot<<<gv, 256, 0, st>>>(vg->n, (uint32_t)limit, cnt, ws.dd_hot, ws.dd_hot + HOT_CAP + 1);
-        uint32_t nhot = 0;
-        cudaError_t e = cudaMemcpyAsync(&nhot, ws.dd_hot, sizeof(nhot), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        eeg_status s = e == cudaSuccess ? EEG_OK : cuda_fail(e, "data-driven PageRank set-up", __FILE__, __LINE__);
-        if (s == EEG_OK && nhot) {
-            if (!ws.dd_col) s = vg_alloc(vg, (void**)&ws.dd_col, sizeof(uint32_t) * slots);
-            if (s == EEG_OK && !ws.dd_rep) s = vg_alloc(vg, (void**)&ws.dd_rep, sizeof(double) * 32 * (size_t)hot_stride(nhot));
-            if (s == EEG_OK) k_dd_cols<<<gs, 256, 0, st>>>(slots, vg->fwd.vcol, cnt, ws.dd_col);
+        auto set_up = [&]() -> eeg_status {
+            if (!ws.dd_hot) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_hot, sizeof(uint32_t) * (HOT_CAP + 1 + words)));
+            const cudaError_t e = cudaMallocAsync((void**)&cnt, sizeof(uint32_t) * vg->n, st);
+            if (e != cudaSuccess) {
+                cnt = nullptr;
+                return cuda_fail(e, "cudaMallocAsync(in-degrees)", __FILE__, __LINE__);
+            }
+            EEG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * vg->n, st));
+            EEG_CUDA(cudaMemsetAsync(ws.dd_hot, 0, sizeof(uint32_t) * (HOT_CAP + 1 + words), st));
+            const uint64_t cap = (uint64_t)sm_count(vg->device) * 8;
+            const unsigned gs = (unsigned)std::min<uint64_t>((slots + 255) / 256, cap * 2);
+            const unsigned gv = (unsigned)std::min<uint64_t>(((uint64_t)vg->n + 255) / 256, cap);
+            k_dd_indeg<<<gs, 256, 0, st>>>(slots, vg->fwd.vcol, cnt);
+            k_dd_hot<<<gv, 256, 0, st>>>(vg->n, (uint32_t)limit, cnt, ws.dd_hot, ws.dd_hot + HOT_CAP + 1);
+            uint32_t nhot = 0;
+            EEG_CUDA(cudaMemcpyAsync(&nhot, ws.dd_hot, sizeof(nhot), cudaMemcpyDeviceToHost, st));
+            EEG_CUDA(cudaStreamSynchronize(st));
+            if (nhot) {
+                if (!ws.dd_col) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_col, sizeof(uint32_t) * slots));
+                if (!ws.dd_rep) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_rep, sizeof(double) * 32 * (size_t)hot_stride(nhot)));
+                k_dd_cols<<<gs, 256, 0, st>>>(slots, vg->fwd.vcol, cnt, ws.dd_col);
+            }
+            EEG_CUDA(cudaGetLastError());
+            ws.dd_nhot = nhot;
+            return EEG_OK;
+        };
+        const eeg_status s = set_up();
+        if (cnt) cudaFreeAsync(cnt, st);
+        if (s == EEG_ERR_NOMEM) {
+            (void)cudaGetLastError();
+            vg_free(vg, ws.dd_col);
+            ws.dd_col = nullptr;
+        } else {
+            EEG_TRY(s);
         }
-        cudaFreeAsync(cnt, st);
-        EEG_TRY(s);
-        EEG_CUDA(cudaGetLastError());
-        ws.dd_nhot = nhot;
     }
     ws.dd_hot_ready = true;
     return EEG_OK;
