@@ -485,10 +485,19 @@ eeg_status run_pagerank_dd(eeg_vgraph* vg, eeg_variant variant, const eeg_option
     // idle after the first round, and a queue's scan of the residuals takes a seventh of a long step's phase A (2^26
     // vertices, 1 M edges: 3.1 ms, 11.5 with long steps; a cycle with 4 M leaves 0.33, 0.65. A tree, two vertices per
     // part, still loses, 0.62 and 0.95 in 20 and 23 rounds; R-MAT graphs, whose mass circulates, gain from there on)
-    const bool accel = !(o.pr_accuracy > 0.f) && o.max_iterations == 0 && vg->fwd.P * 4u >= vg->n;
-    if (accel && !ws.dd_taken) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_taken, sizeof(double) * n));
-    if (accel && !ws.dd_share) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_share, sizeof(double) * n));
-    if (!ws.dd_pq) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_pq, sizeof(uint32_t) * P));
+    bool accel = !(o.pr_accuracy > 0.f) && o.max_iterations == 0 && vg->fwd.P * 4u >= vg->n;
+    if (accel) {  // two arrays more; where they do not fit, the rounds keep a queue
+        eeg_status s = EEG_OK;
+        if (!ws.dd_taken) s = vg_alloc(vg, (void**)&ws.dd_taken, sizeof(double) * n);
+        if (s == EEG_OK && !ws.dd_share) s = vg_alloc(vg, (void**)&ws.dd_share, sizeof(double) * n);
+        if (s == EEG_ERR_NOMEM) {
+            (void)cudaGetLastError();
+            accel = false;
+        } else {
+            EEG_TRY(s);
+        }
+    }
+    if (!accel && !ws.dd_pq) EEG_TRY(vg_alloc(vg, (void**)&ws.dd_pq, sizeof(uint32_t) * P));
     if (!ws.ddctrl) EEG_CUDA(cudaMalloc((void**)&ws.ddctrl, sizeof(PRDDCtrl)));
     if (!ws.ev[0]) {
         EEG_CUDA(cudaEventCreate(&ws.ev[0]));

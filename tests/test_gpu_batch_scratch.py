@@ -9,10 +9,10 @@ pytestmark = pytest.mark.gpu
 
 
 def test_a_large_graph_bounds_the_choice(gpu):
-    """900 queries on a small graph alone would take one CTA each; with 2^24 vertices beside it that is 20 GB of scratch."""
+    """900 queries on a small graph alone would take one CTA each; with 21 M vertices beside it that is 25 GB of scratch."""
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(0)
-    n, big = 1000, 1 << 24
+    n, big = 1000, 5 << 22
     s, d, w = (rng.integers(1 if i == 2 else 0, n, 5000, dtype=np.uint32) for i in range(3))
     with gpu.VirtualGraph.build(n, s, d, w) as a, gpu.VirtualGraph.build(big, s, d, w) as b:
         queries = [(0, "sssp", int(s[i])) for i in range(900)]

@@ -30,3 +30,28 @@ with graph() as vg:
     assert failed() == 1
     assert np.abs(x - want).sum() <= 1e-6 * want.sum()
 """)
+
+
+def test_without_long_steps(gpu, tmp_path):
+    """The values, residuals and amounts are there from a run with a threshold; the two arrays that long steps add are
+    refused."""
+    alloc_fail.run(tmp_path, GRAPH + """
+with graph() as vg:
+    run(vg, pr_accuracy=1e-6)
+    fail(8 * n, 8 * n)
+    x, res = run(vg)
+    assert failed() == 1, sizes()
+    assert res["iterations"] > 2 * full["iterations"]  # the queue's rounds
+    assert np.abs(x - want).sum() <= 1e-6 * want.sum()
+""")
+
+
+def test_the_queue_is_not_asked_for_by_long_steps(gpu, tmp_path):
+    alloc_fail.run(tmp_path, GRAPH + """
+with graph() as vg:
+    fail(1, 0)
+    run(vg)
+    assert 4 * P not in sizes(), sizes()
+    run(vg, pr_accuracy=1e-6)
+    assert 4 * P in sizes(), sizes()
+""")
