@@ -595,11 +595,20 @@ __global__ void k_rank_cols(uint64_t slots, const uint32_t* __restrict__ col, co
 
 }  // namespace
 
-static eeg_status ensure_pr_ws(eeg_vgraph* vg, bool res) {
+// *res: the residual form is asked for; cleared where its array (8 bytes per vertex) does not fit.
+static eeg_status ensure_pr_ws(eeg_vgraph* vg, bool* res) {
     Workspace& ws = vg->ws;
     const size_t n = std::max<uint32_t>(vg->n, 1);
     if (!ws.x) EEG_TRY(vg_alloc(vg, (void**)&ws.x, sizeof(float) * n));
-    if (res && !ws.pr_y) EEG_TRY(vg_alloc(vg, (void**)&ws.pr_y, sizeof(float2) * n));
+    if (*res && !ws.pr_y) {
+        const eeg_status s = vg_alloc(vg, (void**)&ws.pr_y, sizeof(float2) * n);
+        if (s == EEG_ERR_NOMEM) {
+            (void)cudaGetLastError();
+            *res = false;
+        } else {
+            EEG_TRY(s);
+        }
+    }
     if (!ws.contrib[0]) EEG_TRY(vg_alloc(vg, (void**)&ws.contrib[0], sizeof(float) * n));
     if (!ws.contrib[1]) EEG_TRY(vg_alloc(vg, (void**)&ws.contrib[1], sizeof(float) * n));
     if (!ws.acc) EEG_TRY(vg_alloc(vg, (void**)&ws.acc, sizeof(double) * n));
@@ -651,8 +660,8 @@ eeg_status run_pagerank(eeg_vgraph* vg, eeg_variant variant, const eeg_options& 
         return EEG_ERR_INVALID;
     }
     // a run with an explicit sweep cap keeps the plain iterates
-    const bool res_form = o.max_iterations == 0;
-    EEG_TRY(ensure_pr_ws(vg, res_form));
+    bool res_form = o.max_iterations == 0;
+    EEG_TRY(ensure_pr_ws(vg, &res_form));
     EEG_TRY(ensure_pr_rank(vg, st));
     Workspace& ws = vg->ws;
     const float damping = o.pr_damping > 0.f ? o.pr_damping : 0.85f;
