@@ -257,16 +257,21 @@ static eeg_status build_impl(uint32_t n, uint64_t m, const uint32_t* src, const 
     const uint32_t *ms = nullptr, *md = nullptr, *mw = nullptr;
     // a build that reads its input more than once (two directions, both directions of each edge) copies it
     // once (the copy engine moves it as fast as the in-place reads) instead of reading it over the link twice
-    const bool zero_copy = !on_device && m > 0 && !(flags & EEG_VG_REVERSE) && !symmetrize && mapped(src, &ms) &&
-                           mapped(dst, &md) && mapped(w, &mw);
+    const bool in_place = !on_device && m > 0 && !(flags & EEG_VG_REVERSE) && mapped(src, &ms) && mapped(dst, &md) && mapped(w, &mw);
+    bool zero_copy = in_place && !symmetrize;
     cudaEventRecord(e0, st);
+    if (in_place && symmetrize && cudaMallocAsync((void**)&tmp, (size_t)m * (w ? 3 : 2) * sizeof(uint32_t), st) != cudaSuccess) {
+        (void)cudaGetLastError();  // the copy does not fit: read twice after all
+        tmp = nullptr;
+        zero_copy = true;
+    }
     if (zero_copy) {
         ds = ms;
         dd = md;
         dw = mw;
     } else if (!on_device && m > 0) {
         const size_t words = (size_t)m * (w ? 3 : 2);
-        cudaError_t ce = cudaMallocAsync((void**)&tmp, words * sizeof(uint32_t), st);
+        const cudaError_t ce = tmp ? cudaSuccess : cudaMallocAsync((void**)&tmp, words * sizeof(uint32_t), st);
         if (ce != cudaSuccess) {
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
