@@ -944,17 +944,22 @@ eeg_status build_direction(eeg_vgraph* vg, VDir* d, const uint32_t* d_src, const
         if (host_in) EEG_TRY(T.get((void**)&copy, sizeof(uint32_t) * m));
         uint32_t* in_key = nullptr;  // null: the arcs
         uint32_t *in_nb = nullptr, *in_pay = nullptr;
+        void* out_keys[2] = {nullptr, nullptr};
+        uint32_t *out_nbs[2] = {nullptr, nullptr}, *out_pays[2] = {nullptr, nullptr};
         uint32_t lo = low;
         for (uint32_t p = 0; p < passes; ++p) {
             const bool last = p + 1 == passes;
             // bits of this pass (at least 2: the tile kernels take four bins per thread)
             const uint32_t pbits = std::max(2u, last ? std::max(bits, lo) - lo : (high + passes - 1) / passes);
             const uint32_t bins = 1u << pbits;
-            void* out_key = nullptr;
-            uint32_t *out_nb = nullptr, *out_pay = nullptr;
-            EEG_TRY(T.get(&out_key, (low_keys ? sizeof(uint16_t) : sizeof(uint32_t)) * m));
-            EEG_TRY(T.get((void**)&out_nb, sizeof(uint32_t) * m));
-            if (payload) EEG_TRY(T.get((void**)&out_pay, sizeof(uint32_t) * m));
+            // two sets of outputs in turn: the third pass's are the first's
+            if (p < 2) {
+                EEG_TRY(T.get(&out_keys[p], (low_keys ? sizeof(uint16_t) : sizeof(uint32_t)) * m));
+                EEG_TRY(T.get((void**)&out_nbs[p], sizeof(uint32_t) * m));
+                if (payload) EEG_TRY(T.get((void**)&out_pays[p], sizeof(uint32_t) * m));
+            }
+            void* out_key = out_keys[p & 1u];
+            uint32_t *out_nb = out_nbs[p & 1u], *out_pay = out_pays[p & 1u];
             const uint64_t nt = p == 0 ? ntiles : ntiles2, nc = (nt + S_CHUNK - 1) / S_CHUNK;
             if (p == 0)
                 k_bin_counts<true><<<(unsigned)nt, S_TPB, 0, st>>>(s, nullptr, copy, m, lo, bins, hist);

@@ -30,3 +30,15 @@ try:  # pageable input has to be copied
 except E.EEGError:
     pass
 """)
+
+
+def test_two_sets_of_edges(gpu, tmp_path):
+    alloc_fail.run(tmp_path, """
+n, m = (1 << 22) + 5, 500003  # sorted by vertex in three passes
+rng = np.random.default_rng(1)
+s, d = rng.integers(0, n, m, dtype=np.uint32), rng.integers(0, n, m, dtype=np.uint32)
+fail(1, 0)
+with E.VirtualGraph.build(n, s, d, None, K=8) as vg:
+    pass
+assert sizes().count(4 * m) == 6, sizes()  # owners, neighbours and weights, twice
+""")
