@@ -1212,6 +1212,12 @@ eeg_status build_chunks(eeg_ppr* p, const VDir& vd, PPRDir& d) {
     eeg_vgraph* vg = p->vg;
     const uint32_t n = vg->n, K = vg->K;
     const uint32_t CH = PPR_SLOTS / K;
+    // Small graphs: chunks only as large as it takes to give every resident warp one. A chunk's vertices end one after
+    // another (some 230 instructions each), so with full chunks a sweep of a 150^2 grid, 16 columns, was one warp's 16
+    // vertices: 26.8 us, 18.6 so (64 columns 20.6 -> 15.9; a path of 5000 vertices 16.6 -> 11.6). A single column's chunk is
+    // worked on by all lanes at once.
+    const uint64_t warps = (uint64_t)sm_count(vg->device) * 24u;
+    const uint32_t pack = p->W == 1 ? CH : (uint32_t)std::min<uint64_t>(CH, std::max<uint64_t>(1, (vd.P + warps - 1) / warps));
     std::vector<uint32_t> vs((size_t)n + 1);
     EEG_CUDA(cudaMemcpy(vs.data(), vd.vstart, sizeof(uint32_t) * ((size_t)n + 1), cudaMemcpyDeviceToHost));
     std::vector<Chunk> ch;
@@ -1239,7 +1245,7 @@ eeg_status build_chunks(eeg_ppr* p, const VDir& vd, PPRDir& d) {
         const uint32_t p0 = vs[v];
         uint32_t p1 = vs[v + 1];
         ++v;
-        while (v < n && vs[v + 1] - vs[v] <= CH && vs[v + 1] - p0 <= CH) {
+        while (v < n && vs[v + 1] - vs[v] <= CH && vs[v + 1] - p0 <= pack) {
             p1 = vs[v + 1];
             ++v;
         }
