@@ -160,9 +160,9 @@ __device__ __forceinline__ bool grid_barrier(BarrierWords* bw, uint32_t& epoch, 
 // The same barrier for grids whose CTAs arrive together (PageRank's balanced sweeps): the arrival
 // itself releases the CTA's writes (ordered before this thread by the __syncthreads), and each spin is
 // one acquire load of the arrivals and the abort word together, so the last arrival is seen one L2
-// round trip sooner (R-MAT s22 PageRank, 93 barriers: 17.35 -> 17.10 ms). Where CTAs finish at
-// different times the faster polling slowed the CTAs still working (SSSP 0.700 -> 0.719 ms), so the
-// traversals keep grid_barrier.
+// round trip sooner (R-MAT s22 PageRank, 93 barriers: 17.35 -> 17.10 ms). In the traversals, whose CTAs
+// finish at different times, it took the place of grid_barrier at a loss (SSSP 0.700 -> 0.719 ms); their rounds end on
+// round_barrier (traverse.cuh), whose polled word also brings the queue's length.
 __device__ __forceinline__ bool grid_barrier_sync(BarrierWords* bw, uint32_t& epoch, uint64_t timeout_ns) {
     __shared__ uint32_t s_ok2;
     __syncthreads();

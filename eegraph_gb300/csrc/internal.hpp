@@ -126,10 +126,10 @@ struct Workspace {
     double* dd_amt = nullptr;     // n: push amount of each vertex activated in the current round
     double* dd_taken = nullptr;   // n: residual each vertex took in the last round (long steps)
     double* dd_share = nullptr;   // n: d / outdeg (long steps)
-    uint32_t* dd_pq = nullptr;    // P: part queue of the current round
-    uint32_t* dd_hot = nullptr;   // hot targets: their number, up to 4096 of them, a bit per vertex
+    uint32_t* dd_pq = nullptr;    // P: part queue of the current round (runs without long steps)
+    uint32_t* dd_hot = nullptr;   // hot targets: their number, up to HOT_CAP (32768) of them, a bit per vertex
     uint32_t* dd_col = nullptr;   // the targets with hot ones marked (P * K; none without hot targets)
-    double* dd_rep = nullptr;     // dd_nhot x 32 partial residuals
+    double* dd_rep = nullptr;     // 32 x (dd_nhot rounded up to 16) partial residuals
     uint32_t dd_nhot = 0;
     bool dd_hot_ready = false;
     PRDDCtrl* ddctrl = nullptr;

@@ -31,7 +31,7 @@
 // may be negative): with only those above acc, the last decade lost its single mode and some graphs took 60
 // rounds instead of 22-26. So the rounds need no queue: phase A walks the vertices, phase B all parts. A phase
 // A that finds nothing above acc is undone from the recorded residuals. R-MAT s17, K = 8:
-// 10.5 -> 0.66 ms (with the hot targets below).
+// 10.5 -> 0.66 ms (with the hot targets below; a graph's first run also sets those up, 0.88 ms).
 // Hot targets: reductions to one 128-byte line are done one after another (4 ns each on one address, 1 to 1.5 ns
 // within a line by the times below; on lines of their own 175 G/s), so the pushes to an R-MAT graph's first vertices, which share
 // lines, set the round's time. Vertices with more than m / 32768 in-edges (and more than 64) therefore

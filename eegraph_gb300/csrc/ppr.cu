@@ -557,8 +557,11 @@ __device__ __forceinline__ void stage_chunk(const DirTab& g, Stage* s, uint32_t 
 // while the current one is gathered; for 64 columns what is the same in the whole grid, and the FP64 sums,
 // are kept in shared memory (8 row gathers take 32 of a lane's registers; 32 columns, whose vertices end twice
 // as often per gather, keep them in registers: 125 against 147 us a sweep). R-MAT s18 x 64 columns, one sweep: 183 us with
-// the ids loaded step by step and 150 bytes spilled, 158 us so with 3 CTAs per SM (24 warps).
-//   CTAS = 4 (64 registers, rare spills): more rows in flight where they come from beyond L2 or its far half:
+// the ids loaded step by step and 150 bytes spilled, 158 us so with 3 CTAs per SM (24 warps; 56 bytes spilled).
+//   The kinds of vertex end, inlined together, still spill: 168 bytes of stores and 192 to 268 of loads at 64 registers, 164
+// to 232 and 144 to 204 for 32 columns. A function per kind of sweep, called once per sweep, spills 24 to 112 in the loops
+// that count and is slower on R-MAT (s18 156 -> 164 us, 32 columns 125 -> 141).
+//   CTAS = 4 (64 registers): more rows in flight where they come from beyond L2 or its far half:
 // s18 158 -> 155 us, s20 625 -> 575; but s16 51 -> 53, 100 K vertices with K = 16 50 -> 55. So 4 is taken
 // for rows above 48 MB. NQ = W/4 lanes per row.
 constexpr size_t PPR_MANY_ROWS = (size_t)48 << 20;

@@ -203,7 +203,10 @@ EEG_API void eeg_vgraph_destroy(eeg_vgraph* vg);
 /* ------------------------------------------------------------------ runs */
 
 typedef struct eeg_options {
-    uint32_t max_iterations;  /* 0 = default cap (n+2 for traversals, 10000 for PageRank) */
+    uint32_t max_iterations;  /* 0 = default cap (n+2 for traversals, 10000 for PageRank). Any other value keeps the
+                               * plain iterates of the PageRank solvers (eeg_run, eeg_ppr_*), also where the cap is
+                               * not reached: the result after k sweeps is the k-th one, and a run takes several
+                               * times the sweeps of an uncapped one to the same tolerance */
     float pr_tolerance;       /* PageRank stop: bound on ||x - x*||_1 / ||x||_1 (0 = 1e-7) */
     float pr_damping;         /* 0 = 0.85 (src/pr.cu:43) */
     float pr_accuracy;        /* DD PageRank activation threshold on |delta| (0 = derived from tolerance) */
