@@ -439,7 +439,8 @@ __device__ __forceinline__ int end_sweep(const SolveArgs& a, uint32_t s, double 
 
 // A solve with long steps whose L1 test is met after sweep s looks at every element of its iterate (see
 // VertexBound): 0 = one is off, and the control's next step is set for it; 1 = none is; 2 = the grid is aborting.
-// Forward solves only: their values are sums of one sign, so each has a size of its own to be measured by.
+// Forward solves only: their values are sums of one sign, so each has a size of its own to be measured by (a source with
+// a negative entry leaves the look out: what cancels has none, and would keep the solve sweeping).
 // (Adjoints, whose values cancel, came out as close as from plain sweeps, element by element, in the same 64-bit
 // model.) Symmetrised R-MAT s14-s17, 32 seeds a column: elements 1e-4 to 1e-3 off without it, 8e-7 with it, 3e-7 to
 // 2e-6 with plain sweeps; 15 to 25 more sweeps. The estimate (before two more plain sweeps) is there 1e-3 and more, on
@@ -452,6 +453,8 @@ static __device__ __noinline__ int look(const SolveArgs& a, uint32_t width, uint
     const float *f = (s & 1u) ? a.y0 : a.y1, *fo = (s & 1u) ? a.y1 : a.y0, *y = a.y;
     const uint64_t count = (uint64_t)a.n * width;
     uint32_t far = 0;
+    const bool signs = ex->looks == 0u;  // the first look also looks for a negative source
+    const float4* b4 = reinterpret_cast<const float4*>(a.b);
     auto one = [&](float fv, float yv, uint64_t i) {
         far |= vertex_off<true>(most, a.bound.d, fv, yv, [&]() { return fo[i]; }) ? 1u : 0u;
     };
@@ -463,14 +466,21 @@ static __device__ __noinline__ int look(const SolveArgs& a, uint32_t width, uint
         one(fv.y, yv.y, 4u * i + 1u);
         one(fv.z, yv.z, 4u * i + 2u);
         one(fv.w, yv.w, 4u * i + 3u);
+        if (signs && width > 1u) {
+            const float4 b = b4[i];
+            far |= fminf(fminf(b.x, b.y), fminf(b.z, b.w)) < 0.f ? 2u : 0u;
+        }
     }
     for (uint64_t i = count / 4u * 4u + t0; i < count; i += step) one(f[i], y[i], i);
-    far = __syncthreads_or(far);
-    if (threadIdx.x == 0 && far) atomicOr(&a.ctrl->far[s % 3u], 1u);
+    if (signs && width == 1u)  // a single column's source need not be aligned
+        for (uint64_t i = t0; i < count; i += step) far |= a.b[i] < 0.f ? 2u : 0u;
+    far = (__syncthreads_or(far & 1u) ? 1u : 0u) | (__syncthreads_or(far & 2u) ? 2u : 0u);
+    if (threadIdx.x == 0 && far) atomicOr(&a.ctrl->far[s % 3u], far);
     if (!grid_barrier(&a.ctrl->bw, epoch, a.timeout_ns)) return 2;
     __shared__ uint32_t s_far;
     if (threadIdx.x == 0) {
-        s_far = __ldcg(&a.ctrl->far[s % 3u]);
+        const uint32_t found = __ldcg(&a.ctrl->far[s % 3u]);
+        s_far = found == 1u ? 1u : 0u;
         if (s_far) vertices_off(*ex, (double)a.d);
     }
     __syncthreads();

@@ -78,3 +78,25 @@ def test_ppr_element_by_element(gpu, name, C, K):
                 assert np.array_equal(x == 0, want == 0)
                 off = (np.abs(x - want)[want > 0] / want[want > 0]).max()
                 assert off <= 8 * (tol or 1e-7) + 1e-5, (tol, off)
+
+
+@pytest.mark.parametrize("C,K", [(1, 8), (5, 4), (64, 8)])
+def test_ppr_sources_of_both_signs(gpu, C, K):
+    """Values that cancel have no size of their own: the solve ends on its norm, in few sweeps."""
+    sp = pytest.importorskip("scipy.sparse")
+    n = 1 << 13
+    s, d, _ = gpu.gen_rmat(13, 16, seed=2)
+    rng = np.random.default_rng(3)
+    w = (rng.random(len(s)) + 0.05).astype(np.float32)
+    T = rng.standard_normal((n, C)).astype(np.float32)
+    A = sp.csr_matrix((0.85 * w.astype(np.float64) / np.bincount(s, w.astype(np.float64), n)[s], (d, s)), (n, n))
+    f = want = 0.15 * T.astype(np.float64)
+    while np.abs(f).sum() > 1e-16 * np.abs(want).sum():
+        f = A @ f
+        want = want + f
+    with gpu.VirtualGraph.build(n, s, d, None, K=K, reverse=True, edge_ids=True) as vg, gpu.PPR(vg, C) as p:
+        p.set_weights(w)
+        x, res = p.forward(T)
+        assert res["iterations"] < 60, res["iterations"]
+        # the tolerance, and FP32's share as in the elements' test; rows of mixed signs cancel to a quarter at worst here
+        assert np.abs(x - want).sum() <= (1e-7 + 1e-5) * np.abs(want).sum()
